@@ -1,9 +1,9 @@
 // rg_adjoint.cu -- forward side of the differentiated step (FP64, compiled
 // without FMA contraction like rg_fp64.cu):
 //
-//   k_record_slopes  LinearGaussImproved slopes of W_k, as rg_fp64.cu's
-//                    k_slopes computes them, plus the limiter trace the
-//                    reverse slope kernel needs (SlopeTrace)
+//   adj_launch_record_slopes  LinearGaussImproved slopes of W_k with the
+//                    limiter trace the reverse slope kernel needs
+//                    (SlopeTrace): rg_fp64.cu's slopes kernel, its trace build
 //   k_tl_*           tangent-linear model: the same formulas on dual numbers
 //                    (value, tangent).  The value parts follow the production
 //                    kernels' operation order, so a tangent run reproduces the
@@ -42,20 +42,14 @@ __device__ __forceinline__ Dual operator/(Dual a, double b) { return Dual{quot(a
 // quotients of the templated code: rg::quot for double, the operators for Dual
 __device__ __forceinline__ Dual quot(Dual a, Dual b) { return a / b; }
 __device__ __forceinline__ Dual quot(Dual a, double b) { return a / b; }
-__device__ __forceinline__ Dual operator-(Dual a, double b) { return Dual{a.v - b, a.d}; }
 __device__ __forceinline__ Dual dsqrt(Dual a) {
   const double s = root(a.v);
   return Dual{s, quot(a.d, 2.0 * s)};
 }
-__device__ __forceinline__ double dsqrt(double a) { return root(a); }
-__device__ __forceinline__ double val(double x) { return x; }
 __device__ __forceinline__ double val(Dual x) { return x.v; }
 __device__ __forceinline__ double tan_of(Dual x) { return x.d; }
-__device__ __forceinline__ double tan_of(double) { return 0.0; }
 template <class T>
 __device__ __forceinline__ T constant(double x);
-template <>
-__device__ __forceinline__ double constant<double>(double x) { return x; }
 template <>
 __device__ __forceinline__ Dual constant<Dual>(double x) { return Dual{x, 0.0}; }
 
@@ -82,12 +76,6 @@ __device__ __forceinline__ void store_raw(double* c, int i, double a, double b, 
 template <class T>
 __device__ __forceinline__ V4<T> load4(const double* c, const double* dc, int i);
 template <>
-__device__ __forceinline__ V4<double> load4<double>(const double* c, const double*, int i) {
-  V4<double> r;
-  load_raw(c, i, r.v);
-  return r;
-}
-template <>
 __device__ __forceinline__ V4<Dual> load4<Dual>(const double* c, const double* dc, int i) {
   double x[4], t[4];
   load_raw(c, i, x);
@@ -107,7 +95,7 @@ __device__ __forceinline__ int entry_source(const AdjArgs& a, int k) {
 // LinearGaussImproved.cpp:67-134 (naive slope), :136-157 (is_shock),
 // :174-399 (the two limiters) for a real cell with no self-mirror
 // neighbour, in the operation order of rg_fp64.cu's k_slopes.
-template <class T, bool kTrace>
+template <class T>
 __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
   const MeshDev& m = a.mesh;
   const V4<T> cell = load4<T>(a.cells, a.dcells, i);
@@ -137,16 +125,6 @@ __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
     sx.v[q] = vx.v[q] * mi.x + vy.v[q] * mi.y;
     sy.v[q] = vy.v[q] * mi.w + vx.v[q] * mi.z;
   }
-  SlopeTrace* tr = kTrace ? a.trace + i : nullptr;
-  if (kTrace) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      tr->naive[q] = val(sx.v[q]);
-      tr->naive[4 + q] = val(sy.v[q]);
-    }
-  }
-  int code[4] = {kTraceNone, kTraceNone, kTraceNone, kTraceNone};
-  double dphi_at[4] = {0, 0, 0, 0};
   T psi[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) psi[q] = constant<T>(1.0);
@@ -209,23 +187,14 @@ __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
           if (dv > t1 || dv < t2) {
             const bool up = dv > t1;
             const T cand = quot(up ? nmax : nmin, dphi);
-            if (val(cand) < val(psi[q])) {
-              psi[q] = cand;
-              const int ex = up ? amax[q] : amin[q];
-              code[q] = k | ((up ? 0 : 1) << 8) | ((ex + 1) << 16);
-              dphi_at[q] = dv;
-            }
+            if (val(cand) < val(psi[q])) psi[q] = cand;
           }
         } else if (fabs(dv) > 1e-9 * cq) {
           const T nb = load4<T>(a.cells, a.dcells, entry_source(a, b + k)).v[q];
           const T cand = quot(a.theta * (nb - cell.v[q]), dphi);
           const bool clamp = val(cand) < 0.0;  // std::max(cand, 0)
           const T x = clamp ? constant<T>(0.0) : cand;
-          if (val(x) < val(psi[q])) {
-            psi[q] = x;
-            code[q] = k | ((clamp ? 3 : 2) << 8) | ((k + 1) << 16);
-            dphi_at[q] = dv;
-          }
+          if (val(x) < val(psi[q])) psi[q] = x;
         }
       }
     }
@@ -234,14 +203,6 @@ __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
   for (int q = 0; q < 4; ++q) {
     sx.v[q] = sx.v[q] * psi[q];
     sy.v[q] = sy.v[q] * psi[q];
-  }
-  if (kTrace) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      tr->psi[q] = val(psi[q]);
-      tr->dphi[q] = dphi_at[q];
-      tr->code[q] = code[q];
-    }
   }
 }
 
@@ -255,19 +216,11 @@ __device__ __forceinline__ void store_slope(const AdjArgs& a, int i, const V4<T>
   }
 }
 
-__global__ void __launch_bounds__(kBlock) k_record_slopes(AdjArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.mesh.n) return;
-  V4<double> sx, sy;
-  lgi_slope<double, true>(a, i, sx, sy);
-  store_slope(a, i, sx, sy);
-}
-
 __global__ void __launch_bounds__(kBlock) k_tl_slopes(AdjArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.mesh.n) return;
   V4<Dual> sx, sy;
-  lgi_slope<Dual, false>(a, i, sx, sy);
+  lgi_slope<Dual>(a, i, sx, sy);
   store_slope(a, i, sx, sy);
 }
 
@@ -429,8 +382,20 @@ inline int blocks(int n) { return (n + kBlock - 1) / kBlock; }
 }  // namespace
 
 cudaError_t adj_launch_record_slopes(const AdjArgs& a, cudaStream_t s) {
-  k_record_slopes<<<blocks(a.mesh.n), kBlock, 0, s>>>(a);
-  return cudaGetLastError();
+  StepArgs t{};
+  t.mesh = a.mesh;
+  t.geom = a.geom;
+  t.gamma = a.gamma;
+  t.order = 2;
+  t.ghost_kind = RG_GHOST_PERIODIC;
+  t.slf = a.slf;
+  t.delta_v = a.delta_v;
+  t.theta = a.theta;
+  t.delta_p = a.delta_p;
+  t.cells = const_cast<double*>(a.cells);
+  t.slopes = a.slopes;
+  t.status = a.status;
+  return launch_slopes_trace(t, a.trace, s);
 }
 
 cudaError_t tl_launch_init(const AdjArgs& a, cudaStream_t s) {

@@ -124,6 +124,7 @@ void fill_views(MeshSlot& s) {
   s.geom.cflags = at<int>(b, L.cflags);
   s.geom.nbr = at<uint32_t>(b, L.nbr);
   s.geom.hr = at<double2>(b, L.hr);
+  s.geom.dmf = at<float2>(b, L.dmf);
   s.geom.ghost_real = at<int>(b, L.ghost_real);
   s.geom.ghost_unit = at<double2>(b, L.ghost_unit);
   s.geom.cell_order = at<int>(b, L.cell_order);
@@ -538,6 +539,7 @@ rg_status geometry_pass(rg_handle* h, MeshSlot& s, const rg::MeshDev& gm, bool f
   ga.cflags = at<int>(b, s.lay.cflags);
   ga.nbr = at<uint32_t>(b, s.lay.nbr);
   ga.hr = at<double2>(b, s.lay.hr);
+  ga.dmf = at<float2>(b, s.lay.dmf);
   ga.ghost_real = at<int>(b, s.lay.ghost_real);
   ga.ghost_unit = at<double2>(b, s.lay.ghost_unit);
   ga.cell_order = at<int>(b, s.lay.cell_order);
@@ -648,6 +650,10 @@ rg_status rg_create(const rg_config* cfg, rg_handle** out) {
   if (!h) return RG_ERR_OUT_OF_MEMORY;
   h->cfg = *cfg;
   h->mixed = cfg->precision == RG_FP32_MIXED;
+  // the FP64 slopes: the build for three resident blocks of 256 (80 registers),
+  // in blocks of 128 (512^2: 197 us; 245 us as the plain build in blocks of 256,
+  // whose 106 registers leave 16 warps per SM and a coarse last wave)
+  h->shapes64.slopes = rg::LaunchShape{128, 0, 2};
   h->heun = cfg->time_integrator == RG_TIME_ADVANCE_HEUN;
   auto fail = [&](cudaError_t e) {
     rg_destroy(h);

@@ -27,7 +27,12 @@ namespace rg {
 
 RG_CONV_FN uint64_t conv_dbits(double x) {
 #ifdef __CUDA_ARCH__
-  return static_cast<uint64_t>(__double_as_longlong(x));
+  // a move the compiler does not see through: it turns masks of a double's
+  // bits back into FP64 operations (the sign mask into an absolute value),
+  // which issue at two per clock per SM
+  uint64_t u;
+  asm("mov.b64 %0, %1;" : "=l"(u) : "d"(x));
+  return u;
 #else
   uint64_t u;
   memcpy(&u, &x, 8);

@@ -66,7 +66,10 @@ namespace div_detail {
 
 RG_DIV_FN uint64_t d2u(double x) {
 #if defined(__CUDA_ARCH__)
-  return static_cast<uint64_t>(__double_as_longlong(x));
+  // opaque to the compiler, as rg_convert.cuh's conv_dbits
+  uint64_t u;
+  asm("mov.b64 %0, %1;" : "=l"(u) : "d"(x));
+  return u;
 #else
   uint64_t u;
   std::memcpy(&u, &x, sizeof u);

@@ -17,8 +17,10 @@
 // Geometry-only terms are computed once per mesh upload (k_geom_*).
 #include <math.h>
 
+#include "rg_adjoint.cuh"
 #include "rg_fp64.cuh"
 #include "rg_hllc.cuh"
+#include "rg_lgi.cuh"
 
 namespace rg {
 namespace {
@@ -96,8 +98,10 @@ __global__ void __launch_bounds__(kBlock) k_geom_cells(GeomArgs a) {
     const double2 cci = m.cms[i];
     double sxsy = 0, sy2 = 0, sx2 = 0;
     for (int k = 0; k < nn; ++k) {
-      const int2 fc = m.face_cells[m.cell_faces[b + k]];
+      const int e = m.cell_faces[b + k];
+      const int2 fc = m.face_cells[e];
       const bool first = fc.x == i;
+      a.dmf[b + k] = dm_screen((first ? a.dm0 : a.dm1)[e]);
       const int other = first ? fc.y : fc.x;
       const bool mirror = orig_of(m, fc.x) == orig_of(m, fc.y);
       a.nbr[b + k] = static_cast<uint32_t>(other) | (mirror ? kNbrMirror : 0u) | (first ? kNbrFirst : 0u);
@@ -115,9 +119,11 @@ __global__ void __launch_bounds__(kBlock) k_geom_cells(GeomArgs a) {
     record_error(a.status, 0, RG_ERR_TOO_MANY_NEIGHBORS, 2, i, nn);
     a.minv[i] = make_dbl4(0, 0, 0, 0);
     for (int k = 0; k < nn; ++k) {
-      const int2 fc = m.face_cells[m.cell_faces[b + k]];
+      const int e = m.cell_faces[b + k];
+      const int2 fc = m.face_cells[e];
       const bool first = fc.x == i;
       a.nbr[b + k] = static_cast<uint32_t>(first ? fc.y : fc.x) | (first ? kNbrFirst : 0u);
+      a.dmf[b + k] = dm_screen((first ? a.dm0 : a.dm1)[e]);
     }
     return;
   }
@@ -128,6 +134,7 @@ __global__ void __launch_bounds__(kBlock) k_geom_cells(GeomArgs a) {
     const int2 fc = m.face_cells[e];
     const bool first = fc.x == i;
     a.nbr[b + k] = static_cast<uint32_t>(first ? fc.y : fc.x) | (first ? kNbrFirst : 0u);
+    a.dmf[b + k] = dm_screen((first ? a.dm0 : a.dm1)[e]);
     const double2 r = a.rij[e], c = a.cij[e];
     // -r_ij for the second cell: a sign flip of the bit pattern
     const uint64_t flip = first ? 0u : 0x8000000000000000ull;
@@ -336,72 +343,49 @@ __global__ void __launch_bounds__(kBlock) k_ghost_fill(StepArgs a) {
   if (g < a.mesh.g) fill_ghost(a, g);
 }
 
-// LinearGaussImproved.cpp:425-494 calc_slope for one cell (serial build).
-template <bool kBatch>
-__device__ __forceinline__ void k_slopes_item(const StepArgs& a, int i) {
+// LinearGaussImproved.cpp:425-494 calc_slope of one component of one cell:
+// lane q of a quad forms component q of {d, p, vx, vy}.  The four components
+// share the geometry and the shock decision only, so a warp takes eight cells
+// and each lane's chain of dependent operations is a quarter of a cell's; the
+// FP64 operations of a lane are the Green-Gauss sums (8 per neighbour), which
+// the reference's order of additions fixes, plus the limiter's surviving
+// candidates (rg_lgi.cuh).  `quad`: the quad's lanes in the warp (all four run
+// with the same cell).  Bound by the FP64 pipe (85 FP64 instructions per warp
+// of eight cells, 72 % active).  With one thread per cell and every candidate
+// in FP64 (117 per warp of eight cells at full lanes, 5,960 instructions in
+// one chain): 478 us at 512^2, 95 us at 256^2, 89 us at 96 x 101 cells; now
+// 197, 51 and 17 us.
+template <bool kBatch, bool kTrace>
+__device__ __forceinline__ void slopes_lane(const StepArgs& a, int i, int q, unsigned quad, SlopeTrace* trace) {
   const MeshDev& m = a.mesh;
-  const Cell cell = load_cell(a.cells, i);
+  const double c = a.cells[4 * static_cast<size_t>(i) + q];
   const int b = m.cell_off[i], nn = m.cell_off[i + 1] - b;
-  const dbl4 mi = a.geom.minv[i];
-  Cell sx, sy;
-  if (a.geom.cflags[i] & kCellBoundarySlope) {
-    // :401-422 GetBoundarySlope
-    Cell phisy{0, 0, 0, 0}, phisx{0, 0, 0, 0};
-    for (int k = 0; k < nn; ++k) {
-      const Cell nb = point_state(a, static_cast<int>(a.geom.nbr[b + k] & kNbrIdMask));
-      const double2 h = a.geom.hr[b + k];
-      const Cell df{nb.d - cell.d, nb.p - cell.p, nb.vx - cell.vx, nb.vy - cell.vy};
-      phisy.d = phisy.d + df.d * h.y;
-      phisy.p = phisy.p + df.p * h.y;
-      phisy.vx = phisy.vx + df.vx * h.y;
-      phisy.vy = phisy.vy + df.vy * h.y;
-      phisx.d = phisx.d + df.d * h.x;
-      phisx.p = phisx.p + df.p * h.x;
-      phisx.vx = phisx.vx + df.vx * h.x;
-      phisx.vy = phisx.vy + df.vy * h.x;
-    }
-    const double sxsy = mi.x, sx2 = mi.y, sy2 = mi.z, den = mi.w;
-    sx = Cell{quot(phisy.d * sxsy - phisx.d * sy2, den), quot(phisy.p * sxsy - phisx.p * sy2, den),
-              quot(phisy.vx * sxsy - phisx.vx * sy2, den), quot(phisy.vy * sxsy - phisx.vy * sy2, den)};
-    sy = Cell{quot(phisx.d * sxsy - phisy.d * sx2, den), quot(phisx.p * sxsy - phisy.p * sx2, den),
-              quot(phisx.vx * sxsy - phisy.vx * sx2, den), quot(phisx.vy * sxsy - phisy.vy * sx2, den)};
+  const bool boundary = a.geom.cflags[i] & kCellBoundarySlope;
+  const HydroComp load{a, q};
+  double sx, sy;
+  LaneNeighbours nb;
+  const bool fits = nn <= kFit;
+  if (fits) {
+    lane_load(a, b, nn, load, nb);
+    lane_slope(a, i, b, nn, boundary, c, nb, sx, sy);
   } else {
-    // :80-133 calc_naive_slope, right-hand side and solve
-    // the first neighbour starts the sums (cell*h, then + nb*h); the loop
-    // takes the rest, so no iteration joins two computed values
-    Cell vx{0, 0, 0, 0}, vy{0, 0, 0, 0};
-    if (nn > 0) {
-      const Cell nb = point_state(a, static_cast<int>(a.geom.nbr[b] & kNbrIdMask));
-      const double2 h = a.geom.hr[b];
-      vx = Cell{cell.d * h.x, cell.p * h.x, cell.vx * h.x, cell.vy * h.x};
-      vy = Cell{cell.d * h.y, cell.p * h.y, cell.vx * h.y, cell.vy * h.y};
-      addmult(vy, nb, h.y);
-      addmult(vx, nb, h.x);
-    }
-    for (int k = 1; k < nn; ++k) {
-      const Cell nb = point_state(a, static_cast<int>(a.geom.nbr[b + k] & kNbrIdMask));
-      const double2 h = a.geom.hr[b + k];
-      addmult(vx, cell, h.x);
-      addmult(vy, cell, h.y);
-      addmult(vy, nb, h.y);
-      addmult(vx, nb, h.x);
-    }
-    sx = Cell{vx.d * mi.x, vx.p * mi.x, vx.vx * mi.x, vx.vy * mi.x};
-    sy = Cell{vy.d * mi.w, vy.p * mi.w, vy.vx * mi.w, vy.vy * mi.w};
-    addmult(sx, vy, mi.y);
-    addmult(sy, vx, mi.z);
+    lane_slope_any(a, i, b, nn, boundary, c, load, sx, sy);
   }
+  double psi = 1.0, dphi_at = 0.0;
+  int code = kTraceNone;
+  const double nsx = sx, nsy = sy;
   if (a.slf) {
     // :136-157 is_shock / PressureRatio.  cond1 is
     // (div v)*width < -delta_v*cs: false whenever the left side is >= 0,
     // otherwise screened in FP32 against |left| vs delta_v*cs.
-    const double lhs = (sx.vx + sy.vy) * a.geom.width[i];
+    const double lhs = (quad_value(quad, sx, 2) + quad_value(quad, sy, 3)) * a.geom.width[i];
+    const double2 dp = reinterpret_cast<const double2*>(a.cells)[2 * static_cast<size_t>(i)];
     bool shock = false;
     if (lt(lhs, 0.0)) {
-      const double gp = gamma_at<kBatch>(a, i) * cell.p;
+      const double gp = gamma_at<kBatch>(a, i) * dp.y;
       bool decided = false;
-      if (fp32_safe(lhs) && fp32_safe(gp) && fp32_safe(cell.d)) {
-        const float rhs_f = narrow(a.delta_v) * sqrtf(narrow(gp) / narrow(cell.d));
+      if (fp32_safe(lhs) && fp32_safe(gp) && fp32_safe(dp.x)) {
+        const float rhs_f = narrow(a.delta_v) * sqrtf(narrow(gp) / narrow(dp.x));
         const float l_f = -narrow(lhs);
         if (l_f > rhs_f * 1.000002f) {
           shock = true;
@@ -410,104 +394,76 @@ __device__ __forceinline__ void k_slopes_item(const StepArgs& a, int i) {
           decided = true;
         }
       }
-      if (!decided) shock = lhs < (-a.delta_v) * root(quot(gp, cell.d));
+      if (!decided) shock = lhs < (-a.delta_v) * root(quot(gp, dp.x));
     }
     if (!shock && nn == 0) shock = 1.0 < a.delta_p;  // PressureRatio of no neighbours is 1
     if (!shock) {
-      // PressureRatio < delta_p  <=>  some neighbour's ratio < delta_p
-      const float dp_f = narrow(a.delta_p);
-      for (int k = 0; k < nn && !shock; ++k) {
-        const double np_ = point_state(a, static_cast<int>(a.geom.nbr[b + k] & kNbrIdMask)).p;
-        const bool lower = lt(np_, cell.p);
-        const double num = lower ? np_ : cell.p;
-        const double den = lower ? cell.p : np_;
-        if (fp32_safe(num) && fp32_safe(den)) {
-          const float rf = narrow(num) / narrow(den);
-          if (rf < dp_f * 0.999999f) {
+      // PressureRatio < delta_p  <=>  some neighbour's ratio < delta_p: the
+      // quad's lanes take every fourth neighbour each
+      bool dp_ok = true;
+      const float dp_f = trunc32(a.delta_p, dp_ok), pc_f = trunc32(dp.y, dp_ok);
+      for (int k = q; k < nn && !shock; k += 4) {
+        const int p = static_cast<int>(a.geom.nbr[b + k] & kNbrIdMask);
+        const double np_ = a.cells[4 * static_cast<size_t>(copied_cell(a, p)) + 1];
+        const bool lower = lt(np_, dp.y);
+        const double num = lower ? np_ : dp.y;
+        const double den = lower ? dp.y : np_;
+        // num / den against delta_p by a product: three truncations and one
+        // rounding are within 4e-7 of it (pressures are positive here: 1e-30
+        // keeps the product a normal float)
+        bool ok = dp_ok;
+        const float np_f = trunc32(np_, ok);
+        if (ok && fminf(np_f, pc_f) > 1e-30f && dp_f > 1e-6f) {
+          const float nf = fminf(np_f, pc_f), df = fmaxf(np_f, pc_f) * dp_f;
+          if (nf < df * 0.999999f) {
             shock = true;
             break;
           }
-          if (rf > dp_f * 1.000001f) continue;
+          if (nf > df * 1.000001f) continue;
         }
         shock = lt(quot(num, den), a.delta_p);
       }
+      shock = __any_sync(quad, shock);
     }
-    if (a.shock) a.shock[i] = shock ? 1 : 0;
-    // neighbour extrema as bit patterns (std::max / std::min on the integer pipe)
-    uint64_t mx[4] = {conv_dbits(cell.d), conv_dbits(cell.p), conv_dbits(cell.vx), conv_dbits(cell.vy)};
-    uint64_t mn[4] = {mx[0], mx[1], mx[2], mx[3]};
-    for (int k = 0; k < nn; ++k) {
-      const uint32_t w = a.geom.nbr[b + k];
-      if (!shock && (w & kNbrMirror)) continue;  // :194-195 skips self-mirror neighbours
-      if (skipped(a, static_cast<int>(w & kNbrIdMask))) continue;  // :192-193, :314-315 skip_key
-      const Cell nb = point_state(a, static_cast<int>(w & kNbrIdMask));
-      const uint64_t nbb[4] = {conv_dbits(nb.d), conv_dbits(nb.p), conv_dbits(nb.vx), conv_dbits(nb.vy)};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        mx[q] = max_first_u(mx[q], nbb[q]);
-        mn[q] = min_first_u(mn[q], nbb[q]);
-      }
+    if (a.shock && q == 0) a.shock[i] = shock ? 1 : 0;
+    const bool velocity = q >= 2;  // :268-283 the velocities' dead band takes |1e-9*q|
+    if (fits)
+      lane_limit<kTrace>(a, b, nn, c, sx, sy, shock, velocity, false, nb, load, psi, dphi_at, code);
+    else
+      lane_limit_any<kTrace>(a, b, nn, c, sx, sy, shock, velocity, false, load, psi, dphi_at, code);
+    if (conv_dbits(psi) != kOneBits) {
+      sx *= psi;
+      sy *= psi;
     }
-    const Cell maxd{conv_double_bits(mx[0]) - cell.d, conv_double_bits(mx[1]) - cell.p,
-                    conv_double_bits(mx[2]) - cell.vx, conv_double_bits(mx[3]) - cell.vy};
-    const Cell mind{conv_double_bits(mn[0]) - cell.d, conv_double_bits(mn[1]) - cell.p,
-                    conv_double_bits(mn[2]) - cell.vx, conv_double_bits(mn[3]) - cell.vy};
-    const double f = shock ? 0.1 : 0.05;
-    const Cell thr{f * conv_double_bits(max_first_u(abs_u(maxd.d), abs_u(mind.d))),
-                   f * conv_double_bits(max_first_u(abs_u(maxd.p), abs_u(mind.p))),
-                   f * conv_double_bits(max_first_u(abs_u(maxd.vx), abs_u(mind.vx))),
-                   f * conv_double_bits(max_first_u(abs_u(maxd.vy), abs_u(mind.vy)))};
-    uint64_t psi0 = kOneBits, psi1 = kOneBits, psi2 = kOneBits, psi3 = kOneBits;
-    float pf0 = 1, pf1 = 1, pf2 = 1, pf3 = 1;
-    for (int k = 0; k < nn; ++k) {
-      const uint32_t w = a.geom.nbr[b + k];
-      if (shock && skipped(a, static_cast<int>(w & kNbrIdMask))) continue;  // :339-340
-      const int e = m.cell_faces[b + k];
-      const double2 dm = centroid_offset(a.geom, w, e);
-      Cell cv = cell;
-      addmult(cv, sx, dm.x);
-      addmult(cv, sy, dm.y);
-      const Cell dphi{cv.d - cell.d, cv.p - cell.p, cv.vx - cell.vx, cv.vy - cell.vy};
-      if (!shock) {
-        // :174-300 slope_limit
-        limit_comp(dphi.d, cv.d, cell.d, thr.d, maxd.d, mind.d, false, psi0, pf0);
-        limit_comp(dphi.p, cv.p, cell.p, thr.p, maxd.p, mind.p, false, psi1, pf1);
-        limit_comp(dphi.vx, cv.vx, cell.vx, thr.vx, maxd.vx, mind.vx, true, psi2, pf2);
-        limit_comp(dphi.vy, cv.vy, cell.vy, thr.vy, maxd.vy, mind.vy, true, psi3, pf3);
-      } else {
-        // :302-399 shocked_slope_limit
-        const Cell nb = point_state(a, static_cast<int>(w & kNbrIdMask));
-        shocked_comp(dphi.d, cv.d, cell.d, thr.d, nb.d, a.theta, psi0, pf0);
-        shocked_comp(dphi.p, cv.p, cell.p, thr.p, nb.p, a.theta, psi1, pf1);
-        shocked_comp(dphi.vx, cv.vx, cell.vx, thr.vx, nb.vx, a.theta, psi2, pf2);
-        shocked_comp(dphi.vy, cv.vy, cell.vy, thr.vy, nb.vy, a.theta, psi3, pf3);
-      }
-    }
-    const double p0 = conv_double_bits(psi0), p1 = conv_double_bits(psi1), p2 = conv_double_bits(psi2),
-                 p3 = conv_double_bits(psi3);
-    sx.d *= p0; sy.d *= p0;
-    sx.p *= p1; sy.p *= p1;
-    sx.vx *= p2; sy.vx *= p2;
-    sx.vy *= p3; sy.vy *= p3;
   }
-  double2* o = reinterpret_cast<double2*>(a.slopes) + 4 * i;
-  o[0] = make_double2(sx.d, sx.p);
-  o[1] = make_double2(sx.vx, sx.vy);
-  o[2] = make_double2(sy.d, sy.p);
-  o[3] = make_double2(sy.vx, sy.vy);
+  double* o = a.slopes + 8 * static_cast<size_t>(i) + q;
+  o[0] = sx;
+  o[4] = sy;
+  if (kTrace) {
+    SlopeTrace& tr = trace[i];
+    tr.naive[q] = nsx;
+    tr.naive[4 + q] = nsy;
+    tr.psi[q] = psi;
+    tr.dphi[q] = dphi_at;
+    tr.code[q] = code;
+  }
 }
 
-// kMinBlocks > 0: register-capped builds for blocks of up to kCappedBlock
-// threads with kMinBlocks resident per SM (launch-shape variants 2 and 3)
-template <bool kBatch, int kMinBlocks = 0>
+// Four lanes per cell (an item).  kMinBlocks > 0: register-capped builds for
+// blocks of up to kCappedBlock threads with kMinBlocks resident per SM
+// (launch-shape variants 2 and 3)
+template <bool kBatch, int kMinBlocks = 0, bool kTrace = false>
 __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 1)
-    k_slopes(StepArgs a) {
+    k_slopes(StepArgs a, SlopeTrace* trace) {
   // the dt of this step, computed by the previous step's update (the face
   // kernel, launched after this one, reads status->dt)
   if (a.take_next_dt && blockIdx.x == 0 && threadIdx.x == 0) a.status->dt = a.status->dt_next;
   const int* order = a.geom.cell_order;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < a.mesh.n; t += gridDim.x * blockDim.x)
-    k_slopes_item<kBatch>(a, order ? order[t] : t);
+  const int q = threadIdx.x & 3;
+  const unsigned quad = 0xfu << (threadIdx.x & 28);
+  for (long long t = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 2; t < a.mesh.n;
+       t += (gridDim.x * static_cast<long long>(blockDim.x)) >> 2)
+    slopes_lane<kBatch, kTrace>(a, order ? order[t] : static_cast<int>(t), q, quad, trace);
 }
 
 // ---------------------------------------------------------------- faces
@@ -1100,16 +1056,21 @@ cudaError_t launch_ghost_fill(const StepArgs& a, cudaStream_t s) {
 cudaError_t launch_slopes(const StepArgs& a, cudaStream_t s) {
   if (a.mesh.n > 0) {
     const LaunchShape& sh = a.shapes.slopes;
-    const int nb = grid_of(sh, a.mesh.n), bs = sh.block;
+    const int nb = grid_of(sh, 4LL * a.mesh.n), bs = sh.block;
     const bool b = a.cell_problem != nullptr;
     // builds: 0 plain, 2 and 3 register-capped for 3 and 4 resident blocks of
     // up to 256 threads
     switch (sh.variant) {
-      case 2: b ? k_slopes<true, 3><<<nb, bs, 0, s>>>(a) : k_slopes<false, 3><<<nb, bs, 0, s>>>(a); break;
-      case 3: b ? k_slopes<true, 4><<<nb, bs, 0, s>>>(a) : k_slopes<false, 4><<<nb, bs, 0, s>>>(a); break;
-      default: b ? k_slopes<true><<<nb, bs, 0, s>>>(a) : k_slopes<false><<<nb, bs, 0, s>>>(a);
+      case 2: b ? k_slopes<true, 3><<<nb, bs, 0, s>>>(a, nullptr) : k_slopes<false, 3><<<nb, bs, 0, s>>>(a, nullptr); break;
+      case 3: b ? k_slopes<true, 4><<<nb, bs, 0, s>>>(a, nullptr) : k_slopes<false, 4><<<nb, bs, 0, s>>>(a, nullptr); break;
+      default: b ? k_slopes<true><<<nb, bs, 0, s>>>(a, nullptr) : k_slopes<false><<<nb, bs, 0, s>>>(a, nullptr);
     }
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_slopes_trace(const StepArgs& a, SlopeTrace* trace, cudaStream_t s) {
+  if (a.mesh.n > 0) k_slopes<false, 0, true><<<grid_of(kDefaultShape, 4LL * a.mesh.n), kDefaultShape.block, 0, s>>>(a, trace);
   return cudaGetLastError();
 }
 

@@ -78,6 +78,7 @@ struct GeomDev {
   // per CSR entry
   const uint32_t* nbr;
   const double2* hr;     // naive: 0.5*r_ij; boundary: cm[other] - cm[cell]
+  const float2* dmf;     // CalcCentroid(face) - cm[cell], rounded (the limiter's FP32 screen; dm_screen)
   // per ghost
   const int* ghost_real;      // cell whose state the ghost copies / reflects
   const double2* ghost_unit;  // rigid wall: unit normal (x_ghost - x_real)/|.|
@@ -211,8 +212,8 @@ struct LaunchShape {
 };
 constexpr LaunchShape kDefaultShape{256, 0, 0};
 constexpr int kCappedBlock = 256;
-inline int grid_of(const LaunchShape& s, int items) {
-  const int need = items > 0 ? (items + s.block - 1) / s.block : 1;
+inline int grid_of(const LaunchShape& s, long long items) {
+  const int need = items > 0 ? static_cast<int>((items + s.block - 1) / s.block) : 1;
   return s.max_blocks > 0 && need > s.max_blocks ? s.max_blocks : need;
 }
 // per-step kernels of one path (FP64 or FP32-mixed)
@@ -378,6 +379,7 @@ struct GeomArgs {
   int* cflags;
   uint32_t* nbr;
   double2* hr;
+  float2* dmf;
   int* ghost_real;
   double2* ghost_unit;
   int* cell_order;
@@ -395,6 +397,9 @@ cudaError_t launch_geom_ghosts(const GeomArgs& a, cudaStream_t s);  // the ghost
 cudaError_t launch_cfl(const StepArgs& a, cudaStream_t s, bool fill_ghosts);
 cudaError_t launch_ghost_fill(const StepArgs& a, cudaStream_t s);
 cudaError_t launch_slopes(const StepArgs& a, cudaStream_t s);
+// the slopes with the adjoint's limiter trace (periodic meshes, one problem)
+struct SlopeTrace;
+cudaError_t launch_slopes_trace(const StepArgs& a, SlopeTrace* trace, cudaStream_t s);
 cudaError_t launch_faces(const StepArgs& a, cudaStream_t s, bool scaled);
 cudaError_t launch_update(const StepArgs& a, cudaStream_t s, bool from_unscaled, bool extensive, bool cells);
 cudaError_t launch_init_extensives(const StepArgs& a, cudaStream_t s);

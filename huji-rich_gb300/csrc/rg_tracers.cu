@@ -16,163 +16,65 @@
 //                 extensive / mass and the "Entropy" tracer
 //                 (simple_cell_updater.cpp:22-59), or the old tracers of a
 //                 SkipUpdate cell
-// Tracers are cell-major (cell i's tracer j at i*nt + j).  The per-cell
-// kernels are instantiated for each tracer count NT (1..kMaxTracers) so their
-// loops over tracers have exact compile-time bounds: the per-cell arrays stay
-// in registers and no FP64 work is spent on absent tracers.
+// Tracers are cell-major (cell i's tracer j at i*nt + j).  k_tr_update is
+// instantiated for each tracer count NT (1..kMaxTracers) so its loops over
+// tracers have exact compile-time bounds: the per-cell arrays stay in
+// registers and no FP64 work is spent on absent tracers.
 #include <math.h>
 
-#include "rg_fp64.cuh"
+#include "rg_lgi.cuh"
 
 namespace rg {
 namespace {
 
 constexpr int kTrBlock = 256;
 
-__device__ __forceinline__ const double* tracers_of(const StepArgs& a, const TracerArgs& t, int p) {
-  return t.tr + static_cast<size_t>(copied_cell(a, p)) * t.nt;
-}
 
-// LinearGaussImproved.cpp:425-494 calc_slope, tracer part, for cell i.
-template <int NT>
+// LinearGaussImproved.cpp:425-494 calc_slope, tracer part: one thread per
+// tracer of a cell (the hydro slopes' lanes, rg_lgi.cuh), cells in the
+// per-tile neighbour-count order.  Tracers share only the geometry and the
+// shock decision, which the hydro pass kept.
 __global__ void __launch_bounds__(kTrBlock) k_tr_slopes(StepArgs a, TracerArgs t) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const long long id = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const MeshDev& m = a.mesh;
-  if (i >= m.n) return;
-  constexpr int nt = NT;
-  constexpr int kMaxTracers = NT;
+  const int nt = t.nt;
+  const int at = static_cast<int>(id / nt), j = static_cast<int>(id % nt);
+  if (at >= m.n) return;
+  const int i = a.geom.cell_order ? a.geom.cell_order[at] : at;
+  double* o = t.tr_slopes + static_cast<size_t>(i) * 2 * nt + j;
+  if (!((t.limited >> j) & 1u)) {
+    // :470-479 tracers outside calc_tracers get zero slopes
+    o[0] = 0.0;
+    o[nt] = 0.0;
+    return;
+  }
+  const TracerComp load{a, t.tr, nt, j};
+  const double c = load.at(i);
   const int b = m.cell_off[i], nn = m.cell_off[i + 1] - b;
-  const dbl4 mi = a.geom.minv[i];
-  double ct[kMaxTracers], sx[kMaxTracers], sy[kMaxTracers];
-#pragma unroll
-  for (int j = 0; j < kMaxTracers; ++j) {
-    ct[j] = j < nt ? t.tr[static_cast<size_t>(i) * nt + j] : 0.0;
-    sx[j] = sy[j] = 0.0;
-  }
-  if (a.geom.cflags[i] & kCellBoundarySlope) {
-    // :401-422 GetBoundarySlope: PhiS += (nb - cell)*(cm_nb - cm_cell)
-    double py[kMaxTracers], px[kMaxTracers];
-#pragma unroll
-    for (int j = 0; j < kMaxTracers; ++j) py[j] = px[j] = 0.0;
-    for (int k = 0; k < nn; ++k) {
-      const double* nb = tracers_of(a, t, static_cast<int>(a.geom.nbr[b + k] & kNbrIdMask));
-      const double2 h = a.geom.hr[b + k];
-#pragma unroll
-      for (int j = 0; j < kMaxTracers; ++j) {
-        if (j < nt) {
-          const double df = nb[j] - ct[j];
-          py[j] = py[j] + df * h.y;
-          px[j] = px[j] + df * h.x;
-        }
-      }
-    }
-    const double sxsy = mi.x, sx2 = mi.y, sy2 = mi.z, den = mi.w;
-#pragma unroll
-    for (int j = 0; j < kMaxTracers; ++j) {
-      sx[j] = quot(py[j] * sxsy - px[j] * sy2, den);
-      sy[j] = quot(px[j] * sxsy - py[j] * sx2, den);
-    }
+  const bool boundary = a.geom.cflags[i] & kCellBoundarySlope;
+  const bool fits = nn <= kFit;
+  LaneNeighbours nb;
+  double sx, sy;
+  if (fits) {
+    lane_load(a, b, nn, load, nb);
+    lane_slope(a, i, b, nn, boundary, c, nb, sx, sy);
   } else {
-    // :80-133 calc_naive_slope with the mesh's 0.5*r_ij and inverse matrix
-    double vx[kMaxTracers], vy[kMaxTracers];
-#pragma unroll
-    for (int j = 0; j < kMaxTracers; ++j) vx[j] = vy[j] = 0.0;
-    for (int k = 0; k < nn; ++k) {
-      const double* nb = tracers_of(a, t, static_cast<int>(a.geom.nbr[b + k] & kNbrIdMask));
-      const double2 h = a.geom.hr[b + k];
-#pragma unroll
-      for (int j = 0; j < kMaxTracers; ++j) {
-        if (j < nt) {
-          if (k == 0) {
-            vx[j] = ct[j] * h.x;
-            vy[j] = ct[j] * h.y;
-          } else {
-            vx[j] += ct[j] * h.x;
-            vy[j] += ct[j] * h.y;
-          }
-          const double q = nb[j];
-          vy[j] += q * h.y;
-          vx[j] += q * h.x;
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kMaxTracers; ++j) {
-      sx[j] = vx[j] * mi.x;
-      sy[j] = vy[j] * mi.w;
-      sx[j] += vy[j] * mi.y;
-      sy[j] += vx[j] * mi.z;
-    }
+    lane_slope_any(a, i, b, nn, boundary, c, load, sx, sy);
   }
-  // :470-479 tracers outside calc_tracers get zero slopes
-#pragma unroll
-  for (int j = 0; j < kMaxTracers; ++j)
-    if (!((t.limited >> j) & 1u)) sx[j] = sy[j] = 0.0;
   if (a.slf) {
+    // both limiters take |1e-9*t| (:268-283, :367-385)
     const bool shock = a.shock[i] != 0;
-    uint64_t cmax[kMaxTracers], cmin[kMaxTracers];  // bit patterns
-#pragma unroll
-    for (int j = 0; j < kMaxTracers; ++j) cmax[j] = cmin[j] = conv_dbits(ct[j]);
-    for (int k = 0; k < nn; ++k) {
-      const uint32_t w = a.geom.nbr[b + k];
-      if (!shock && (w & kNbrMirror)) continue;  // :194-195
-      if (skipped(a, static_cast<int>(w & kNbrIdMask))) continue;
-      const double* nb = tracers_of(a, t, static_cast<int>(w & kNbrIdMask));
-#pragma unroll
-      for (int j = 0; j < kMaxTracers; ++j) {
-        if (j < nt) {
-          cmax[j] = max_first_u(cmax[j], conv_dbits(nb[j]));
-          cmin[j] = min_first_u(cmin[j], conv_dbits(nb[j]));
-        }
-      }
-    }
-    const double f = shock ? 0.1 : 0.05;
-    double maxd[kMaxTracers], mind[kMaxTracers], thr[kMaxTracers];
-    uint64_t psi[kMaxTracers];
-    float pf[kMaxTracers];
-#pragma unroll
-    for (int j = 0; j < kMaxTracers; ++j) {
-      maxd[j] = conv_double_bits(cmax[j]) - ct[j];
-      mind[j] = conv_double_bits(cmin[j]) - ct[j];
-      thr[j] = f * conv_double_bits(max_first_u(abs_u(maxd[j]), abs_u(mind[j])));
-      psi[j] = kOneBits;
-      pf[j] = 1.0f;
-    }
-    for (int k = 0; k < nn; ++k) {
-      const uint32_t w = a.geom.nbr[b + k];
-      const int other = static_cast<int>(w & kNbrIdMask);
-      if (shock && skipped(a, other)) continue;  // :339-340
-      const int e = m.cell_faces[b + k];
-      const double2 dm = centroid_offset(a.geom, w, e);
-      const double* nb = tracers_of(a, t, other);
-#pragma unroll
-      for (int j = 0; j < kMaxTracers; ++j) {
-        if (j < nt) {
-          double cv = ct[j];
-          cv += sx[j] * dm.x;
-          cv += sy[j] * dm.y;
-          const double dphi = cv - ct[j];
-          if (!shock)
-            limit_comp(dphi, cv, ct[j], thr[j], maxd[j], mind[j], true, psi[j], pf[j]);  // :268-283
-          else
-            shocked_comp(dphi, cv, ct[j], thr[j], nb[j], a.theta, psi[j], pf[j], true);  // :367-385
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kMaxTracers; ++j) {
-      sx[j] *= conv_double_bits(psi[j]);
-      sy[j] *= conv_double_bits(psi[j]);
-    }
+    double psi, dphi_at;
+    int code;
+    if (fits)
+      lane_limit<false>(a, b, nn, c, sx, sy, shock, true, true, nb, load, psi, dphi_at, code);
+    else
+      lane_limit_any<false>(a, b, nn, c, sx, sy, shock, true, true, load, psi, dphi_at, code);
+    sx *= psi;
+    sy *= psi;
   }
-  double* o = t.tr_slopes + static_cast<size_t>(i) * 2 * nt;
-#pragma unroll
-  for (int j = 0; j < kMaxTracers; ++j) {
-    if (j < nt) {
-      o[j] = sx[j];
-      o[nt + j] = sy[j];
-    }
-  }
+  o[0] = sx;
+  o[nt] = sy;
 }
 
 // dt*area of face e (simple_extensive_updater.cpp:26-27); in a batch the dt
@@ -391,7 +293,8 @@ inline int tr_blocks(int n) { return (n + kTrBlock - 1) / kTrBlock; }
 
 cudaError_t launch_tr_slopes(const StepArgs& a, const TracerArgs& t, cudaStream_t s) {
   if (a.mesh.n > 0 && t.nt > 0 && t.nt <= kMaxTracers) {
-    RG_TR_DISPATCH(k_tr_slopes, tr_blocks(a.mesh.n), s, a, t)
+    const long long lanes = static_cast<long long>(a.mesh.n) * t.nt;
+    k_tr_slopes<<<static_cast<unsigned>((lanes + kTrBlock - 1) / kTrBlock), kTrBlock, 0, s>>>(a, t);
   }
   return cudaGetLastError();
 }
