@@ -212,6 +212,25 @@ __global__ void __launch_bounds__(kBlock) k3_update(Step3Args a, int from_unscal
   }
 }
 
+// Records of 5 doubles (the host's) <-> 6 (the device's, the last one 0), one
+// value per thread, coalesced on both sides.  The copies between host and
+// device then move one contiguous block: a pitched copy of 40-byte rows runs
+// at 3.8 GB/s host to device (35 MB, the 96^3 cells: 9.25 ms; 0.19 ms as one
+// block at 190 GB/s plus 18 us here).
+__global__ void __launch_bounds__(kBlock) k3_unpack(const double* packed, double* rec, int rows) {
+  const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  if (t >= 6LL * rows) return;
+  const long long r = t / 6;
+  const int q = static_cast<int>(t - 6 * r);
+  rec[t] = q < 5 ? packed[5 * r + q] : 0.0;
+}
+__global__ void __launch_bounds__(kBlock) k3_pack(const double* rec, double* packed, int rows) {
+  const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  if (t >= 5LL * rows) return;
+  const long long r = t / 5;
+  packed[t] = rec[6 * r + (t - 5 * r)];
+}
+
 __global__ void __launch_bounds__(kBlock) k3_init(Step3Args a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.mesh.n) return;
@@ -222,9 +241,18 @@ __global__ void __launch_bounds__(kBlock) k3_init(Step3Args a) {
   store6(a.ext, i, V * c.d, mom.x * V, mom.y * V, mom.z * V, V * en);
 }
 
-inline int blocks(int n) { return n > 0 ? (n + kBlock - 1) / kBlock : 1; }
+inline int blocks(long long n) { return n > 0 ? static_cast<int>((n + kBlock - 1) / kBlock) : 1; }
 
 }  // namespace
+
+cudaError_t launch3_unpack(const double* packed, double* rec, int rows, cudaStream_t s) {
+  k3_unpack<<<blocks(6LL * rows), kBlock, 0, s>>>(packed, rec, rows);
+  return cudaGetLastError();
+}
+cudaError_t launch3_pack(const double* rec, double* packed, int rows, cudaStream_t s) {
+  k3_pack<<<blocks(5LL * rows), kBlock, 0, s>>>(rec, packed, rows);
+  return cudaGetLastError();
+}
 
 cudaError_t launch3_validate(const Mesh3Dev& m, DevStatus* st, cudaStream_t s) {
   k3_validate<<<blocks(m.e > m.n ? m.e : m.n), kBlock, 0, s>>>(m, st);

@@ -75,6 +75,9 @@ cudaError_t launch3m_cfl(const Mixed3Args& a, cudaStream_t s);
 cudaError_t launch3m_faces(const Mixed3Args& a, bool scaled, cudaStream_t s);
 cudaError_t launch3m_update(const Mixed3Args& a, bool from_unscaled, bool do_ext, bool do_cells, cudaStream_t s);
 
+// 5-double records (the host's) to and from the 6-double ones
+cudaError_t launch3_unpack(const double* packed, double* rec, int rows, cudaStream_t s);
+cudaError_t launch3_pack(const double* rec, double* packed, int rows, cudaStream_t s);
 cudaError_t launch3_validate(const Mesh3Dev& m, DevStatus* st, cudaStream_t s);
 cudaError_t launch3_geometry(const Mesh3Dev& m, dbl4* nhat, int* fsign, cudaStream_t s);
 cudaError_t launch3_init_extensives(const Step3Args& a, cudaStream_t s);

@@ -1,8 +1,8 @@
 // rg_3d_api.cu -- C ABI of the 3D first-order path (rg3_* in
 // include/rich_gb300.h): a handle owning the packed 3D mesh (validated on the
 // device before use), the cell / extensive state and the face fluxes, all on
-// one stream.  Host records of 5 doubles are moved to and from the device's
-// 48-byte records with pitched copies.
+// one stream.  Host records of 5 doubles are moved as one block through a
+// device staging buffer and repacked to the 48-byte records there.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -44,6 +44,7 @@ struct rg3_handle {
   bool have_mesh = false, have_cells = false, have_ext = false, have_fluxes = false;
   Buf face_cells, normal, area, volume, width, cell_off, cell_faces, nhat, fsign;
   Buf cells, ext, fluxes, fvel, status_buf;
+  Buf stage;  // 5-double records on their way to or from the host
   bool fvel_set = false;
   // FP32-mixed path (rg_config.precision == RG_FP32_MIXED)
   bool mixed = false;
@@ -146,16 +147,34 @@ rg_status sync_cells64(rg3_handle* h) {
   return RG_OK;
 }
 
-// 5-double host records <-> 6-double device records
+// 5-double host records <-> 6-double device records, through the staging
+// buffer; where there is no memory for it, by a (slow) pitched copy.
+bool staged(rg3_handle* h, int rows) {
+  if (h->stage.ensure(40 * static_cast<size_t>(rows)) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
 rg_status put5(rg3_handle* h, Buf& dst, const double* src, int rows) {
-  RG3_CUDA(h, cudaMemcpy2DAsync(dst.p, 48, src, 40, 40, static_cast<size_t>(rows), cudaMemcpyHostToDevice,
-                                h->stream));
+  if (staged(h, rows)) {
+    RG3_CUDA(h, cudaMemcpyAsync(h->stage.p, src, 40 * static_cast<size_t>(rows), cudaMemcpyHostToDevice, h->stream));
+    RG3_CUDA(h, rg::launch3_unpack(static_cast<const double*>(h->stage.p), static_cast<double*>(dst.p), rows,
+                                   h->stream));
+  } else {
+    RG3_CUDA(h, cudaMemcpy2DAsync(dst.p, 48, src, 40, 40, static_cast<size_t>(rows), cudaMemcpyHostToDevice,
+                                  h->stream));
+  }
   RG3_CUDA(h, cudaStreamSynchronize(h->stream));
   return RG_OK;
 }
 rg_status get5(rg3_handle* h, double* dst, const Buf& src, int rows) {
-  RG3_CUDA(h, cudaMemcpy2DAsync(dst, 40, src.p, 48, 40, static_cast<size_t>(rows), cudaMemcpyDeviceToHost,
-                                h->stream));
+  if (staged(h, rows)) {
+    RG3_CUDA(h, rg::launch3_pack(static_cast<const double*>(src.p), static_cast<double*>(h->stage.p), rows,
+                                 h->stream));
+    RG3_CUDA(h, cudaMemcpyAsync(dst, h->stage.p, 40 * static_cast<size_t>(rows), cudaMemcpyDeviceToHost, h->stream));
+  } else {
+    RG3_CUDA(h, cudaMemcpy2DAsync(dst, 40, src.p, 48, 40, static_cast<size_t>(rows), cudaMemcpyDeviceToHost,
+                                  h->stream));
+  }
   RG3_CUDA(h, cudaStreamSynchronize(h->stream));
   return RG_OK;
 }
@@ -233,7 +252,7 @@ rg_status rg3_destroy(rg3_handle* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (Buf* b : {&h->face_cells, &h->normal, &h->area, &h->volume, &h->width, &h->cell_off, &h->cell_faces,
                  &h->nhat, &h->fsign, &h->cells, &h->ext, &h->fluxes, &h->fvel, &h->status_buf, &h->nhat32,
-                 &h->area32, &h->width32, &h->cells32, &h->vz32, &h->flux32, &h->fen32, &h->fvel32})
+                 &h->area32, &h->width32, &h->cells32, &h->vz32, &h->flux32, &h->fen32, &h->fvel32, &h->stage})
     b->release();
   if (h->h_status) cudaFreeHost(h->h_status);
   for (cudaEvent_t& v : h->ev)
@@ -279,6 +298,7 @@ rg_status rg3_upload_mesh(rg3_handle* h, const rg_mesh3d_view* v) {
   RG3_CUDA(h, h->fvel.ensure(24 * E));
   if (n != h->n) h->have_cells = h->have_ext = false;
   RG3_CUDA(h, h->cells.ensure(48 * N));
+  staged(h, n);  // set-up time, not the first transfer's
   RG3_CUDA(h, h->ext.ensure(48 * N));
   RG3_CUDA(h, cudaMemcpyAsync(h->face_cells.p, v->face_cells, 8 * E, cudaMemcpyHostToDevice, h->stream));
   RG3_CUDA(h, cudaMemcpyAsync(h->normal.p, v->face_normal, 24 * E, cudaMemcpyHostToDevice, h->stream));
