@@ -179,6 +179,7 @@ rg::StepArgs step_args(rg_handle* h) {
   a.mesh = s->mesh;
   a.geom = s->geom;
   a.gamma = h->cfg.gamma;
+  a.gm1 = rg::divisor(h->cfg.gamma - 1, rg::RcpSeedHost{});
   a.cfl = h->cfg.cfl;
   a.order = h->cfg.order;
   a.ghost_kind = h->cfg.ghost_kind;
@@ -650,10 +651,13 @@ rg_status rg_create(const rg_config* cfg, rg_handle** out) {
   if (!h) return RG_ERR_OUT_OF_MEMORY;
   h->cfg = *cfg;
   h->mixed = cfg->precision == RG_FP32_MIXED;
-  // the FP64 slopes: the build for three resident blocks of 256 (80 registers),
-  // in blocks of 128 (512^2: 197 us; 245 us as the plain build in blocks of 256,
-  // whose 106 registers leave 16 warps per SM and a coarse last wave)
-  h->shapes64.slopes = rg::LaunchShape{128, 0, 2};
+  // the FP64 slopes: the build for four resident blocks of 256 (64 registers).
+  // Bound by the FP64 unit's latency and issue, they gain from every warp
+  // (512^2: 172 us; 179 us with three resident blocks, 211 us as the plain
+  // build's two)
+  h->shapes64.slopes = rg::LaunchShape{256, 0, 3};
+  // the FP64 faces in blocks of 512 (k_faces)
+  h->shapes64.faces = rg::LaunchShape{512, 0, 0};
   h->heun = cfg->time_integrator == RG_TIME_ADVANCE_HEUN;
   auto fail = [&](cudaError_t e) {
     rg_destroy(h);

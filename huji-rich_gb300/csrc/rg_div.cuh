@@ -155,6 +155,9 @@ constexpr uint64_t kSign = uint64_t(1) << 63;
 }  // namespace div_detail
 
 // The FP32 reciprocal approximation of the device (the seed of step 2).
+struct RcpSeedHost {
+  float operator()(float f) const { return 1.0f / f; }
+};
 struct RcpSeedDevice {
 #if defined(__CUDACC__)
   __device__ __forceinline__ float operator()(float f) const {
@@ -165,46 +168,63 @@ struct RcpSeedDevice {
 #endif
 };
 
-// a / b on the fast path; returns false (and leaves *q) where the operands are
-// outside it.  Seed: a callable float -> float approximating 1/f on [1, 2).
+// A divisor prepared for several quotients: steps 2 of the method, which only
+// read b.  ok: b is normal and the seed within its bound.
+struct Divisor {
+  uint64_t mb, R1;
+  float r0;
+  uint32_t eb;    // exponent field
+  uint32_t sign;  // the sign bit of the high word
+  bool ok;
+};
 template <class Seed>
-RG_DIV_FN bool div_rn_fast(double a, double b, const Seed& seed, double* q) {
+RG_DIV_FN Divisor divisor(double b, const Seed& seed) {
   using namespace div_detail;
-  const uint64_t ua = d2u(a), ub = d2u(b);
-  const uint32_t ea = static_cast<uint32_t>(ua >> 52) & 0x7ffu, eb = static_cast<uint32_t>(ub >> 52) & 0x7ffu;
-  const uint64_t sign = (ua ^ ub) & kSign;
-  if (eb - 1u >= 2046u) return false;  // b zero, subnormal, infinite or NaN
-  if (ea == 0u && (ua & kFrac) == 0u) {
-    *q = u2d(sign);  // +-0 / normal
-    return true;
-  }
-  const int d = static_cast<int>(ea) - static_cast<int>(eb);
-  if (ea - 1u >= 2046u || d < -1021 || d > 1022) return false;  // a subnormal / special, quotient not normal
-  const uint64_t ma = (ua & kFrac) | kHidden, mb = (ub & kFrac) | kHidden;
-  const uint32_t borrow = ma < mb ? 1u : 0u;
-  const uint64_t A = ma << borrow;
-  // step 2: seed and one float-float Newton step
-  const float f_hi = u2f(0x3f800000u | static_cast<uint32_t>((mb & kFrac) >> 29));
-  const float f_lo = mul32(static_cast<float>(static_cast<uint32_t>(mb & 0x1fffffffu)), 2.220446049250313e-16f);
-  const float r0 = seed(f_hi);
-  float e = fma32(-f_hi, r0, 1.0f);
-  e = fma32(-f_lo, r0, e);
-  if (!(e <= 2.384185791015625e-07f && e >= -2.384185791015625e-07f)) return false;  // |e| <= 2^-22
-  const float c = mul32(r0, e);
+  Divisor D;
+  const uint64_t ub = d2u(b);
+  D.eb = static_cast<uint32_t>(ub >> 52) & 0x7ffu;
+  D.sign = static_cast<uint32_t>(ub >> 32) & 0x80000000u;
+  D.mb = (ub & kFrac) | kHidden;
+  // seed and one float-float Newton step
+  const float f_hi = u2f(0x3f800000u | static_cast<uint32_t>((D.mb & kFrac) >> 29));
+  const float f_lo = mul32(static_cast<float>(static_cast<uint32_t>(D.mb & 0x1fffffffu)), 2.220446049250313e-16f);
+  D.r0 = seed(f_hi);
+  float e = fma32(-f_hi, D.r0, 1.0f);
+  e = fma32(-f_lo, D.r0, e);
+  // b normal, |e| <= 2^-22
+  D.ok = D.eb - 1u < 2046u && e <= 2.384185791015625e-07f && e >= -2.384185791015625e-07f;
+  const float c = mul32(D.r0, e);
   // r0 in [0.25, 1] (the test above fails otherwise): r0 * 2^25 is an integer
   // below 2^26; |c| < 2^-21.9, so |c * 2^50| < 2^29
-  const uint32_t r0i = f2u_int(mul32(r0, 33554432.0f));
+  const uint32_t r0i = f2u_int(mul32(D.r0, 33554432.0f));
   const int32_t ci = f2i_rn(mul32(c, 1125899906842624.0f));
-  const uint64_t R1 = (static_cast<uint64_t>(r0i) << 38) + static_cast<uint64_t>(static_cast<int64_t>(ci) * 8192);
+  D.R1 = (static_cast<uint64_t>(r0i) << 38) + static_cast<uint64_t>(static_cast<int64_t>(ci) * 8192);
+  return D;
+}
+
+// a / b for the divisor b; returns false (*q is then meaningless) where the
+// operands are outside the fast path.
+RG_DIV_FN bool div_by(double a, const Divisor& D, double* q) {
+  using namespace div_detail;
+  const uint64_t ua = d2u(a);
+  const uint32_t ahi = static_cast<uint32_t>(ua >> 32);
+  const uint32_t ea = (ahi >> 20) & 0x7ffu;
+  const uint32_t sign = (ahi & 0x80000000u) ^ D.sign;
+  const bool zero = ((ahi << 1) | static_cast<uint32_t>(ua)) == 0u;  // +-0 / normal is +-0
+  const int d = static_cast<int>(ea) - static_cast<int>(D.eb);
+  const bool in = ea - 1u < 2046u && d >= -1021 && d <= 1022;  // a normal, the quotient normal
+  const uint64_t ma = (ua & kFrac) | kHidden, mb = D.mb;
+  const uint32_t borrow = ma < mb ? 1u : 0u;
+  const uint64_t A = ma << borrow;
   // step 3: quotient estimate from three 32 x 32-bit products
   const uint64_t X = A << 1;
   const uint32_t x1 = static_cast<uint32_t>(X >> 32), x0 = static_cast<uint32_t>(X);
-  const uint32_t y1 = static_cast<uint32_t>(R1 >> 32), y0 = static_cast<uint32_t>(R1);
+  const uint32_t y1 = static_cast<uint32_t>(D.R1 >> 32), y0 = static_cast<uint32_t>(D.R1);
   const uint64_t Q0 = static_cast<uint64_t>(x1) * y1 + mulhi32(x1, y0) + mulhi32(x0, y1);
   // step 4: exact remainder (modulo 2^64)
   const int64_t R = static_cast<int64_t>((A << 52) - mb * Q0);
   // step 5: nearest integer to R / Mb (|R / Mb| < 910; R >> 32 fits 31 bits)
-  const int32_t k = f2i_rn(mul32(mul32(static_cast<float>(static_cast<int32_t>(R >> 32)), r0), 9.5367431640625e-07f));
+  const int32_t k = f2i_rn(mul32(mul32(static_cast<float>(static_cast<int32_t>(R >> 32)), D.r0), 9.5367431640625e-07f));
   const int64_t R2 = R - static_cast<int64_t>(k) * static_cast<int64_t>(mb);
   // step 6: round to nearest
   const int64_t twice = R2 * 2;
@@ -212,8 +232,17 @@ RG_DIV_FN bool div_rn_fast(double a, double b, const Seed& seed, double* q) {
   const uint64_t Q = Q0 + static_cast<uint64_t>(static_cast<int64_t>(k)) + (twice > m ? 1u : 0u) -
                      (twice < -m ? 1u : 0u);
   // exponent field d + 1023 - borrow; Q's hidden bit (or Q = 2^53) adds to it
-  *q = u2d(sign | ((static_cast<uint64_t>(d + 1022 - static_cast<int>(borrow)) << 52) + Q));
-  return true;
+  const uint64_t r = (static_cast<uint64_t>(static_cast<uint32_t>(d + 1022 - static_cast<int>(borrow))) << 52) + Q;
+  *q = u2d(zero ? static_cast<uint64_t>(sign) << 32 : (static_cast<uint64_t>(sign) << 32) | r);
+  return D.ok && (in || zero);
+}
+
+// a / b on the fast path; returns false (*q is then meaningless) where the
+// operands are outside it.  Seed: a callable float -> float approximating 1/f
+// on [1, 2).
+template <class Seed>
+RG_DIV_FN bool div_rn_fast(double a, double b, const Seed& seed, double* q) {
+  return div_by(a, divisor(b, seed), q);
 }
 
 // The FP32 reciprocal square root approximation of the device (the seed of sqrt_rn_fast).
@@ -228,7 +257,7 @@ struct RsqrtSeedDevice {
 };
 
 // sqrt(x) correctly rounded on the fast path (x a positive normal double or
-// a zero); returns false (and leaves *r) otherwise.  Seed: a callable float
+// a zero); returns false (*r is then meaningless) otherwise.  Seed: a callable float
 // -> float approximating 1/sqrt(f) on [1, 4).  With Mx the 53-bit
 // significand, x = m * 2^E, m = Mx * 2^(odd - 52) in [1, 4), E even, the
 // result significand is S = nearest integer to sqrt(N), N = Mx * 2^(52 + odd):
@@ -249,12 +278,9 @@ template <class Seed>
 RG_DIV_FN bool sqrt_rn_fast(double x, const Seed& seed, double* r) {
   using namespace div_detail;
   const uint64_t ux = d2u(x);
-  if ((ux & ~kSign) == 0u) {
-    *r = x;  // sqrt(+-0) = +-0
-    return true;
-  }
+  const bool zero = (ux & ~kSign) == 0u;                // sqrt(+-0) = +-0
   const uint32_t ex = static_cast<uint32_t>(ux >> 52);  // with the sign: negative x is out of range
-  if (ex - 1u >= 2046u) return false;                   // negative, subnormal, infinite or NaN
+  const bool in = ex - 1u < 2046u;                      // else negative, subnormal, infinite or NaN
   const uint32_t odd = (ex & 1u) ^ 1u;                  // ex - 1023 odd
   const uint64_t mx = (ux & kFrac) | kHidden;
   // step 1 (f in [1, 4); the low part is the 29 bits below f's significand)
@@ -263,7 +289,7 @@ RG_DIV_FN bool sqrt_rn_fast(double x, const Seed& seed, double* r) {
                            odd ? 4.440892098500626e-16f : 2.220446049250313e-16f);
   const float y = seed(f);
   const float e = fma32(-f, mul32(y, y), 1.0f);
-  if (!(e <= 4.76837158203125e-07f && e >= -4.76837158203125e-07f)) return false;  // |e| <= 2^-21
+  const bool ok = e <= 4.76837158203125e-07f && e >= -4.76837158203125e-07f;  // |e| <= 2^-21
   const float s0 = mul32(f, y);
   const float p = mul32(s0, s0);
   const float pe = fma32(s0, s0, -p);
@@ -289,8 +315,8 @@ RG_DIV_FN bool sqrt_rn_fast(double x, const Seed& seed, double* r) {
   const uint64_t S = S2 + (R > s2 ? 1u : 0u) - (R <= -s2 ? 1u : 0u);
   // exponent field E/2 + 1023 (E = ex - 1023 - odd, even); S's hidden bit adds the one
   const int field = (static_cast<int>(ex) - static_cast<int>(odd) - 1023) / 2 + 1022;
-  *r = u2d((static_cast<uint64_t>(field) << 52) + S);
-  return true;
+  *r = u2d(zero ? ux : (static_cast<uint64_t>(field) << 52) + S);
+  return (in && ok) || zero;
 }
 
 #if defined(__CUDACC__)

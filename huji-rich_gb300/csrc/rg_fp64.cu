@@ -18,6 +18,7 @@
 #include <math.h>
 
 #include "rg_adjoint.cuh"
+#include "rg_face.cuh"
 #include "rg_fp64.cuh"
 #include "rg_hllc.cuh"
 #include "rg_lgi.cuh"
@@ -510,6 +511,41 @@ __device__ __forceinline__ bool solve_face_lagrangian(Prim l, Prim r, double vel
   return true;
 }
 
+// simple_flux_calculator.cpp:130-165 rotate / Hllc / rotate_back between the
+// states l and r of face e with velocity w; false where an operand is outside
+// the integer forms' range (the face then goes to its *_exact form).
+template <bool kBatch>
+__device__ __forceinline__ bool solve_face_fast(const StepArgs& a, int e, double g, const Cell& l, const Cell& r,
+                                                double2 w, Cons& out) {
+  FaceOps o;
+  const double2 n = a.geom.nrm[e], p = a.geom.par[e];
+  const Divisor dn = o.by(a.geom.nabs[e]), dp = o.by(a.geom.area[e]);
+  double speed = 0.0;
+  bool moving = false;
+  if (!a.ev_zero && !(is_zero(w.x) && is_zero(w.y))) {
+    speed = o.div(n.x * w.x + n.y * w.y, dn);
+    moving = !is_zero(speed);
+  }
+  const FaceSide ls{l.d, l.p, o.div(l.vx * n.x + l.vy * n.y, dn)};
+  const FaceSide rs{r.d, r.p, o.div(r.vx * n.x + r.vy * n.y, dn)};
+  Cons f;
+  bool left;
+  const Divisor gm1 = kBatch ? o.by(g - 1) : a.gm1;
+  o.ok = o.ok && gm1.ok;
+  hllc_face(
+      o, ls, rs, g, gm1, moving, speed,
+      [&](bool lft) {
+        const double vx = lft ? l.vx : r.vx, vy = lft ? l.vy : r.vy;
+        return o.div(vx * p.x + vy * p.y, dp);
+      },
+      f, left);
+  out.m = f.m;
+  out.mx = o.div(o.mul(n.x, f.mx), dn) + o.div(o.mul(p.x, f.my), dp);
+  out.my = o.div(o.mul(n.y, f.mx), dn) + o.div(o.mul(p.y, f.my), dp);
+  out.en = f.en;
+  return o.ok;
+}
+
 template <bool kBatch>
 __device__ __forceinline__ void write_flux(const StepArgs& a, int e, int real_side, const Cons& c, bool scaled,
                                            double area) {
@@ -521,13 +557,20 @@ __device__ __forceinline__ void write_flux(const StepArgs& a, int e, int real_si
   }
 }
 
-// ModularFluxCalculator (modular_flux_calculator.cpp:39-71) with the face
-// states of LinearGaussImproved (:570-590 real sides, :596-634 ghost sides).
-template <bool kScaled, bool kBatch>
-__device__ __forceinline__ void k_faces_lgi_item(const StepArgs& a, int e) {
+// simple_flux_calculator.cpp:17-25 reflect (Reflect, geometry.cpp:117-120);
+// keeps the source's energy and sound speed.
+__device__ __forceinline__ Prim reflect(Prim q, double2 axis, double aa) {
+  const double s = 2 * (q.vx * axis.x + q.vy * axis.y);
+  const double pp = aa * aa;
+  const double tx = quot(axis.x * s, pp), ty = quot(axis.y * s, pp);
+  q.vx = tx - q.vx;
+  q.vy = ty - q.vy;
+  return q;
+}
+
+// The face states of LinearGaussImproved (:570-590 real sides, :596-634 ghost sides).
+__device__ __forceinline__ void lgi_states(const StepArgs& a, int e, int2 fc, Cell side[2]) {
   const MeshDev& m = a.mesh;
-  const int2 fc = m.face_cells[e];
-  Cell side[2];
   const int ids[2] = {fc.x, fc.y};
   const double2 dms[2] = {a.geom.dm0[e], a.geom.dm1[e]};
 #pragma unroll
@@ -549,16 +592,57 @@ __device__ __forceinline__ void k_faces_lgi_item(const StepArgs& a, int e) {
       gx = Cell{s0.x, s0.y, s1.x, s1.y};
       gy = Cell{s2.x, s2.y, s3.x, s3.y};
     }
-    addmult(c, gx, dms[s].x);
-    addmult(c, gy, dms[s].y);
+    const MulFactor fx = mul_factor(dms[s].x), fy = mul_factor(dms[s].y);
+    c.d += mul_rn(fx, dms[s].x, gx.d);
+    c.p += mul_rn(fx, dms[s].x, gx.p);
+    c.vx += mul_rn(fx, dms[s].x, gx.vx);
+    c.vy += mul_rn(fx, dms[s].x, gx.vy);
+    c.d += mul_rn(fy, dms[s].y, gy.d);
+    c.p += mul_rn(fy, dms[s].y, gy.p);
+    c.vx += mul_rn(fy, dms[s].y, gy.vx);
+    c.vy += mul_rn(fy, dms[s].y, gy.vy);
     side[s] = c;
   }
-  const double2 w = a.ev_zero ? make_double2(0.0, 0.0) : reinterpret_cast<const double2*>(a.ev)[e];
+}
+__device__ __forceinline__ double2 face_velocity(const StepArgs& a, int e) {
+  return a.ev_zero ? make_double2(0.0, 0.0) : reinterpret_cast<const double2*>(a.ev)[e];
+}
+// The cell states of SimpleFluxCalculator (simple_flux_calculator.cpp:80-126):
+// a self-mirror ghost is its neighbour's reflection, any other its source.
+__device__ __forceinline__ void pcm_states(const StepArgs& a, int e, int2 fc, Cell side[2]) {
+  const MeshDev& m = a.mesh;
+  const int oa = orig_of(m, fc.x), ob = orig_of(m, fc.y);
+  side[0] = load_cell(a.cells, oa);
+  side[1] = load_cell(a.cells, ob);
+  if (oa == ob && (fc.x >= m.n || fc.y >= m.n)) {
+    // both sides hold the real cell's state
+    const Prim q = reflect(Prim{side[0].d, side[0].p, side[0].vx, side[0].vy, 0.0, 0.0}, a.geom.par[e], a.geom.area[e]);
+    if (fc.x < m.n) {
+      side[1].vx = q.vx;
+      side[1].vy = q.vy;
+    } else {
+      side[0].vx = q.vx;
+      side[0].vy = q.vy;
+    }
+  }
+}
+
+// Face e by hllc() itself: operands outside solve_face_fast's range, and its
+// failures (recorded here).
+template <bool kScaled, bool kBatch, bool kLgi>
+static __device__ __noinline__ void face_exact(const StepArgs& a, int e) {
+  const int2 fc = a.mesh.face_cells[e];
+  Cell side[2];
+  if (kLgi)
+    lgi_states(a, e, fc, side);
+  else
+    pcm_states(a, e, fc, side);
+  const double2 w = face_velocity(a, e);
   const double2 n = a.geom.nrm[e], p = a.geom.par[e];
   const double na = a.geom.nabs[e], pa = a.geom.area[e];
   // a face at rest has speed +-0 (the sign only reaches signs of zeros)
   const double speed = (w.x == 0.0 && w.y == 0.0) ? 0.0 : quot(n.x * w.x + n.y * w.y, na);
-  const int real_side = fc.x < m.n ? fc.x : fc.y;
+  const int real_side = fc.x < a.mesh.n ? fc.x : fc.y;
   const double g = gamma_at<kBatch>(a, real_side);
   Cons c;
   if (!solve_face(to_prim(g, side[0]), to_prim(g, side[1]), speed, n, na, p, pa, c, a, e)) return;
@@ -566,59 +650,35 @@ __device__ __forceinline__ void k_faces_lgi_item(const StepArgs& a, int e) {
   write_flux<kBatch>(a, e, real_side, c, kScaled, a.geom.xarea[e]);
 }
 
-template <bool kScaled, bool kBatch>
-__global__ void __launch_bounds__(kMaxBlock) k_faces_lgi(StepArgs a) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.mesh.e; e += gridDim.x * blockDim.x)
-    k_faces_lgi_item<kScaled, kBatch>(a, e);
-}
-
-// simple_flux_calculator.cpp:17-25 reflect (Reflect, geometry.cpp:117-120);
-// keeps the source's energy and sound speed.
-__device__ __forceinline__ Prim reflect(Prim q, double2 axis, double aa) {
-  const double s = 2 * (q.vx * axis.x + q.vy * axis.y);
-  const double pp = aa * aa;
-  const double tx = quot(axis.x * s, pp), ty = quot(axis.y * s, pp);
-  q.vx = tx - q.vx;
-  q.vy = ty - q.vy;
-  return q;
-}
-
-// SimpleFluxCalculator (simple_flux_calculator.cpp:80-126 riemann_reduce,
-// :216-244).  A ghost that is not its neighbour's own mirror takes its source
-// cell's state.
-template <bool kScaled, bool kBatch>
-__device__ __forceinline__ void k_faces_pcm_item(const StepArgs& a, int e) {
-  const MeshDev& m = a.mesh;
-  const int2 fc = m.face_cells[e];
-  const double2 p = a.geom.par[e], n = a.geom.nrm[e];
-  const double pa = a.geom.area[e], na = a.geom.nabs[e];
-  const bool va = fc.x < m.n, vb = fc.y < m.n;
-  const int oa = orig_of(m, fc.x), ob = orig_of(m, fc.y);
-  const int real_side = va ? fc.x : fc.y;
-  const double g = gamma_at<kBatch>(a, real_side);
-  Prim l, r;
-  if (!va) {
-    r = to_prim(g, load_cell(a.cells, fc.y));
-    l = oa == ob ? reflect(r, p, pa) : to_prim(g, load_cell(a.cells, oa));
-  } else if (!vb) {
-    l = to_prim(g, load_cell(a.cells, fc.x));
-    r = oa == ob ? reflect(l, p, pa) : to_prim(g, load_cell(a.cells, ob));
-  } else {
-    l = to_prim(g, load_cell(a.cells, fc.x));
-    r = to_prim(g, load_cell(a.cells, fc.y));
-  }
-  const double2 w = a.ev_zero ? make_double2(0.0, 0.0) : reinterpret_cast<const double2*>(a.ev)[e];
-  const double velocity = (w.x == 0.0 && w.y == 0.0) ? 0.0 : quot(n.x * w.x + n.y * w.y, na);
+// ModularFluxCalculator (modular_flux_calculator.cpp:39-71, kLgi) or
+// SimpleFluxCalculator (simple_flux_calculator.cpp:216-244) for one face.
+template <bool kScaled, bool kBatch, bool kLgi>
+__device__ __forceinline__ void k_faces_item(const StepArgs& a, int e) {
+  const int2 fc = a.mesh.face_cells[e];
+  Cell side[2];
+  if (kLgi)
+    lgi_states(a, e, fc, side);
+  else
+    pcm_states(a, e, fc, side);
+  const int real_side = fc.x < a.mesh.n ? fc.x : fc.y;
   Cons c;
-  if (!solve_face(l, r, velocity, n, na, p, pa, c, a, e)) return;
+  if (!solve_face_fast<kBatch>(a, e, gamma_at<kBatch>(a, real_side), side[0], side[1], face_velocity(a, e), c)) {
+    face_exact<kScaled, kBatch, kLgi>(a, e);
+    return;
+  }
   if (a.mflux) a.mflux[e] = c.m;
   write_flux<kBatch>(a, e, real_side, c, kScaled, a.geom.xarea[e]);
 }
 
-template <bool kScaled, bool kBatch>
-__global__ void __launch_bounds__(kMaxBlock) k_faces_pcm(StepArgs a) {
+// One thread per face.  Bound by the FP64 unit (85 FP64 instructions per warp,
+// the integer pipes a third busy beside it) and by its 4,500 instructions of
+// code: blocks of 512 run it in step and miss the instruction cache less.  64
+// registers (two such blocks per SM) spill 300 bytes and still gain.  512^2
+// (786,430 faces, RoundCells face velocities) 205 -> 141 us, 256^2 66 -> 45 us.
+template <bool kScaled, bool kBatch, bool kLgi>
+__global__ void __launch_bounds__(kMaxBlock, 2) k_faces(StepArgs a) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.mesh.e; e += gridDim.x * blockDim.x)
-    k_faces_pcm_item<kScaled, kBatch>(a, e);
+    k_faces_item<kScaled, kBatch, kLgi>(a, e);
 }
 
 // ---------------------------------------------------------------- condition/action fluxes
@@ -693,7 +753,7 @@ __device__ __forceinline__ void k_faces_cas_item(const StepArgs& a, int e) {
     const double sign = 2.0 * (a.rules[chosen][4] != 0 ? 1.0 : 0.0) - 1.0;
     action = (nx * sc.vx + ny * sc.vy) * sign < 0 ? RG_ACT_FREE_FLOW : RG_ACT_RIGID_WALL2;
   }
-  // LinearGaussImproved face states (order 2), as k_faces_lgi_item forms them
+  // LinearGaussImproved face states (order 2), as lgi_states forms them
   Cell s0 = c0, s1 = c1;
   if (action == RG_ACT_REGULAR2 || action == RG_ACT_RIGID_WALL2 || action == RG_ACT_LAGRANGIAN) {
     const int ids[2] = {fc.x, fc.y};
@@ -1055,7 +1115,7 @@ cudaError_t launch_ghost_fill(const StepArgs& a, cudaStream_t s) {
 
 cudaError_t launch_slopes(const StepArgs& a, cudaStream_t s) {
   if (a.mesh.n > 0) {
-    const LaunchShape& sh = a.shapes.slopes;
+    const LaunchShape sh = fit_shape(a.shapes.slopes, 4LL * a.mesh.n);
     const int nb = grid_of(sh, 4LL * a.mesh.n), bs = sh.block;
     const bool b = a.cell_problem != nullptr;
     // builds: 0 plain, 2 and 3 register-capped for 3 and 4 resident blocks of
@@ -1076,7 +1136,8 @@ cudaError_t launch_slopes_trace(const StepArgs& a, SlopeTrace* trace, cudaStream
 
 cudaError_t launch_faces(const StepArgs& a, cudaStream_t s, bool scaled) {
   if (a.mesh.e == 0) return cudaSuccess;
-  const int nb = grid_of(a.shapes.faces, a.mesh.e), bs = a.shapes.faces.block;
+  const LaunchShape sh = fit_shape(a.shapes.faces, a.mesh.e);
+  const int nb = grid_of(sh, a.mesh.e), bs = sh.block;
   const bool b = a.cell_problem != nullptr;
   if (a.n_rules > 0) {
     scaled ? k_faces_cas<true><<<nb, bs, 0, s>>>(a) : k_faces_cas<false><<<nb, bs, 0, s>>>(a);
@@ -1084,14 +1145,14 @@ cudaError_t launch_faces(const StepArgs& a, cudaStream_t s, bool scaled) {
   }
   if (a.order == 1) {
     if (scaled)
-      b ? k_faces_pcm<true, true><<<nb, bs, 0, s>>>(a) : k_faces_pcm<true, false><<<nb, bs, 0, s>>>(a);
+      b ? k_faces<true, true, false><<<nb, bs, 0, s>>>(a) : k_faces<true, false, false><<<nb, bs, 0, s>>>(a);
     else
-      b ? k_faces_pcm<false, true><<<nb, bs, 0, s>>>(a) : k_faces_pcm<false, false><<<nb, bs, 0, s>>>(a);
+      b ? k_faces<false, true, false><<<nb, bs, 0, s>>>(a) : k_faces<false, false, false><<<nb, bs, 0, s>>>(a);
   } else {
     if (scaled)
-      b ? k_faces_lgi<true, true><<<nb, bs, 0, s>>>(a) : k_faces_lgi<true, false><<<nb, bs, 0, s>>>(a);
+      b ? k_faces<true, true, true><<<nb, bs, 0, s>>>(a) : k_faces<true, false, true><<<nb, bs, 0, s>>>(a);
     else
-      b ? k_faces_lgi<false, true><<<nb, bs, 0, s>>>(a) : k_faces_lgi<false, false><<<nb, bs, 0, s>>>(a);
+      b ? k_faces<false, true, true><<<nb, bs, 0, s>>>(a) : k_faces<false, false, true><<<nb, bs, 0, s>>>(a);
   }
   return cudaGetLastError();
 }

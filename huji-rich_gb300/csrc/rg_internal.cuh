@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "rg_convert.cuh"
+#include "rg_div.cuh"
 #include "rich_gb300.h"
 
 namespace rg {
@@ -212,6 +213,14 @@ struct LaunchShape {
 };
 constexpr LaunchShape kDefaultShape{256, 0, 0};
 constexpr int kCappedBlock = 256;
+// A one-thread-per-item grid of large blocks that would leave SMs without one
+// is launched in smaller blocks (256 x 66-face meshes and the like: the FP64
+// faces of 96 x 101 cells take 16 us in blocks of 64 to 256, 20 us as 57 of 512).
+constexpr int kSms = 152;
+inline LaunchShape fit_shape(LaunchShape s, long long items) {
+  while (s.max_blocks == 0 && s.block > 64 && s.block % 64 == 0 && items < 2LL * kSms * s.block) s.block /= 2;
+  return s;
+}
 inline int grid_of(const LaunchShape& s, long long items) {
   const int need = items > 0 ? static_cast<int>((items + s.block - 1) / s.block) : 1;
   return s.max_blocks > 0 && need > s.max_blocks ? s.max_blocks : need;
@@ -230,6 +239,7 @@ struct StepArgs {
   MeshDev mesh;
   GeomDev geom;
   double gamma, cfl;
+  Divisor gm1;          // gamma - 1 as a divisor (one problem)
   int order, ghost_kind, slf;
   double delta_v, theta, delta_p;
   double* cells;        // 4*np (ghost entries at the end), read by every pass
