@@ -173,38 +173,57 @@ __global__ void __launch_bounds__(kBlock) k3_faces(Step3Args a) {
   }
 }
 
-__global__ void __launch_bounds__(kBlock) k3_update(Step3Args a, int from_unscaled, int do_ext, int do_cells) {
+// kExt / kUnscaled / kCells: template arguments, since FP64 instructions of a
+// form that is off still take the FP64 unit where the compiler predicates them
+template <bool kUnscaled, bool kExt, bool kCells>
+__global__ void __launch_bounds__(kBlock) k3_update(Step3Args a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const Mesh3Dev& m = a.mesh;
   if (i >= m.n) return;
   const double2* e2 = reinterpret_cast<const double2*>(a.ext) + 3 * i;
   const double2 e01 = e2[0], e23 = e2[1], e45 = e2[2];
   double u[5] = {e01.x, e01.y, e23.x, e23.y, e45.x};
-  if (do_ext) {
-    const double dt = from_unscaled ? (a.dt_from_device ? a.status->dt : a.dt_host) : 0.0;
+  if (kExt) {
+    const double dt = kUnscaled ? (a.dt_from_device ? a.status->dt : a.dt_host) : 0.0;
     for (int k = m.cell_off[i]; k < m.cell_off[i + 1]; ++k) {
       const int fs = a.fsign[k];
       const int f = fs & 0x7fffffff;
       const double2* fl = reinterpret_cast<const double2*>(a.fluxes) + 3 * f;
       const double2 f01 = fl[0], f23 = fl[1], f45 = fl[2];
       double d[5] = {f01.x, f01.y, f23.x, f23.y, f45.x};
-      if (from_unscaled) {
+      if (kUnscaled) {
         const double s = dt * m.area[f];  // dt*GetArea()*flux (hdsim_3d.cpp:69)
 #pragma unroll
         for (int q = 0; q < 5; ++q) d[q] = s * d[q];
       }
 #pragma unroll
-      for (int q = 0; q < 5; ++q) u[q] = fs < 0 ? u[q] - d[q] : u[q] + d[q];
+      for (int q = 0; q < 5; ++q) u[q] += flip_sign(d[q], static_cast<uint32_t>(fs) & 0x80000000u);
     }
     store6(a.ext, i, u[0], u[1], u[2], u[3], u[4]);
   }
-  if (do_cells) {
-    const double V = m.volume[i];
-    const double density = quot(u[0], V);
-    const V3 vel = vdiv(V3{quot(u[1], V), quot(u[2], V), quot(u[3], V)}, density);
-    const double thermal = quot(u[4], V) - 0.5 * density * vdot(vel, vel);
-    const double eint = quot(thermal, density);
-    if (eint < 0) {
+  if (kCells) {
+    // nine quotients by two divisors
+    const Divisor dv = divisor(m.volume[i], RcpSeedDevice{});
+    bool ok = true;
+    auto by = [&ok](double x, const Divisor& D) {
+      double q;
+      ok = div_by(x, D, &q) && ok;
+      return q;
+    };
+    double density = by(u[0], dv);
+    const Divisor dd = divisor(density, RcpSeedDevice{});
+    V3 vel{by(by(u[1], dv), dd), by(by(u[2], dv), dd), by(by(u[3], dv), dd)};
+    double ev = by(u[4], dv);
+    if (!ok) {
+      const double V = m.volume[i];
+      density = quot(u[0], V);
+      vel = vdiv(V3{quot(u[1], V), quot(u[2], V), quot(u[3], V)}, density);
+      ev = quot(u[4], V);
+    }
+    const double thermal = ev - 0.5 * density * vdot(vel, vel);
+    double eint;
+    if (!ok || !div_by(thermal, dd, &eint)) eint = quot(thermal, density);
+    if (lt(eint, 0.0)) {
       record_error(a.status, a.step, RG_ERR_NEGATIVE_ENERGY, 5, i, eint);
       return;
     }
@@ -284,7 +303,15 @@ cudaError_t launch3_faces(const Step3Args& a, bool scaled, cudaStream_t s) {
 }
 
 cudaError_t launch3_update(const Step3Args& a, bool from_unscaled, bool do_ext, bool do_cells, cudaStream_t s) {
-  k3_update<<<blocks(a.mesh.n), kBlock, 0, s>>>(a, from_unscaled ? 1 : 0, do_ext ? 1 : 0, do_cells ? 1 : 0);
+  const int nb = blocks(a.mesh.n);
+  if (do_ext && do_cells)
+    k3_update<false, true, true><<<nb, kBlock, 0, s>>>(a);  // (the fused step's fluxes are scaled)
+  else if (do_ext && from_unscaled)
+    k3_update<true, true, false><<<nb, kBlock, 0, s>>>(a);
+  else if (do_ext)
+    k3_update<false, true, false><<<nb, kBlock, 0, s>>>(a);
+  else
+    k3_update<false, false, true><<<nb, kBlock, 0, s>>>(a);
   return cudaGetLastError();
 }
 

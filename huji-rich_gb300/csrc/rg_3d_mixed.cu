@@ -89,11 +89,11 @@ __global__ void __launch_bounds__(kBlock) k3m_to64(const float4* c32, const floa
   if (i >= n) return;
   const float4 c = c32[i];
   double* o = c64 + 6 * i;
-  o[0] = c.x;
-  o[1] = c.y;
-  o[2] = c.z;
-  o[3] = c.w;
-  o[4] = vz[i];
+  o[0] = widen_exact(c.x);
+  o[1] = widen_exact(c.y);
+  o[2] = widen_exact(c.z);
+  o[3] = widen_exact(c.w);
+  o[4] = widen_exact(vz[i]);
   o[5] = 0.0;
 }
 
@@ -102,11 +102,11 @@ __global__ void __launch_bounds__(kBlock) k3m_flux_to64(const float4* f32, const
   if (f >= e) return;
   const float4 v = f32[f];
   double* o = f64 + 6 * f;
-  o[0] = v.x;
-  o[1] = v.y;
-  o[2] = v.z;
-  o[3] = v.w;
-  o[4] = fen[f];
+  o[0] = widen_exact(v.x);
+  o[1] = widen_exact(v.y);
+  o[2] = widen_exact(v.z);
+  o[3] = widen_exact(v.w);
+  o[4] = widen_exact(fen[f]);
   o[5] = 0.0;
 }
 

@@ -77,6 +77,14 @@ RG_CONV_FN double conv_double(uint32_t hi, uint32_t lo) {
 #endif
 }
 
+// The conversions that narrow() and widen_exact() leave to the hardware, out
+// of line on the device: inlined, the compiler predicates the instruction, and
+// a predicated-off one still takes the FP64 unit's clocks.
+#ifdef __CUDACC__
+static __device__ __noinline__ float cvt_narrow(double x) { return __double2float_rn(x); }
+static __device__ __noinline__ double cvt_widen(float f) { return static_cast<double>(f); }
+#endif
+
 // double -> float rounded to nearest, ties to even: static_cast<float>(x)
 // for every x.  Results in the normal float range and zeros are formed on
 // the integer pipe (the 29 dropped significand bits decide the rounding; a
@@ -95,7 +103,11 @@ RG_CONV_FN float narrow(double x) {
     return conv_float(f);
   }
   if (((hi & 0x7fffffffu) | lo) == 0u) return conv_float(hi & 0x80000000u);
+#ifdef __CUDA_ARCH__
+  return cvt_narrow(x);
+#else
   return static_cast<float>(x);
+#endif
 }
 
 // float -> double, exact (static_cast<double>(f) for every f): zeros,
@@ -104,7 +116,13 @@ RG_CONV_FN float narrow(double x) {
 RG_CONV_FN double widen_exact(float f) {
   const uint32_t u = conv_fbits(f);
   const uint32_t ex = (u >> 23) & 0xffu, mant = u & 0x7fffffu;
-  if (ex == 0u && mant != 0u) return static_cast<double>(f);
+  if (ex == 0u && mant != 0u) {
+#ifdef __CUDA_ARCH__
+    return cvt_widen(f);
+#else
+    return static_cast<double>(f);
+#endif
+  }
   const uint32_t dex = ex == 0u ? 0u : (ex == 0xffu ? 0x7ffu : ex + 896u);  // rebias 127 -> 1023
   return conv_double((u & 0x80000000u) | (dex << 20) | (mant >> 3), mant << 29);
 }
@@ -114,6 +132,13 @@ RG_CONV_FN double widen_exact(float f) {
 
 constexpr uint64_t kMagMask = 0x7fffffffffffffffull;
 constexpr uint64_t kInfBits64 = 0x7ff0000000000000ull;
+
+// x with the bits of `flip` (0 or the sign bit of the high word) exclusive-ored
+// in: a - b is a + (-b) bit for bit, where a choice between the two would put
+// both on the FP64 unit
+RG_CONV_FN double flip_sign(double x, uint32_t flip) {
+  return conv_double_bits(conv_dbits(x) ^ (static_cast<uint64_t>(flip) << 32));
+}
 
 // |a| > t for t >= 0 or NaN
 RG_CONV_FN bool abs_gt(double a, double t) {

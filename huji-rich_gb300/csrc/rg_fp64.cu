@@ -282,58 +282,114 @@ __global__ void __launch_bounds__(kBlock) k_validate(MeshDev m, DevStatus* st) {
 
 // ---------------------------------------------------------------- per step
 
-// simple_cfl.cpp:28-47 (per cell) and :58-71 + lazy_list.hpp:185-191 (min, times cfl).
+// Cell i's SimpleCFL bound (simple_cfl.cpp:28-47) with state c: the bit pattern
+// of 1 / max_e((cs + |v - w_e|) / R), which orders as an integer.  fmax over
+// faces of (cs + sqrt(q_e)) / R equals (cs + sqrt(max q_e)) / R exactly: sqrt, +
+// and / are correctly rounded, hence monotone, so the maximum commutes with
+// them.  NaN terms are skipped as fmax skips them.
+template <bool kBatch>
+static __device__ __noinline__ unsigned long long cfl_bound_bits(const StepArgs& a, int i, Cell c) {
+  const MeshDev& m = a.mesh;
+  const double cs = root(quot(gamma_at<kBatch>(a, i) * c.p, c.d));
+  double q = 0;
+  bool any = false;
+  const int b = m.cell_off[i], e1 = m.cell_off[i + 1];
+  if (a.ev_zero) {
+    // every face at rest: each term is vx^2 + vy^2 (v - 0 == v)
+    const double qq = c.vx * c.vx + c.vy * c.vy;
+    if (e1 > b && !isnan(qq)) {
+      q = fmax(q, qq);
+      any = true;
+    }
+  } else {
+    for (int k = b; k < e1; ++k) {
+      const double2 w = reinterpret_cast<const double2*>(a.ev)[m.cell_faces[k]];
+      const double dx = c.vx - w.x, dy = c.vy - w.y;
+      const double qq = dx * dx + dy * dy;
+      if (!isnan(qq)) {
+        q = fmax(q, qq);
+        any = true;
+      }
+    }
+  }
+  const double res = any ? fmax(0.0, quot(cs + root(q), a.geom.width[i])) : 0.0;
+  return static_cast<unsigned long long>(__double_as_longlong(quot(1.0, res)));
+}
+
+// FP32 bounds lo <= max_e((cs + |v - w_e|) / R) <= hi of that rate.  The
+// truncations to 24 bits leave each difference v - w_e within
+// 2^-23 (|v| + |w_e|) and a rounding; cs, the root and the quotient carry a few
+// 2^-24 each.  hi is infinite (and lo 0) where an operand is outside the normal
+// floats or a value is not finite.
+template <bool kBatch>
+__device__ __forceinline__ void cfl_estimate(const StepArgs& a, int i, const Cell& c, float& lo, float& hi) {
+  const MeshDev& m = a.mesh;
+  bool ok = true;
+  const float d = trunc32(c.d, ok), p = trunc32(c.p, ok), vx = trunc32_any(c.vx, ok), vy = trunc32_any(c.vy, ok);
+  const float g = trunc32(gamma_at<kBatch>(a, i), ok), r = trunc32(a.geom.width[i], ok);
+  const float cs = sqrtf(__fdividef(g * p, d));
+  const int b = m.cell_off[i], e1 = m.cell_off[i + 1];
+  float q = 0.0f, w1 = 0.0f;
+  if (a.ev_zero) {
+    q = fmaf(vx, vx, vy * vy);
+  } else {
+    for (int k = b; k < e1; ++k) {
+      const double2 w = reinterpret_cast<const double2*>(a.ev)[m.cell_faces[k]];
+      const float wx = trunc32_any(w.x, ok), wy = trunc32_any(w.y, ok);
+      const float dx = vx - wx, dy = vy - wy;
+      q = fmaxf(q, fmaf(dx, dx, dy * dy));
+      w1 = fmaxf(w1, fabsf(wx) + fabsf(wy));
+    }
+  }
+  const float err = 3e-7f * (fabsf(vx) + fabsf(vy) + w1) + 1e-18f;
+  const float v = sqrtf(q);
+  lo = __fdividef(0.99999f * cs + fmaxf(0.99999f * v - err, 0.0f), r) * 0.99999f;
+  hi = __fdividef(1.00001f * cs + 1.00001f * v + err, r) * 1.00001f;
+  if (!(ok && e1 > b && hi < 1e30f && cs > 1e-15f && r > 0.0f)) {
+    lo = 0.0f;
+    hi = 3e38f;
+  }
+}
+
+// The smallest exact bound of the block's cells, on the threads whose cell can
+// hold it (the others return +inf): every thread of the block calls this, with
+// live = false where it has no cell.  Only a cell whose estimate reaches the
+// block's largest lower estimate is formed exactly: its quotients, roots and
+// per-face FP64 differences are a third of the update kernel's work.
+template <bool kBatch>
+__device__ __forceinline__ unsigned long long cfl_block_bits(const StepArgs& a, bool live, int i, const Cell& c) {
+  __shared__ unsigned best;
+  float lo = 0.0f, hi = -1.0f;
+  if (threadIdx.x == 0) best = 0u;
+  if (live) cfl_estimate<kBatch>(a, i, c, lo, hi);
+  __syncthreads();
+  const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(lo));
+  if ((threadIdx.x & 31) == 0) atomicMax(&best, top);
+  __syncthreads();
+  const bool need = live && hi >= __uint_as_float(best);
+  __syncthreads();  // best is reused by the next call
+  return need ? cfl_bound_bits<kBatch>(a, i, c) : kInfBits;
+}
+
+// simple_cfl.cpp:58-71 + lazy_list.hpp:185-191 (min over the cells, times cfl)
 template <bool kBatch>
 __global__ void __launch_bounds__(kMaxBlock) k_cfl(StepArgs a, int fill_ghosts) {
   const MeshDev& m = a.mesh;
   const int total = fill_ghosts ? m.n + m.g : m.n;
-  // this thread's minimum of 1/bound as a bit pattern (positive doubles and
-  // +inf order as integers)
   unsigned long long bits = kInfBits;
-  // the trip count is uniform across a warp (base is per block), as the
-  // warp-aggregated per-problem minimum of the batch form needs
+  // the trip count is uniform across a block (base is per block)
   for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
     const int t = base + threadIdx.x;
-    double x = __longlong_as_double(static_cast<long long>(kInfBits));
-    if (t < m.n) {
-      const Cell c = load_cell(a.cells, t);
-      const double radius = a.geom.width[t];
-      const double cs = root(quot(gamma_at<kBatch>(a, t) * c.p, c.d));
-      // fmax over faces of (cs + sqrt(q_e)) / radius equals (cs + sqrt(max q_e)) /
-      // radius exactly: sqrt, + and / are correctly rounded, hence monotone, so
-      // the maximum commutes with them.  NaN terms are skipped as fmax skips them.
-      double q = 0;
-      bool any = false;
-      const int b = m.cell_off[t], e1 = m.cell_off[t + 1];
-      if (a.ev_zero) {
-        // every face at rest: each term is vx^2 + vy^2 (v - 0 == v)
-        const double qq = c.vx * c.vx + c.vy * c.vy;
-        if (e1 > b && !isnan(qq)) {
-          q = fmax(q, qq);
-          any = true;
-        }
-      } else {
-        for (int k = b; k < e1; ++k) {
-          const double2 w = reinterpret_cast<const double2*>(a.ev)[m.cell_faces[k]];
-          const double dx = c.vx - w.x, dy = c.vy - w.y;
-          const double qq = dx * dx + dy * dy;
-          if (!isnan(qq)) {
-            q = fmax(q, qq);
-            any = true;
-          }
-        }
-      }
-      const double res = any ? fmax(0.0, quot(cs + root(q), radius)) : 0.0;
-      x = quot(1.0, res);
-    } else if (t < total) {
-      fill_ghost(a, t - m.n);
-    }
-    const unsigned long long xb = static_cast<unsigned long long>(__double_as_longlong(x));
-    if (kBatch)
+    if (t >= m.n && t < total) fill_ghost(a, t - m.n);
+    if (kBatch) {
       // per-problem minimum; the update kernel turns it into the problem's dt
+      const unsigned long long xb = t < m.n ? cfl_bound_bits<kBatch>(a, t, load_cell(a.cells, t)) : kInfBits;
       problem_min(a.dtmin_p, t < m.n ? a.cell_problem[t] : -1, xb);
-    else
+    } else {
+      const bool live = t < m.n;
+      const unsigned long long xb = cfl_block_bits<kBatch>(a, live, t, live ? load_cell(a.cells, t) : Cell{1, 1, 0, 0});
       bits = xb < bits ? xb : bits;
+    }
   }
   if (kBatch) return;
   grid_min_times(a.status, bits, a.cfl, &a.status->dt);
@@ -864,73 +920,46 @@ __global__ void __launch_bounds__(kMaxBlock) k_faces_cas(StepArgs a) {
 
 // ---------------------------------------------------------------- cells
 
-// The next step's SimpleCFL bound of cell i with state (d, pres, vx, vy), as
-// k_cfl computes it, as the bit pattern of 1/bound.
-template <bool kBatch>
-__device__ __forceinline__ unsigned long long cfl_bound_bits(const StepArgs& a, int i, double d, double pres,
-                                                             double vx, double vy) {
-  const MeshDev& m = a.mesh;
-  const double cs = root(quot(gamma_at<kBatch>(a, i) * pres, d));
-  double q = 0;
-  bool any = false;
-  if (a.ev_zero) {
-    const double qq = vx * vx + vy * vy;
-    if (m.cell_off[i + 1] > m.cell_off[i] && !isnan(qq)) {
-      q = fmax(q, qq);
-      any = true;
-    }
-  } else {
-    for (int k = m.cell_off[i]; k < m.cell_off[i + 1]; ++k) {
-      const double2 w = reinterpret_cast<const double2*>(a.ev)[m.cell_faces[k]];
-      const double dx = vx - w.x, dy = vy - w.y;
-      const double qq = dx * dx + dy * dy;
-      if (!isnan(qq)) {
-        q = fmax(q, qq);
-        any = true;
-      }
-    }
-  }
-  const double res = any ? fmax(0.0, quot(cs + root(q), a.geom.width[i])) : 0.0;
-  return static_cast<unsigned long long>(__double_as_longlong(quot(1.0, res)));
-}
+// What one launch of the update kernel does
+constexpr int kUpFused = 0;     // extensives from the scaled fluxes, then the cells
+constexpr int kUpAverage = 1;   // the same, the extensives averaged with ext_avg (Heun)
+constexpr int kUpUnscaled = 2;  // extensives only, from unscaled fluxes
+constexpr int kUpScaled = 3;    // extensives only, from scaled fluxes
+constexpr int kUpCells = 4;     // cells only
 
 // SimpleExtensiveUpdater (simple_extensive_updater.cpp:11-35) as a gather:
 // each cell applies its faces' contributions in ascending face order, which
 // is the order the reference's edge loop applies them to that cell; then
-// SimpleCellUpdater::regular_update (simple_cell_updater.cpp:22-59).
-template <bool kBatch>
-__device__ __forceinline__ unsigned long long k_update_item(const StepArgs& a, int i, int from_unscaled, int do_ext,
-                                                         int do_cells) {
+// SimpleCellUpdater::regular_update (simple_cell_updater.cpp:22-59).  Returns
+// whether c holds the cell's new state.  kMode is a compile-time constant: the
+// FP64 instructions of a mode that is off would still take the FP64 unit where
+// the compiler predicates them, and so would a choice between + and -.
+template <bool kBatch, int kMode>
+__device__ __forceinline__ bool update_cell(const StepArgs& a, int i, Cell& c) {
   const MeshDev& m = a.mesh;
   double2* ext2 = reinterpret_cast<double2*>(a.ext);
   double2 e01 = ext2[2 * i], e23 = ext2[2 * i + 1];
   double mass = e01.x, en = e01.y, px = e23.x, py = e23.y;
-  if (do_ext) {
-    const double dt = from_unscaled ? step_dt(a) : 0.0;
+  if (kMode != kUpCells) {
+    const double dt = kMode == kUpUnscaled ? step_dt(a) : 0.0;
     const int b = m.cell_off[i], e1 = m.cell_off[i + 1];
     for (int k = b; k < e1; ++k) {
       const int e = m.cell_faces[k];
       const double2* f = reinterpret_cast<const double2*>(a.fluxes) + 2 * e;
       const double2 f01 = f[0], f23 = f[1];
       double dm = f01.x, de = f01.y, dx = f23.x, dy = f23.y;
-      if (from_unscaled) {
+      if (kMode == kUpUnscaled) {
         const double s = dt * a.geom.xarea[e];
         dm *= s;
         de *= s;
         dx *= s;
         dy *= s;
       }
-      if (a.geom.nbr[k] & kNbrFirst) {
-        mass -= dm;
-        en -= de;
-        px -= dx;
-        py -= dy;
-      } else {
-        mass += dm;
-        en += de;
-        px += dx;
-        py += dy;
-      }
+      const uint32_t flip = a.geom.nbr[k] & kNbrFirst;  // bit 31
+      mass += flip_sign(dm, flip);
+      en += flip_sign(de, flip);
+      px += flip_sign(dx, flip);
+      py += flip_sign(dy, flip);
     }
     if (a.lag_update) {
       const double f = lag_factor(a, i);
@@ -939,7 +968,7 @@ __device__ __forceinline__ unsigned long long k_update_item(const StepArgs& a, i
       px *= f;
       py *= f;
     }
-    if (a.ext_avg) {
+    if (kMode == kUpAverage) {
       // hdsim2d.cpp:311-320 average_extensive: 0.5*(mid + old)
       const double2* o = reinterpret_cast<const double2*>(a.ext_avg);
       const double2 o01 = o[2 * i], o23 = o[2 * i + 1];
@@ -951,39 +980,49 @@ __device__ __forceinline__ unsigned long long k_update_item(const StepArgs& a, i
     double2* out2 = reinterpret_cast<double2*>(a.ext_out ? a.ext_out : a.ext);
     out2[2 * i] = make_double2(mass, en);
     out2[2 * i + 1] = make_double2(px, py);
+    if (kMode == kUpUnscaled || kMode == kUpScaled) return false;
   }
-  if (do_cells) {
-    if (a.frozen_mask && (a.stickers[i] & a.frozen_mask)) {
-      // simple_cell_updater.cpp:61-83 with (HasSticker, SkipUpdate): the old
-      // cell stays (its extensives above still took the fluxes)
-      const Cell c = load_cell(a.cells, i);
-      if (a.cells_out) store4(a.cells_out, i, c.d, c.p, c.vx, c.vy);
-      if (!a.cfl_next) return kInfBits;
-      return cfl_bound_bits<kBatch>(a, i, c.d, c.p, c.vx, c.vy);
-    }
-    const double d = quot(mass, m.cd_volume[i]);
-    if (d < 0) {
-      record_error(a.status, a.step, RG_ERR_NEGATIVE_DENSITY, 5, i, d);
-      return kInfBits;
-    }
-    const double vx = quot(px, mass), vy = quot(py, mass);
-    const double energy = quot(en, mass) - 0.5 * (vx * vx + vy * vy);
-    if (energy < 0) {
-      record_error(a.status, a.step, RG_ERR_NEGATIVE_ENERGY, 5, i, energy);
-      return kInfBits;
-    }
-    const double pres = (gamma_at<kBatch>(a, i) - 1) * energy * d;
-    store4(a.cells_out ? a.cells_out : a.cells, i, d, pres, vx, vy);
-    // the next step's SimpleCFL bound of this cell, from the record just stored
-    if (a.cfl_next) return cfl_bound_bits<kBatch>(a, i, d, pres, vx, vy);
+  if (a.frozen_mask && (a.stickers[i] & a.frozen_mask)) {
+    // simple_cell_updater.cpp:61-83 with (HasSticker, SkipUpdate): the old
+    // cell stays (its extensives above still took the fluxes)
+    c = load_cell(a.cells, i);
+    if (a.cells_out) store4(a.cells_out, i, c.d, c.p, c.vx, c.vy);
+    return true;
   }
-  return kInfBits;
+  const double d = quot(mass, m.cd_volume[i]);
+  if (lt(d, 0.0)) {
+    record_error(a.status, a.step, RG_ERR_NEGATIVE_DENSITY, 5, i, d);
+    return false;
+  }
+  // four quotients by the mass share its preparation
+  const Divisor dm = divisor(mass, RcpSeedDevice{});
+  double vx, vy, em;
+  bool ok = div_by(px, dm, &vx);
+  ok = div_by(py, dm, &vy) && ok;
+  ok = div_by(en, dm, &em) && ok;
+  if (!ok) {
+    vx = quot(px, mass);
+    vy = quot(py, mass);
+    em = quot(en, mass);
+  }
+  const double energy = em - 0.5 * (vx * vx + vy * vy);
+  if (lt(energy, 0.0)) {
+    record_error(a.status, a.step, RG_ERR_NEGATIVE_ENERGY, 5, i, energy);
+    return false;
+  }
+  c = Cell{d, (gamma_at<kBatch>(a, i) - 1) * energy * d, vx, vy};
+  store4(a.cells_out ? a.cells_out : a.cells, i, c.d, c.p, c.vx, c.vy);
+  return true;
 }
 
-template <bool kBatch>
-__global__ void __launch_bounds__(kMaxBlock) k_update(StepArgs a, int from_unscaled, int do_ext, int do_cells) {
+// Bound by the FP64 unit and its gathers.  512^2 with face velocities, with the
+// next dt: 76 -> 44 us (256^2: 15 -> 10 us).  The modes as template arguments,
+// signs flipped instead of + / - chosen and the CFL bound estimated took a
+// warp's FP64 instructions from 128 to about 40.
+template <bool kBatch, int kMode>
+__global__ void __launch_bounds__(kMaxBlock) k_update(StepArgs a) {
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  if (kBatch && do_ext && !from_unscaled && !a.batch_keep_dt) {
+  if (kBatch && kMode <= kUpAverage && !a.batch_keep_dt) {
     for (int p = t0; p < a.n_problems; p += stride) {
       // every face of this step has read its problem's minimum: record the dt,
       // advance the problem's time and reset the minimum for the next step
@@ -995,11 +1034,23 @@ __global__ void __launch_bounds__(kMaxBlock) k_update(StepArgs a, int from_unsca
   }
   unsigned long long bits = kInfBits;
   const int* order = a.geom.cell_order;
-  for (int t = t0; t < a.mesh.n; t += stride) {
-    const unsigned long long b = k_update_item<kBatch>(a, order ? order[t] : t, from_unscaled, do_ext, do_cells);
-    bits = b < bits ? b : bits;
+  // the next step's SimpleCFL minimum, from the states just stored
+  const bool next = !kBatch && kMode <= kUpAverage && a.cfl_next;
+  for (int base = blockIdx.x * blockDim.x; base < a.mesh.n; base += stride) {
+    const int t = base + threadIdx.x;
+    Cell c{1, 1, 0, 0};
+    bool live = false;
+    int i = 0;
+    if (t < a.mesh.n) {
+      i = order ? order[t] : t;
+      live = update_cell<kBatch, kMode>(a, i, c);
+    }
+    if (next) {
+      const unsigned long long b = cfl_block_bits<kBatch>(a, live, i, c);
+      bits = b < bits ? b : bits;
+    }
   }
-  if (!kBatch && a.cfl_next) grid_min_times(a.status, bits, a.cfl, &a.status->dt_next);
+  if (next) grid_min_times(a.status, bits, a.cfl, &a.status->dt_next);
 }
 
 // hdsim2d.cpp:41-67 init_extensives
@@ -1160,10 +1211,22 @@ cudaError_t launch_faces(const StepArgs& a, cudaStream_t s, bool scaled) {
 cudaError_t launch_update(const StepArgs& a, cudaStream_t s, bool from_unscaled, bool extensive, bool cells) {
   const int work = a.cell_problem && a.n_problems > a.mesh.n ? a.n_problems : a.mesh.n;
   if (work > 0) {
-    if (a.cell_problem)
-      k_update<true><<<grid_of(a.shapes.update, work), a.shapes.update.block, 0, s>>>(a, from_unscaled ? 1 : 0, extensive ? 1 : 0, cells ? 1 : 0);
-    else
-      k_update<false><<<grid_of(a.shapes.update, work), a.shapes.update.block, 0, s>>>(a, from_unscaled ? 1 : 0, extensive ? 1 : 0, cells ? 1 : 0);
+    const LaunchShape sh = fit_shape(a.shapes.update, work);
+    const int nb = grid_of(sh, work), bs = sh.block;
+    const bool b = a.cell_problem != nullptr;
+    if (extensive && cells) {
+      // (the fused update reads scaled fluxes)
+      if (a.ext_avg)
+        b ? k_update<true, kUpAverage><<<nb, bs, 0, s>>>(a) : k_update<false, kUpAverage><<<nb, bs, 0, s>>>(a);
+      else
+        b ? k_update<true, kUpFused><<<nb, bs, 0, s>>>(a) : k_update<false, kUpFused><<<nb, bs, 0, s>>>(a);
+    } else if (extensive && from_unscaled) {
+      b ? k_update<true, kUpUnscaled><<<nb, bs, 0, s>>>(a) : k_update<false, kUpUnscaled><<<nb, bs, 0, s>>>(a);
+    } else if (extensive) {
+      b ? k_update<true, kUpScaled><<<nb, bs, 0, s>>>(a) : k_update<false, kUpScaled><<<nb, bs, 0, s>>>(a);
+    } else {
+      b ? k_update<true, kUpCells><<<nb, bs, 0, s>>>(a) : k_update<false, kUpCells><<<nb, bs, 0, s>>>(a);
+    }
   }
   return cudaGetLastError();
 }

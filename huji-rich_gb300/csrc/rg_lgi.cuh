@@ -49,6 +49,16 @@ __device__ __forceinline__ float trunc32(double x, bool& ok) {
   const uint32_t t = __funnelshift_l(lo, hi, 3);
   return in ? __uint_as_float(((t ^ 0x40000000u) & 0x7fffffffu) | (hi & 0x80000000u)) : 0.0f;
 }
+// the same where a value below the normal floats may become 0 (an absolute
+// error of 2^-126)
+__device__ __forceinline__ float trunc32_any(double x, bool& ok) {
+  const uint64_t u = conv_dbits(x);
+  const uint32_t hi = static_cast<uint32_t>(u >> 32), lo = static_cast<uint32_t>(u);
+  const uint32_t m = hi & 0x7fffffffu;
+  ok = ok && m < 0x47f00000u;
+  const uint32_t t = __funnelshift_l(lo, hi, 3);
+  return m >= 0x38100000u ? __uint_as_float(((t ^ 0x40000000u) & 0x7fffffffu) | (hi & 0x80000000u)) : 0.0f;
+}
 // the same for a magnitude that only needs a lower bound: values below the
 // normal floats become 0
 __device__ __forceinline__ float trunc32_low(double x, bool& ok) {

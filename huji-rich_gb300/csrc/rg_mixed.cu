@@ -968,9 +968,18 @@ __device__ __forceinline__ void two_sum(float& s, float& c, float x) {
 // contribution enters its two cells with opposite signs and the extensives
 // keep FP64 precision across steps.  e = E/m - v^2/2 is formed in FP64 with a
 // Newton-refined reciprocal of m.
-template <bool kBatch>
-__device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArgs& a, int i, int from_unscaled,
-                                                               int do_ext, int do_cells) {
+// What one launch of the update kernel does: compile-time, since the FP64
+// instructions of a form that is off still take the FP64 unit where the
+// compiler predicates them (a warp's update has 15 of its own).
+constexpr int kUpFused = 0;     // extensives from the scaled fluxes, then the cells
+constexpr int kUpAverage = 1;   // the same, the extensives averaged with ext_avg (Heun)
+constexpr int kUpUnscaled = 2;  // extensives only, from unscaled fluxes
+constexpr int kUpScaled = 3;    // extensives only, from scaled fluxes
+constexpr int kUpCells = 4;     // cells only
+template <bool kBatch, int kMode>
+__device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArgs& a, int i) {
+  constexpr bool do_ext = kMode != kUpCells, do_cells = kMode != kUpUnscaled && kMode != kUpScaled;
+  constexpr bool from_unscaled = kMode == kUpUnscaled;
   const MeshDev& m = a.mesh;
   double2* ext2 = reinterpret_cast<double2*>(a.ext);
   const double2 e01 = ext2[2 * i], e23 = ext2[2 * i + 1];
@@ -996,7 +1005,7 @@ __device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArg
     en += widen(s1) + widen(c1);
     px += widen(s2) + widen(c2);
     py += widen(s3) + widen(c3);
-    if (a.ext_avg) {
+    if (kMode == kUpAverage) {
       const double2* o = reinterpret_cast<const double2*>(a.ext_avg);
       const double2 o01 = o[2 * i], o23 = o[2 * i + 1];
       mass = 0.5 * (mass + o01.x);
@@ -1042,7 +1051,7 @@ __device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArg
     // e = E/m - v^2/2 in FP64 (the cancellation at high Mach numbers)
     const double vx = px * r, vy = py * r;
     const double energy = en * r - 0.5 * (vx * vx + vy * vy);
-    if (energy < 0) {
+    if (lt(energy, 0.0)) {
       record_error(a.status, a.step, RG_ERR_NEGATIVE_ENERGY, 5, i, energy);
       return kInfBits;
     }
@@ -1071,11 +1080,11 @@ __device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArg
 
 // kMinBlocks > 0: register-capped builds for blocks of up to kCappedBlock
 // threads with kMinBlocks resident per SM (launch-shape variants 2 and 3)
-template <bool kBatch, int kMinBlocks = 0>
+template <bool kBatch, int kMode, int kMinBlocks = 0>
 __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 1)
-    k_update_mixed(MixedArgs a, int from_unscaled, int do_ext, int do_cells) {
+    k_update_mixed(MixedArgs a) {
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  if (kBatch && do_ext && !from_unscaled && !a.batch_keep_dt) {
+  if (kBatch && kMode <= kUpAverage && !a.batch_keep_dt) {
     for (int p = t0; p < a.n_problems; p += stride) {
       const double dt = a.cfl * __longlong_as_double(static_cast<long long>(a.dtmin_p[p]));
       a.dt_p[p] = dt;
@@ -1085,7 +1094,7 @@ __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlo
   }
   unsigned long long bits = kInfBits;
   for (int i = t0; i < a.mesh.n; i += stride) {
-    const unsigned long long b = k_update_mixed_item<kBatch>(a, i, from_unscaled, do_ext, do_cells);
+    const unsigned long long b = k_update_mixed_item<kBatch, kMode>(a, i);
     bits = b < bits ? b : bits;
   }
   if (!kBatch && a.cfl_next) grid_min_times(a.status, bits, a.cfl, &a.status->dt_next, &a.status->dt_next32);
@@ -1130,7 +1139,7 @@ __global__ void __launch_bounds__(kPersistBlock, 4)
       a.dtmin_p[p] = kInfBits;
       if (p == 0 && dt_trace) dt_trace[k] = dt;
     }
-    for (int i = t0; i < m.n; i += stride) k_update_mixed_item<true>(a, i, 0, 1, 1);
+    for (int i = t0; i < m.n; i += stride) k_update_mixed_item<true, kUpFused>(a, i);
     if (!grid_sync(gb, gen, expected, s_ok, a.status, a.step)) return;
   }
 }
@@ -1275,24 +1284,34 @@ cudaError_t launch_faces32(const MixedArgs& a, cudaStream_t s, bool scaled) {
   }
   return cudaGetLastError();
 }
+template <bool kBatch, int kMode>
+static void update_mixed_build(const MixedArgs& a, const LaunchShape& sh, int nb, cudaStream_t s) {
+  // builds: 0 plain, 2 and 3 register-capped for 5 and 6 resident blocks of up
+  // to 256 threads
+  switch (sh.variant) {
+    case 2: k_update_mixed<kBatch, kMode, 5><<<nb, sh.block, 0, s>>>(a); break;
+    case 3: k_update_mixed<kBatch, kMode, 6><<<nb, sh.block, 0, s>>>(a); break;
+    default: k_update_mixed<kBatch, kMode><<<nb, sh.block, 0, s>>>(a);
+  }
+}
 cudaError_t launch_update_mixed(const MixedArgs& a, cudaStream_t s, bool from_unscaled, bool extensive, bool cells) {
   const int work = a.cell_problem && a.n_problems > a.mesh.n ? a.n_problems : a.mesh.n;
   if (work > 0) {
-    const LaunchShape& sh = a.shapes.update;
-    const int nb = grid_of(sh, work), bs = sh.block;
-    const int fu = from_unscaled ? 1 : 0, ex = extensive ? 1 : 0, ce = cells ? 1 : 0;
+    const LaunchShape sh = fit_shape(a.shapes.update, work);
+    const int nb = grid_of(sh, work);
     const bool b = a.cell_problem != nullptr;
-    // builds: 0 plain, 2 and 3 register-capped for 5 and 6 resident blocks
-    // of up to 256 threads
-    switch (sh.variant) {
-      case 2:
-        b ? k_update_mixed<true, 5><<<nb, bs, 0, s>>>(a, fu, ex, ce) : k_update_mixed<false, 5><<<nb, bs, 0, s>>>(a, fu, ex, ce);
-        break;
-      case 3:
-        b ? k_update_mixed<true, 6><<<nb, bs, 0, s>>>(a, fu, ex, ce) : k_update_mixed<false, 6><<<nb, bs, 0, s>>>(a, fu, ex, ce);
-        break;
-      default:
-        b ? k_update_mixed<true><<<nb, bs, 0, s>>>(a, fu, ex, ce) : k_update_mixed<false><<<nb, bs, 0, s>>>(a, fu, ex, ce);
+    if (extensive && cells) {
+      // (the fused update reads scaled fluxes)
+      if (a.ext_avg)
+        b ? update_mixed_build<true, kUpAverage>(a, sh, nb, s) : update_mixed_build<false, kUpAverage>(a, sh, nb, s);
+      else
+        b ? update_mixed_build<true, kUpFused>(a, sh, nb, s) : update_mixed_build<false, kUpFused>(a, sh, nb, s);
+    } else if (extensive && from_unscaled) {
+      b ? update_mixed_build<true, kUpUnscaled>(a, sh, nb, s) : update_mixed_build<false, kUpUnscaled>(a, sh, nb, s);
+    } else if (extensive) {
+      b ? update_mixed_build<true, kUpScaled>(a, sh, nb, s) : update_mixed_build<false, kUpScaled>(a, sh, nb, s);
+    } else {
+      b ? update_mixed_build<true, kUpCells>(a, sh, nb, s) : update_mixed_build<false, kUpCells>(a, sh, nb, s);
     }
   }
   return cudaGetLastError();

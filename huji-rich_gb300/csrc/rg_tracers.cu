@@ -188,9 +188,10 @@ __global__ void __launch_bounds__(kTrBlock) k_tr_faces_pcm(StepArgs a, TracerArg
 // SimpleExtensiveUpdater for the extensive tracers (gather in ascending face
 // order) and SimpleCellUpdater's tracer part; runs after the hydro update,
 // whose new mass, density and pressure it reads.
-template <int NT>
-__global__ void __launch_bounds__(kTrBlock) k_tr_update(StepArgs a, TracerArgs t, int from_unscaled, int do_ext,
-                                                         int do_cells) {
+// kUnscaled, kAverage: template arguments, since the FP64 products of a form
+// that is off still take the FP64 unit where the compiler predicates them.
+template <int NT, bool kUnscaled, bool kAverage>
+__global__ void __launch_bounds__(kTrBlock) k_tr_update(StepArgs a, TracerArgs t, int do_ext, int do_cells) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
@@ -201,20 +202,16 @@ __global__ void __launch_bounds__(kTrBlock) k_tr_update(StepArgs a, TracerArgs t
 #pragma unroll
   for (int j = 0; j < kMaxTracers; ++j) te[j] = j < nt ? ext_t[j] : 0.0;
   if (do_ext) {
-    const double dt = from_unscaled ? step_dt(a) : 0.0;
+    const double dt = kUnscaled ? step_dt(a) : 0.0;
     for (int k = m.cell_off[i]; k < m.cell_off[i + 1]; ++k) {
       const int e = m.cell_faces[k];
-      const bool minus = (a.geom.nbr[k] & kNbrFirst) != 0;
-      const double s = from_unscaled ? dt * a.geom.xarea[e] : 1.0;
+      const uint32_t flip = a.geom.nbr[k] & kNbrFirst;  // bit 31
+      const double s = kUnscaled ? dt * a.geom.xarea[e] : 1.0;
       const double* f = t.tr_flux + static_cast<size_t>(e) * nt;
 #pragma unroll
       for (int j = 0; j < kMaxTracers; ++j) {
         if (j < nt) {
-          const double d = from_unscaled ? f[j] * s : f[j];
-          if (minus)
-            te[j] -= d;
-          else
-            te[j] += d;
+          te[j] += flip_sign(kUnscaled ? f[j] * s : f[j], flip);
         }
       }
     }
@@ -226,7 +223,7 @@ __global__ void __launch_bounds__(kTrBlock) k_tr_update(StepArgs a, TracerArgs t
         if (j < nt) te[j] *= f;
     }
   }
-  if (t.tr_ext_avg) {
+  if (kAverage) {
     // hdsim2d.cpp:311-320 average_extensive: 0.5*(mid + old)
     const double* o = t.tr_ext_avg + static_cast<size_t>(i) * nt;
 #pragma unroll
@@ -277,18 +274,20 @@ inline int tr_blocks(int n) { return (n + kTrBlock - 1) / kTrBlock; }
 
 }  // namespace
 
-// kernel K instantiated for NT = t.nt
-#define RG_TR_DISPATCH(K, grid, s, ...)                                  \
-  switch (t.nt) {                                                         \
-    case 1: K<1><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;           \
-    case 2: K<2><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;           \
-    case 3: K<3><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;           \
-    case 4: K<4><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;           \
-    case 5: K<5><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;           \
-    case 6: K<6><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;           \
-    case 7: K<7><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;           \
-    case 8: K<8><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;           \
-    default: break;                                                       \
+// k_tr_update for NT = t.nt
+#define RG_TR_CASE(NT, U, A, grid, s, ...) \
+  case NT: k_tr_update<NT, U, A><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;
+#define RG_TR_DISPATCH(U, A, grid, s, ...)  \
+  switch (t.nt) {                           \
+    RG_TR_CASE(1, U, A, grid, s, __VA_ARGS__) \
+    RG_TR_CASE(2, U, A, grid, s, __VA_ARGS__) \
+    RG_TR_CASE(3, U, A, grid, s, __VA_ARGS__) \
+    RG_TR_CASE(4, U, A, grid, s, __VA_ARGS__) \
+    RG_TR_CASE(5, U, A, grid, s, __VA_ARGS__) \
+    RG_TR_CASE(6, U, A, grid, s, __VA_ARGS__) \
+    RG_TR_CASE(7, U, A, grid, s, __VA_ARGS__) \
+    RG_TR_CASE(8, U, A, grid, s, __VA_ARGS__) \
+    default: break;                         \
   }
 
 cudaError_t launch_tr_slopes(const StepArgs& a, const TracerArgs& t, cudaStream_t s) {
@@ -314,8 +313,15 @@ cudaError_t launch_tr_faces(const StepArgs& a, const TracerArgs& t, cudaStream_t
 cudaError_t launch_tr_update(const StepArgs& a, const TracerArgs& t, cudaStream_t s, bool from_unscaled,
                              bool extensive, bool cells) {
   if (a.mesh.n > 0 && t.nt > 0 && t.nt <= kMaxTracers) {
-    const int fu = from_unscaled ? 1 : 0, ex = extensive ? 1 : 0, ce = cells ? 1 : 0;
-    RG_TR_DISPATCH(k_tr_update, tr_blocks(a.mesh.n), s, a, t, fu, ex, ce)
+    const int ex = extensive ? 1 : 0, ce = cells ? 1 : 0;
+    // (only the fused Heun step, whose fluxes are scaled, averages)
+    if (t.tr_ext_avg) {
+      RG_TR_DISPATCH(false, true, tr_blocks(a.mesh.n), s, a, t, ex, ce)
+    } else if (from_unscaled) {
+      RG_TR_DISPATCH(true, false, tr_blocks(a.mesh.n), s, a, t, ex, ce)
+    } else {
+      RG_TR_DISPATCH(false, false, tr_blocks(a.mesh.n), s, a, t, ex, ce)
+    }
   }
   return cudaGetLastError();
 }
