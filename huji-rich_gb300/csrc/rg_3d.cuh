@@ -30,7 +30,9 @@ struct Step3Args {
   Mesh3Dev mesh;
   const dbl4* nhat;       // unit normals (x, y, z, 0)
   const int* fsign;       // per CSR entry: face | bit 31 when the cell is the face's first neighbour
+  const unsigned char* axis;  // per face: the axis its normal lies along (k3_geometry)
   double gamma, cfl;
+  Divisor gm1;            // gamma - 1 as a divisor
   double* cells;          // 6 per cell
   double* ext;            // 6 per cell
   double* fluxes;         // 6 per face
@@ -39,6 +41,9 @@ struct Step3Args {
   double dt_host;
   int dt_from_device;
   int step;
+  int cfl_next;           // the fused update also computes the next step's dt (status->dt_next)
+  int take_next_dt;       // the face kernel moves status->dt_next to status->dt and scales by it
+  double* dt_trace;       // where the step's dt is kept, or nullptr
 };
 
 // FP32-mixed 3D path (rg_3d_mixed.cu): FP32 primitives, unit normals,
@@ -63,6 +68,8 @@ struct Mixed3Args {
   float dt32;                 // dt given by the caller (split API)
   int dt_from_device;
   int step;
+  int cfl_next, take_next_dt;  // as Step3Args
+  double* dt_trace;
 };
 
 cudaError_t launch3m_geometry(const Mesh3Dev& m, const dbl4* nhat, float4* nhat32, float* area32, float* width32,
@@ -79,7 +86,7 @@ cudaError_t launch3m_update(const Mixed3Args& a, bool from_unscaled, bool do_ext
 cudaError_t launch3_unpack(const double* packed, double* rec, int rows, cudaStream_t s);
 cudaError_t launch3_pack(const double* rec, double* packed, int rows, cudaStream_t s);
 cudaError_t launch3_validate(const Mesh3Dev& m, DevStatus* st, cudaStream_t s);
-cudaError_t launch3_geometry(const Mesh3Dev& m, dbl4* nhat, int* fsign, cudaStream_t s);
+cudaError_t launch3_geometry(const Mesh3Dev& m, dbl4* nhat, int* fsign, unsigned char* axis, cudaStream_t s);
 cudaError_t launch3_init_extensives(const Step3Args& a, cudaStream_t s);
 cudaError_t launch3_cfl(const Step3Args& a, cudaStream_t s);
 // scaled: fluxes times dt*area (the fused step); otherwise the reference's

@@ -8,7 +8,6 @@
 #include <algorithm>
 #include <cstring>
 #include <new>
-#include <vector>
 
 #include "rg_3d.cuh"
 
@@ -42,9 +41,16 @@ struct rg3_handle {
   cudaStream_t stream = nullptr;
   int n = 0, e = 0, m = 0;
   bool have_mesh = false, have_cells = false, have_ext = false, have_fluxes = false;
-  Buf face_cells, normal, area, volume, width, cell_off, cell_faces, nhat, fsign;
+  Buf face_cells, normal, area, volume, width, cell_off, cell_faces, nhat, fsign, axis;
   Buf cells, ext, fluxes, fvel, status_buf;
   Buf stage;  // 5-double records on their way to or from the host
+  // status->dt_next is the next step's dt (the last fused update's); any other
+  // change of the cells or the mesh clears it
+  bool dt_next_ready = false;
+  Buf dt_trace;                  // rg3_run's dt of each step
+  double* step_trace = nullptr;  // where the step being enqueued keeps its dt
+  double* h_dts = nullptr;       // pinned, h_dts_len doubles
+  size_t h_dts_len = 0;
   bool fvel_set = false;
   // FP32-mixed path (rg_config.precision == RG_FP32_MIXED)
   bool mixed = false;
@@ -86,6 +92,7 @@ rg_status collect(rg3_handle* h, double* dt = nullptr) {
   RG3_CUDA(h, cudaGetLastError());
   if (dt) *dt = h->h_status->dt;
   if (h->h_status->err_key != ~0ull) {
+    h->dt_next_ready = false;
     const unsigned long long key = h->h_status->err_key;
     h->last = rg_error{h->h_status->err_status, static_cast<int32_t>((key >> rg::kKeyPhaseShift) & 0xf),
                        static_cast<int64_t>(key & rg::kKeyIndexMask), h->h_status->err_value};
@@ -109,7 +116,9 @@ rg::Step3Args args(rg3_handle* h) {
   a.mesh.cell_faces = static_cast<const int*>(h->cell_faces.p);
   a.nhat = static_cast<const rg::dbl4*>(h->nhat.p);
   a.fsign = static_cast<const int*>(h->fsign.p);
+  a.axis = static_cast<const unsigned char*>(h->axis.p);
   a.gamma = h->cfg.gamma;
+  a.gm1 = rg::divisor(h->cfg.gamma - 1, rg::RcpSeedHost{});
   a.cfl = h->cfg.cfl;
   a.cells = static_cast<double*>(h->cells.p);
   a.ext = static_cast<double*>(h->ext.p);
@@ -179,28 +188,38 @@ rg_status get5(rg3_handle* h, double* dst, const Buf& src, int rows) {
   return RG_OK;
 }
 
+// One fused step: the CFL pass only where the previous step's update has not
+// left this step's dt.
 rg_status enqueue_step(rg3_handle* h, int step, bool timed = false) {
+  const bool have_dt = h->dt_next_ready;
   if (timed) RG3_CUDA(h, cudaEventRecord(h->ev[0], h->stream));
   if (h->mixed) {
     rg::Mixed3Args a = margs(h);
     a.dt_from_device = 1;
     a.step = step;
-    RG3_CUDA(h, rg::launch3m_cfl(a, h->stream));
+    a.dt_trace = h->step_trace;
+    if (!have_dt) RG3_CUDA(h, rg::launch3m_cfl(a, h->stream));
     if (timed) RG3_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
+    a.take_next_dt = have_dt;
     RG3_CUDA(h, rg::launch3m_faces(a, true, h->stream));
     if (timed) RG3_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
+    a.cfl_next = 1;
     RG3_CUDA(h, rg::launch3m_update(a, false, true, true, h->stream));
   } else {
     rg::Step3Args a = args(h);
     a.dt_from_device = 1;
     a.step = step;
-    RG3_CUDA(h, rg::launch3_cfl(a, h->stream));
+    a.dt_trace = h->step_trace;
+    if (!have_dt) RG3_CUDA(h, rg::launch3_cfl(a, h->stream));
     if (timed) RG3_CUDA(h, cudaEventRecord(h->ev[1], h->stream));
+    a.take_next_dt = have_dt;
     RG3_CUDA(h, rg::launch3_faces(a, true, h->stream));
     if (timed) RG3_CUDA(h, cudaEventRecord(h->ev[2], h->stream));
+    a.cfl_next = 1;
     RG3_CUDA(h, rg::launch3_update(a, false, true, true, h->stream));
   }
   if (timed) RG3_CUDA(h, cudaEventRecord(h->ev[3], h->stream));
+  h->dt_next_ready = true;
   h->have_fluxes = false;
   return RG_OK;
 }
@@ -252,9 +271,10 @@ rg_status rg3_destroy(rg3_handle* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (Buf* b : {&h->face_cells, &h->normal, &h->area, &h->volume, &h->width, &h->cell_off, &h->cell_faces,
                  &h->nhat, &h->fsign, &h->cells, &h->ext, &h->fluxes, &h->fvel, &h->status_buf, &h->nhat32,
-                 &h->area32, &h->width32, &h->cells32, &h->vz32, &h->flux32, &h->fen32, &h->fvel32, &h->stage})
+                 &h->area32, &h->width32, &h->cells32, &h->vz32, &h->flux32, &h->fen32, &h->fvel32, &h->stage, &h->axis, &h->dt_trace})
     b->release();
   if (h->h_status) cudaFreeHost(h->h_status);
+  if (h->h_dts) cudaFreeHost(h->h_dts);
   for (cudaEvent_t& v : h->ev)
     if (v) cudaEventDestroy(v);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -271,6 +291,7 @@ rg_status rg3_last_error(const rg3_handle* h, rg_error* err) {
 
 rg_status rg3_upload_mesh(rg3_handle* h, const rg_mesh3d_view* v) {
   if (!h) return RG_ERR_INVALID_ARGUMENT;
+  h->dt_next_ready = false;
   h->last = rg_error{};
   auto bad = [h](int64_t idx) {
     h->last = rg_error{RG_ERR_INVALID_ARGUMENT, 0, idx, 0};
@@ -294,6 +315,7 @@ rg_status rg3_upload_mesh(rg3_handle* h, const rg_mesh3d_view* v) {
   RG3_CUDA(h, h->cell_faces.ensure(4 * M));
   RG3_CUDA(h, h->nhat.ensure(32 * E));
   RG3_CUDA(h, h->fsign.ensure(4 * M));
+  RG3_CUDA(h, h->axis.ensure(E));
   RG3_CUDA(h, h->fluxes.ensure(48 * E));
   RG3_CUDA(h, h->fvel.ensure(24 * E));
   if (n != h->n) h->have_cells = h->have_ext = false;
@@ -323,7 +345,7 @@ rg_status rg3_upload_mesh(rg3_handle* h, const rg_mesh3d_view* v) {
     return RG_ERR_INVALID_ARGUMENT;
   }
   RG3_CUDA(h, rg::launch3_geometry(a.mesh, static_cast<rg::dbl4*>(h->nhat.p), static_cast<int*>(h->fsign.p),
-                                   h->stream));
+                                   static_cast<unsigned char*>(h->axis.p), h->stream));
   if (h->mixed) {
     RG3_CUDA(h, h->nhat32.ensure(16 * E));
     RG3_CUDA(h, h->area32.ensure(4 * E));
@@ -345,6 +367,7 @@ rg_status rg3_upload_mesh(rg3_handle* h, const rg_mesh3d_view* v) {
 rg_status rg3_set_cells(rg3_handle* h, const double* cells) {
   if (!h || !cells) return RG_ERR_INVALID_ARGUMENT;
   if (!h->have_mesh) return not_ready(h);
+  h->dt_next_ready = false;
   if (rg_status st = put5(h, h->cells, cells, h->n)) return st;
   if (h->mixed) {
     RG3_CUDA(h, rg::launch3m_cells_to32(static_cast<const double*>(h->cells.p), static_cast<float4*>(h->cells32.p),
@@ -451,6 +474,7 @@ rg_status rg3_cell_update(rg3_handle* h) {
   if (!h) return RG_ERR_INVALID_ARGUMENT;
   if (!h->have_ext) return not_ready(h);
   h->last = rg_error{};
+  h->dt_next_ready = false;
   if (rg_status st = reset(h)) return st;
   if (h->mixed)
     RG3_CUDA(h, rg::launch3m_update(margs(h), false, false, true, h->stream));
@@ -489,24 +513,27 @@ rg_status rg3_run(rg3_handle* h, int32_t n_steps, double* dts) {
   if (!h->have_cells || !h->have_ext) return not_ready(h);
   h->last = rg_error{};
   if (rg_status st = reset(h)) return st;
-  std::vector<double> hd;
-  double* pinned = nullptr;
-  if (dts && n_steps > 0) RG3_CUDA(h, cudaMallocHost(&pinned, sizeof(double) * static_cast<size_t>(n_steps)));
+  const size_t steps = static_cast<size_t>(n_steps);
+  if (dts && steps > 0) {
+    if (steps > h->h_dts_len) {
+      if (h->h_dts) cudaFreeHost(h->h_dts);
+      h->h_dts = nullptr;
+      h->h_dts_len = 0;
+      RG3_CUDA(h, cudaMallocHost(&h->h_dts, sizeof(double) * steps));
+      h->h_dts_len = steps;
+    }
+    RG3_CUDA(h, h->dt_trace.ensure(sizeof(double) * steps));
+  }
   rg_status st = RG_OK;
   for (int k = 0; k < n_steps && st == RG_OK; ++k) {
+    h->step_trace = dts ? static_cast<double*>(h->dt_trace.p) + k : nullptr;
     st = enqueue_step(h, std::min(k, 0x1fff));
-    if (st == RG_OK && pinned) {
-      const cudaError_t ce = cudaMemcpyAsync(pinned + k, &h->d_status->dt, sizeof(double), cudaMemcpyDeviceToHost,
-                                             h->stream);
-      if (ce != cudaSuccess) st = fail(h, ce);
-    }
   }
+  h->step_trace = nullptr;
+  if (st == RG_OK && dts && steps > 0)
+    RG3_CUDA(h, cudaMemcpyAsync(h->h_dts, h->dt_trace.p, sizeof(double) * steps, cudaMemcpyDeviceToHost, h->stream));
   if (st == RG_OK) st = collect(h);
-  if (pinned) {
-    cudaStreamSynchronize(h->stream);
-    if (dts) std::memcpy(dts, pinned, sizeof(double) * static_cast<size_t>(n_steps));
-    cudaFreeHost(pinned);
-  }
+  if (dts && steps > 0) std::memcpy(dts, h->h_dts, sizeof(double) * steps);
   return st;
 }
 

@@ -6,6 +6,7 @@
 // Mach numbers).  Same structure as the FP64 kernels in rg_3d.cu.
 #include <math.h>
 
+#include "rg_launch.cuh"
 #include "rg_3d.cuh"
 #include "rg_convert.cuh"
 #include "rg_hllc.cuh"
@@ -110,19 +111,28 @@ __global__ void __launch_bounds__(kBlock) k3m_flux_to64(const float4* f32, const
   o[5] = 0.0;
 }
 
+// cell i's CFL bound, as the bit pattern of its FP64 value
+__device__ __forceinline__ unsigned long long cfl3m_bits(const Mixed3Args& a, int i, const C3& c) {
+  const float b = a.width32[i] / (fabs3(c.v) + sqrtf(a.gamma * c.p / c.d));
+  return static_cast<unsigned long long>(__double_as_longlong(widen_exact(b)));
+}
+
 __global__ void __launch_bounds__(kBlock) k3m_cfl(Mixed3Args a) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned long long bits = kInfBits;
-  if (i < a.mesh.n) {
-    const C3 c = load32(a, i);
-    const float b = a.width32[i] / (fabs3(c.v) + sqrtf(a.gamma * c.p / c.d));
-    bits = static_cast<unsigned long long>(__double_as_longlong(widen_exact(b)));
-  }
-  grid_min_times(a.status, bits, a.cfl, &a.status->dt, &a.status->dt32);
+  const unsigned long long bits = i < a.mesh.n ? cfl3m_bits(a, i, load32(a, i)) : kInfBits;
+  grid_min_times(a.status, bits, a.cfl, &a.status->dt, &a.status->dt32, a.dt_trace);
 }
 
 template <bool kScaled>
 __global__ void __launch_bounds__(kBlock) k3m_faces(Mixed3Args a) {
+  chain_wait();
+  if (a.take_next_dt && blockIdx.x == 0 && threadIdx.x == 0) {
+    const double dt = a.status->dt_next;
+    a.status->dt = dt;
+    a.status->dt32 = a.status->dt_next32;
+    if (a.dt_trace) *a.dt_trace = dt;
+  }
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= a.mesh.e) return;
   const int2 fc = a.mesh.face_cells[f];
@@ -151,27 +161,29 @@ __global__ void __launch_bounds__(kBlock) k3m_faces(Mixed3Args a) {
     par = parallel32(sol.m > 0.0f ? ca.v : cb.v, n);
   }
   const F3 mom{fmaf(sol.my, par.x, sol.mx * n.x), fmaf(sol.my, par.y, sol.mx * n.y), fmaf(sol.my, par.z, sol.mx * n.z)};
-  const float s = kScaled ? (a.dt_from_device ? a.status->dt32 : a.dt32) * a.area32[f] : 1.0f;
+  const float s =
+      kScaled ? (a.take_next_dt ? a.status->dt_next32 : (a.dt_from_device ? a.status->dt32 : a.dt32)) * a.area32[f] : 1.0f;
   a.flux32[f] = make_float4(s * sol.m, s * mom.x, s * mom.y, s * mom.z);
   a.fen32[f] = s * sol.en;
 }
 
-__global__ void __launch_bounds__(kBlock) k3m_update(Mixed3Args a, int from_unscaled, int do_ext, int do_cells) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// kUnscaled / kExt / kCells: template arguments, as the FP64 update's.  Returns
+// whether c holds the cell's new state.
+template <bool kUnscaled, bool kExt, bool kCells>
+__device__ __forceinline__ bool update_cell3m(const Mixed3Args& a, int i, C3& cell) {
   const Mesh3Dev& m = a.mesh;
-  if (i >= m.n) return;
   double2* e2 = reinterpret_cast<double2*>(a.ext) + 3 * i;
   const double2 e01 = e2[0], e23 = e2[1], e45 = e2[2];
   double u[5] = {e01.x, e01.y, e23.x, e23.y, e45.x};
-  if (do_ext) {
+  if (kExt) {
     float s[5] = {0, 0, 0, 0, 0}, c[5] = {0, 0, 0, 0, 0};
-    const float dt = from_unscaled ? (a.dt_from_device ? a.status->dt32 : a.dt32) : 1.0f;
+    const float dt = kUnscaled ? (a.dt_from_device ? a.status->dt32 : a.dt32) : 1.0f;
     for (int k = m.cell_off[i]; k < m.cell_off[i + 1]; ++k) {
       const int fs = a.fsign[k];
       const int f = fs & 0x7fffffff;
       const float4 v = a.flux32[f];
       float d[5] = {v.x, v.y, v.z, v.w, a.fen32[f]};
-      const float sc = from_unscaled ? dt * a.area32[f] : 1.0f;
+      const float sc = kUnscaled ? dt * a.area32[f] : 1.0f;
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
         // a separately rounded product (no contraction into the sum): the
@@ -186,7 +198,7 @@ __global__ void __launch_bounds__(kBlock) k3m_update(Mixed3Args a, int from_unsc
     e2[1] = make_double2(u[2], u[3]);
     e2[2] = make_double2(u[4], 0.0);
   }
-  if (do_cells) {
+  if (kCells) {
     const double V = m.volume[i];
     const float mf = narrow(u[0]);
     // 1/m from the FP32 reciprocal and one Newton step
@@ -194,15 +206,26 @@ __global__ void __launch_bounds__(kBlock) k3m_update(Mixed3Args a, int from_unsc
     r = r * (2.0 - u[0] * r);
     const double vx = u[1] * r, vy = u[2] * r, vz = u[3] * r;
     const double eint = u[4] * r - 0.5 * (vx * vx + vy * vy + vz * vz);  // FP64: the cancellation
-    if (eint < 0) {
+    if (lt(eint, 0.0)) {
       record_error(a.status, a.step, RG_ERR_NEGATIVE_ENERGY, 5, i, eint);
-      return;
+      return false;
     }
     // m / V in FP32 from the rounded mass and volume (the result is stored in FP32)
     const float d = mf / narrow(V);
-    a.cells32[i] = make_float4(d, (a.gamma - 1.0f) * narrow(eint) * d, narrow(vx), narrow(vy));
-    a.vz32[i] = narrow(vz);
+    cell = C3{d, (a.gamma - 1.0f) * narrow(eint) * d, F3{narrow(vx), narrow(vy), narrow(vz)}};
+    a.cells32[i] = make_float4(cell.d, cell.p, cell.v.x, cell.v.y);
+    a.vz32[i] = cell.v.z;
   }
+  return kCells;
+}
+template <bool kUnscaled, bool kExt, bool kCells>
+__global__ void __launch_bounds__(kBlock) k3m_update(Mixed3Args a) {
+  chain_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  C3 c{1.0f, 1.0f, F3{0.0f, 0.0f, 0.0f}};
+  const bool live = i < a.mesh.n && update_cell3m<kUnscaled, kExt, kCells>(a, i, c);
+  if (kExt && kCells && a.cfl_next)
+    grid_min_times(a.status, live ? cfl3m_bits(a, i, c) : kInfBits, a.cfl, &a.status->dt_next, &a.status->dt_next32);
 }
 
 __global__ void __launch_bounds__(kBlock) k3m_d2f(const double* a, float* b, int n) {
@@ -237,19 +260,27 @@ cudaError_t launch3m_flux_to64(const float4* f32, const float* fen32, double* f6
   return cudaGetLastError();
 }
 cudaError_t launch3m_cfl(const Mixed3Args& a, cudaStream_t s) {
-  k3m_cfl<<<blocks(a.mesh.n), kBlock, 0, s>>>(a);
+  chain(s, blocks(a.mesh.n), kBlock, k3m_cfl, a);
   return cudaGetLastError();
 }
 cudaError_t launch3m_faces(const Mixed3Args& a, bool scaled, cudaStream_t s) {
   if (a.mesh.e == 0) return cudaSuccess;
   if (scaled)
-    k3m_faces<true><<<blocks(a.mesh.e), kBlock, 0, s>>>(a);
+    chain(s, blocks(a.mesh.e), kBlock, k3m_faces<true>, a);
   else
-    k3m_faces<false><<<blocks(a.mesh.e), kBlock, 0, s>>>(a);
+    chain(s, blocks(a.mesh.e), kBlock, k3m_faces<false>, a);
   return cudaGetLastError();
 }
 cudaError_t launch3m_update(const Mixed3Args& a, bool from_unscaled, bool do_ext, bool do_cells, cudaStream_t s) {
-  k3m_update<<<blocks(a.mesh.n), kBlock, 0, s>>>(a, from_unscaled ? 1 : 0, do_ext ? 1 : 0, do_cells ? 1 : 0);
+  const int nb = blocks(a.mesh.n);
+  if (do_ext && do_cells)
+    chain(s, nb, kBlock, k3m_update<false, true, true>, a);  // (the fused step's fluxes are scaled)
+  else if (do_ext && from_unscaled)
+    chain(s, nb, kBlock, k3m_update<true, true, false>, a);
+  else if (do_ext)
+    chain(s, nb, kBlock, k3m_update<false, true, false>, a);
+  else
+    chain(s, nb, kBlock, k3m_update<false, false, true>, a);
   return cudaGetLastError();
 }
 

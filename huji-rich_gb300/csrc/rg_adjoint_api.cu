@@ -47,11 +47,11 @@ struct rg_adjoint_state {
   DevBuf ubar0, ubar1, side_bar, self_bar, entry_bar, io;
   DevBuf dcells, dslopes, dflux, dext;
   // FP32-mixed recomputation: the interval's running FP32 primitives and extensives
-  DevBuf w_cells32, w_ext;
+  DevBuf w_cells32;
   void release() {
     for (DevBuf* b : {&side_off, &sides, &target_off, &targets, &ckpt_cells, &ckpt_ext, &final_ext, &seg_cells,
                       &seg_ext, &seg_slopes, &seg_trace, &ubar0, &ubar1, &side_bar, &self_bar, &entry_bar, &io,
-                      &dcells, &dslopes, &dflux, &dext, &w_cells32, &w_ext})
+                      &dcells, &dslopes, &dflux, &dext, &w_cells32})
       b->release();
     adjacency = have_forward = false;
   }
@@ -183,7 +183,6 @@ rg_status ensure_adjacency(rg_handle* h) {
 // The plain FP64 step with a fixed dt, from a.cells / a.ext into
 // a.cells_out / a.ext_out (nullptr: in place).
 rg_status enqueue_plain_step(rg_handle* h, const rg::StepArgs& a, bool faces_and_update = true) {
-  RG_CUDA(h, rg::launch_ghost_fill(a, h->stream));
   RG_CUDA(h, rg::launch_slopes(a, h->stream));
   if (faces_and_update) {
     RG_CUDA(h, rg::launch_faces(a, h->stream, true));
@@ -307,7 +306,6 @@ rg_status rg_step_bwd(rg_handle* h, const double* cells_bar, double* cells0_bar)
   a.dt_host = A->dt;
   if (h->mixed) {
     RG_CUDA(h, A->w_cells32.ensure(16 * np));
-    RG_CUDA(h, A->w_ext.ensure(32 * n));
   }
   for (int c = A->n_ckpt - 1; c >= 0 && h->mixed; --c) {
     // FP32-mixed: recompute the interval with the mixed kernels, recording
@@ -316,15 +314,15 @@ rg_status rg_step_bwd(rg_handle* h, const double* cells_bar, double* cells0_bar)
     const int len = std::min(A->every, A->n_steps - start);
     RG_CUDA(h, cudaMemcpyAsync(A->w_cells32.p, ptr<double>(A->ckpt_cells, 4 * n * static_cast<size_t>(c)), 16 * n,
                                cudaMemcpyDeviceToDevice, h->stream));
-    RG_CUDA(h, cudaMemcpyAsync(A->w_ext.p, ptr<double>(A->ckpt_ext, 4 * n * static_cast<size_t>(c)), 32 * n,
+    RG_CUDA(h, cudaMemcpyAsync(A->seg_ext.p, ptr<double>(A->ckpt_ext, 4 * n * static_cast<size_t>(c)), 32 * n,
                                cudaMemcpyDeviceToDevice, h->stream));
     rg::MixedArgs mx = mixed_fixed_dt(h, A->dt);
     mx.cells32 = static_cast<float4*>(A->w_cells32.p);
-    mx.ext = ptr<double>(A->w_ext);
     for (int j = 0; j < len; ++j) {
       const size_t J = static_cast<size_t>(j);
-      RG_CUDA(h, cudaMemcpyAsync(ptr<double>(A->seg_ext, 4 * n * J), A->w_ext.p, 32 * n, cudaMemcpyDeviceToDevice,
-                                 h->stream));
+      // each step's update writes its extensives into the next step's record
+      mx.ext = ptr<double>(A->seg_ext, 4 * n * J);
+      mx.ext_out = ptr<double>(A->seg_ext, 4 * n * (J + 1));
       RG_CUDA(h, rg::launch_cells_to64(mx.cells32, ptr<double>(A->seg_cells, 4 * np * J), s->n, h->stream));
       RG_CUDA(h, rg::launch_slopes32_trace(mx, ptr<double>(A->seg_slopes, 8 * n * J),
                                            ptr<rg::SlopeTrace>(A->seg_trace, n * J), h->stream));
@@ -365,7 +363,6 @@ rg_status rg_step_bwd(rg_handle* h, const double* cells_bar, double* cells0_bar)
       aj.slopes = ptr<double>(A->seg_slopes, 8 * n * J);
       aj.cells_out = ptr<double>(A->seg_cells, 4 * np * (J + 1));
       aj.ext_out = ptr<double>(A->seg_ext, 4 * n * (J + 1));
-      RG_CUDA(h, rg::launch_ghost_fill(aj, h->stream));
       rg::AdjArgs r = base;
       r.cells = aj.cells;
       r.slopes = aj.slopes;

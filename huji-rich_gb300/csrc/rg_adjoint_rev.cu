@@ -26,6 +26,7 @@
 // one-sided derivative.
 #include <math.h>
 
+#include "rg_launch.cuh"
 #include "rg_adjoint.cuh"
 #include "rg_div.cuh"
 
@@ -116,6 +117,7 @@ __device__ __forceinline__ void cell_update_transpose(double gamma, double V, co
 }
 
 __global__ void __launch_bounds__(kBlock) k_adj_seed(AdjArgs a, const double* wbar, double* ubar) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.mesh.n) return;
   double u[4], w[4], ub[4] = {0, 0, 0, 0};
@@ -260,6 +262,7 @@ __device__ __forceinline__ void face_state(const AdjArgs& a, int pid, rv2 dm, re
 }
 
 __global__ void __launch_bounds__(kBlock) k_adj_faces(AdjArgs a, const double* ubar) {
+  chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (e >= m.e) return;
@@ -292,6 +295,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_faces(AdjArgs a, const double* u
 }
 
 __global__ void __launch_bounds__(kBlock) k_adj_cell(AdjArgs a) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
@@ -374,6 +378,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_cell(AdjArgs a) {
 #if RG_ADJ_FP64
 __global__ void __launch_bounds__(kBlock) k_adj_update(AdjArgs a, const double* ubar_in, double* ubar_out,
                                                        double* grad) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
@@ -422,27 +427,27 @@ cudaError_t adj_launch_check(const AdjArgs& a, cudaStream_t s) {
 }
 
 cudaError_t adj_launch_seed(const AdjArgs& a, const double* wbar, double* ubar, cudaStream_t s) {
-  k_adj_seed<<<blocks(a.mesh.n), kBlock, 0, s>>>(a, wbar, ubar);
+  chain(s, blocks(a.mesh.n), kBlock, k_adj_seed, a, wbar, ubar);
   return cudaGetLastError();
 }
 
 cudaError_t adj_launch_update(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
                               cudaStream_t s) {
-  k_adj_update<<<blocks(a.mesh.n), kBlock, 0, s>>>(a, ubar_in, ubar_out, grad);
+  chain(s, blocks(a.mesh.n), kBlock, k_adj_update, a, ubar_in, ubar_out, grad);
   return cudaGetLastError();
 }
 
 cudaError_t adj_launch_reverse(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
                                cudaStream_t s) {
-  k_adj_faces<<<blocks(a.mesh.e), kBlock, 0, s>>>(a, ubar_in);
-  k_adj_cell<<<blocks(a.mesh.n), kBlock, 0, s>>>(a);
+  chain(s, blocks(a.mesh.e), kBlock, k_adj_faces, a, ubar_in);
+  chain(s, blocks(a.mesh.n), kBlock, k_adj_cell, a);
   return adj_launch_update(a, ubar_in, ubar_out, grad, s);
 }
 #else
 cudaError_t adj_launch_reverse32(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
                                  cudaStream_t s) {
-  k_adj_faces<<<blocks(a.mesh.e), kBlock, 0, s>>>(a, ubar_in);
-  k_adj_cell<<<blocks(a.mesh.n), kBlock, 0, s>>>(a);
+  chain(s, blocks(a.mesh.e), kBlock, k_adj_faces, a, ubar_in);
+  chain(s, blocks(a.mesh.n), kBlock, k_adj_cell, a);
   return adj_launch_update(a, ubar_in, ubar_out, grad, s);
 }
 #endif

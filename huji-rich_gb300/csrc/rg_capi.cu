@@ -196,6 +196,7 @@ rg::StepArgs step_args(rg_handle* h) {
   a.dt_host = 0;
   a.dt_from_device = 0;
   a.step = 0;
+  a.dt_trace = h->step_trace;
   a.shapes = h->shapes64;
   a.ev_zero = h->ev_zero && !h->external_state;
   if (h->n_problems > 0) {
@@ -262,6 +263,7 @@ rg::MixedArgs mixed_args(rg_handle* h) {
   a.dt32 = 0;
   a.dt32_from_device = 0;
   a.step = 0;
+  a.dt_trace = h->step_trace;
   a.shapes = h->shapes32;
   a.ev_zero = h->ev_zero && !h->external_state;
   if (h->n_problems > 0) {
@@ -319,10 +321,10 @@ rg_status mesh_error(rg_handle* h) {
 
 namespace {
 
-// Fused steps (the update computes the next step's dt): one problem, order 2
-// (the slopes kernel moves the dt into place before the face kernel reads
-// it), no caller access to the device buffers.
-bool fusable(const rg_handle* h) { return h->cfg.order == 2 && h->n_problems == 0 && !h->external_state; }
+// Fused steps (the update computes the next step's dt): one problem, no caller
+// access to the device buffers.  The dt is moved into place by the slopes
+// kernel, or by the face kernel at first order.
+bool fusable(const rg_handle* h) { return h->n_problems == 0 && !h->external_state; }
 
 // hdsim::TimeAdvance2Heun on a fixed mesh (hdsim2d.cpp:323-449): dt once;
 // pass 1 on the cells writes the mid extensives and mid cells; pass 2 on the
@@ -337,7 +339,7 @@ rg_status enqueue_heun(rg_handle* h, int step, cudaEvent_t* ev) {
     float4* mid_c = static_cast<float4*>(h->mid_cells32.p);
     double* mid_e = static_cast<double*>(h->mid_ext.p);
     if (ev) RG_CUDA(h, cudaEventRecord(ev[0], h->stream));
-    RG_CUDA(h, rg::launch_cfl32(a, h->stream, o2));
+    RG_CUDA(h, rg::launch_cfl32(a, h->stream));
     if (ev) RG_CUDA(h, cudaEventRecord(ev[1], h->stream));
     if (o2) RG_CUDA(h, rg::launch_slopes32(a, h->stream));
     RG_CUDA(h, rg::launch_faces32(a, h->stream, true));
@@ -350,7 +352,6 @@ rg_status enqueue_heun(rg_handle* h, int step, cudaEvent_t* ev) {
     rg::MixedArgs a2 = a;
     a2.cells32 = mid_c;
     if (o2) {
-      RG_CUDA(h, rg::launch_ghost_fill32(a2, h->stream));
       RG_CUDA(h, rg::launch_slopes32(a2, h->stream));
     }
     RG_CUDA(h, rg::launch_faces32(a2, h->stream, true));
@@ -379,7 +380,7 @@ rg_status enqueue_heun(rg_handle* h, int step, cudaEvent_t* ev) {
     ta3.tr_ext_out = ta.tr_ext;
     ta3.tr_ext_avg = ta.tr_ext;
     if (ev) RG_CUDA(h, cudaEventRecord(ev[0], h->stream));
-    RG_CUDA(h, rg::launch_cfl(a, h->stream, o2));
+    RG_CUDA(h, rg::launch_cfl(a, h->stream));
     if (ev) RG_CUDA(h, cudaEventRecord(ev[1], h->stream));
     if (o2) {
       RG_CUDA(h, rg::launch_slopes(a, h->stream));
@@ -397,7 +398,6 @@ rg_status enqueue_heun(rg_handle* h, int step, cudaEvent_t* ev) {
     rg::StepArgs a2 = a;
     a2.cells = mid_c;
     if (o2) {
-      RG_CUDA(h, rg::launch_ghost_fill(a2, h->stream));
       RG_CUDA(h, rg::launch_slopes(a2, h->stream));
       if (tr) RG_CUDA(h, rg::launch_tr_slopes(a2, ta2, h->stream));
     }
@@ -434,14 +434,17 @@ rg_status enqueue_step(rg_handle* h, int step, cudaEvent_t* ev = nullptr) {
     a64.step = step;
     const rg::TracerArgs ta = tracer_args(h);
     if (ev) RG_CUDA(h, cudaEventRecord(ev[0], h->stream));
-    if (!have_dt) RG_CUDA(h, rg::launch_cfl32(a, h->stream, false));
+    if (!have_dt) RG_CUDA(h, rg::launch_cfl32(a, h->stream));
     if (ev) RG_CUDA(h, cudaEventRecord(ev[1], h->stream));
     a.take_next_dt = have_dt;
-    if (h->cfg.order == 2) RG_CUDA(h, rg::launch_slopes32(a, h->stream));
-    a.take_next_dt = 0;
+    if (h->cfg.order == 2) {
+      RG_CUDA(h, rg::launch_slopes32(a, h->stream));
+      a.take_next_dt = 0;
+    }
     if (tr && h->cfg.order == 2) RG_CUDA(h, rg::launch_tr_slopes(a64, ta, h->stream));
     if (ev) RG_CUDA(h, cudaEventRecord(ev[2], h->stream));
     RG_CUDA(h, rg::launch_faces32(a, h->stream, true));
+    a.take_next_dt = 0;
     if (tr) RG_CUDA(h, rg::launch_tr_faces(a64, ta, h->stream, true));
     if (ev) RG_CUDA(h, cudaEventRecord(ev[3], h->stream));
     a.cfl_next = fuse;
@@ -464,14 +467,17 @@ rg_status enqueue_step(rg_handle* h, int step, cudaEvent_t* ev = nullptr) {
   const bool tr = h->tcfg.n_tracers > 0;
   const rg::TracerArgs ta = tracer_args(h);
   if (ev) RG_CUDA(h, cudaEventRecord(ev[0], h->stream));
-  if (!have_dt) RG_CUDA(h, rg::launch_cfl(a, h->stream, false));
+  if (!have_dt) RG_CUDA(h, rg::launch_cfl(a, h->stream));
   if (ev) RG_CUDA(h, cudaEventRecord(ev[1], h->stream));
   a.take_next_dt = have_dt;
-  if (h->cfg.order == 2) RG_CUDA(h, rg::launch_slopes(a, h->stream));
-  a.take_next_dt = 0;
+  if (h->cfg.order == 2) {
+    RG_CUDA(h, rg::launch_slopes(a, h->stream));
+    a.take_next_dt = 0;
+  }
   if (tr && h->cfg.order == 2) RG_CUDA(h, rg::launch_tr_slopes(a, ta, h->stream));
   if (ev) RG_CUDA(h, cudaEventRecord(ev[2], h->stream));
   RG_CUDA(h, rg::launch_faces(a, h->stream, true));
+  a.take_next_dt = 0;
   if (tr) RG_CUDA(h, rg::launch_tr_faces(a, ta, h->stream, true));
   if (ev) RG_CUDA(h, cudaEventRecord(ev[3], h->stream));
   a.cfl_next = fuse;
@@ -1081,10 +1087,10 @@ rg_status rg_cfl_dt(rg_handle* h, double* dt) {
   h->last = rg_error{};
   RG_TRY(reset_status(h, h->d_status, h->stream));
   if (h->mixed) {
-    RG_CUDA(h, rg::launch_cfl32(mixed_args(h), h->stream, false));
+    RG_CUDA(h, rg::launch_cfl32(mixed_args(h), h->stream));
   } else {
     rg::StepArgs a = step_args(h);
-    RG_CUDA(h, rg::launch_cfl(a, h->stream, false));
+    RG_CUDA(h, rg::launch_cfl(a, h->stream));
   }
   rg_status st = collect(h, h->d_status, h->stream);
   *dt = h->last_dt;
@@ -1105,7 +1111,6 @@ rg_status rg_flux(rg_handle* h, double dt, double* fluxes_out) {
     a64.dt_host = dt;
     const rg::TracerArgs ta = tracer_args(h);
     if (h->cfg.order == 2) {
-      RG_CUDA(h, rg::launch_ghost_fill32(a, h->stream));
       RG_CUDA(h, rg::launch_slopes32(a, h->stream));
       if (tr) RG_CUDA(h, rg::launch_tr_slopes(a64, ta, h->stream));
     }
@@ -1117,7 +1122,6 @@ rg_status rg_flux(rg_handle* h, double dt, double* fluxes_out) {
     const bool tr = h->tcfg.n_tracers > 0;
     const rg::TracerArgs ta = tracer_args(h);
     if (h->cfg.order == 2) {
-      RG_CUDA(h, rg::launch_ghost_fill(a, h->stream));
       RG_CUDA(h, rg::launch_slopes(a, h->stream));
       if (tr) RG_CUDA(h, rg::launch_tr_slopes(a, ta, h->stream));
     }
@@ -1240,14 +1244,23 @@ rg_status rg_run(rg_handle* h, int32_t n_steps, double* dt_out) {
   h->last = rg_error{};
   if (h->step_mode == RG_STEP_PERSISTENT) return run_persistent(h, n_steps, dt_out);
   RG_TRY(reset_status(h, h->d_status, h->stream));
-  if (dt_out) RG_CUDA(h, h->host_dts.ensure(sizeof(double) * static_cast<size_t>(std::max(n_steps, 1))));
+  // each step's dt goes to a device record, copied once at the end (a copy of 8
+  // bytes behind every step cost 7 us of a step's 40 to 88)
+  const size_t dt_bytes = sizeof(double) * static_cast<size_t>(std::max(n_steps, 1));
+  if (dt_out) {
+    RG_CUDA(h, h->host_dts.ensure(dt_bytes));
+    RG_CUDA(h, h->dt_trace.ensure(dt_bytes));
+  }
   double* hd = static_cast<double*>(h->host_dts.p);
   for (int k = 0; k < n_steps; ++k) {
-    if (rg_status st = enqueue_step(h, std::min(k, 0x1fff))) return st;
-    if (dt_out)
-      RG_CUDA(h, cudaMemcpyAsync(hd + k, h->n_problems > 0 ? static_cast<double*>(h->dt_p.p) : &h->d_status->dt,
-                                 sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    h->step_trace = dt_out ? static_cast<double*>(h->dt_trace.p) + k : nullptr;
+    const rg_status st = enqueue_step(h, std::min(k, 0x1fff));
+    h->step_trace = nullptr;
+    if (st != RG_OK) return st;
   }
+  if (dt_out && n_steps > 0)
+    RG_CUDA(h, cudaMemcpyAsync(hd, h->dt_trace.p, sizeof(double) * static_cast<size_t>(n_steps),
+                               cudaMemcpyDeviceToHost, h->stream));
   rg_status st = collect(h, h->d_status, h->stream);
   if (dt_out) std::memcpy(dt_out, hd, sizeof(double) * static_cast<size_t>(n_steps));
   return st;

@@ -7,8 +7,7 @@
 // restates (paths relative to the RICH source root).
 //
 // Passes of one step (hdsim::TimeAdvance, hdsim2d.cpp:149-241, fixed mesh):
-//   k_cfl        per cell: SimpleCFL bound, block min, last block writes dt;
-//                extra threads fill the ghost states
+//   k_cfl        per cell: SimpleCFL bound, block min, last block writes dt
 //   k_slopes     per cell: LinearGaussImproved slope + limiter (order 2)
 //   k_faces_*    per face: reconstruction to the face, HLLC in the face frame,
 //                rotation back, optional dt*area scaling
@@ -17,6 +16,7 @@
 // Geometry-only terms are computed once per mesh upload (k_geom_*).
 #include <math.h>
 
+#include "rg_launch.cuh"
 #include "rg_adjoint.cuh"
 #include "rg_face.cuh"
 #include "rg_fp64.cuh"
@@ -373,14 +373,13 @@ __device__ __forceinline__ unsigned long long cfl_block_bits(const StepArgs& a, 
 
 // simple_cfl.cpp:58-71 + lazy_list.hpp:185-191 (min over the cells, times cfl)
 template <bool kBatch>
-__global__ void __launch_bounds__(kMaxBlock) k_cfl(StepArgs a, int fill_ghosts) {
+__global__ void __launch_bounds__(kMaxBlock) k_cfl(StepArgs a) {
+  chain_wait();
   const MeshDev& m = a.mesh;
-  const int total = fill_ghosts ? m.n + m.g : m.n;
   unsigned long long bits = kInfBits;
   // the trip count is uniform across a block (base is per block)
-  for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
+  for (int base = blockIdx.x * blockDim.x; base < m.n; base += gridDim.x * blockDim.x) {
     const int t = base + threadIdx.x;
-    if (t >= m.n && t < total) fill_ghost(a, t - m.n);
     if (kBatch) {
       // per-problem minimum; the update kernel turns it into the problem's dt
       const unsigned long long xb = t < m.n ? cfl_bound_bits<kBatch>(a, t, load_cell(a.cells, t)) : kInfBits;
@@ -392,12 +391,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_cfl(StepArgs a, int fill_ghosts) 
     }
   }
   if (kBatch) return;
-  grid_min_times(a.status, bits, a.cfl, &a.status->dt);
-}
-
-__global__ void __launch_bounds__(kBlock) k_ghost_fill(StepArgs a) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < a.mesh.g) fill_ghost(a, g);
+  grid_min_times(a.status, bits, a.cfl, &a.status->dt, nullptr, a.dt_trace);
 }
 
 // LinearGaussImproved.cpp:425-494 calc_slope of one component of one cell:
@@ -512,9 +506,8 @@ __device__ __forceinline__ void slopes_lane(const StepArgs& a, int i, int q, uns
 template <bool kBatch, int kMinBlocks = 0, bool kTrace = false>
 __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 1)
     k_slopes(StepArgs a, SlopeTrace* trace) {
-  // the dt of this step, computed by the previous step's update (the face
-  // kernel, launched after this one, reads status->dt)
-  if (a.take_next_dt && blockIdx.x == 0 && threadIdx.x == 0) a.status->dt = a.status->dt_next;
+  chain_wait();
+  take_next_dt(a);
   const int* order = a.geom.cell_order;
   const int q = threadIdx.x & 3;
   const unsigned quad = 0xfu << (threadIdx.x & 28);
@@ -733,6 +726,8 @@ __device__ __forceinline__ void k_faces_item(const StepArgs& a, int e) {
 // (786,430 faces, RoundCells face velocities) 205 -> 141 us, 256^2 66 -> 45 us.
 template <bool kScaled, bool kBatch, bool kLgi>
 __global__ void __launch_bounds__(kMaxBlock, 2) k_faces(StepArgs a) {
+  chain_wait();
+  if (!kLgi) take_next_dt(a);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.mesh.e; e += gridDim.x * blockDim.x)
     k_faces_item<kScaled, kBatch, kLgi>(a, e);
 }
@@ -914,6 +909,8 @@ __device__ __forceinline__ void k_faces_cas_item(const StepArgs& a, int e) {
 
 template <bool kScaled>
 __global__ void __launch_bounds__(kMaxBlock) k_faces_cas(StepArgs a) {
+  chain_wait();
+  if (a.order == 1) take_next_dt(a);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.mesh.e; e += gridDim.x * blockDim.x)
     k_faces_cas_item<kScaled>(a, e);
 }
@@ -1021,6 +1018,7 @@ __device__ __forceinline__ bool update_cell(const StepArgs& a, int i, Cell& c) {
 // warp's FP64 instructions from 128 to about 40.
 template <bool kBatch, int kMode>
 __global__ void __launch_bounds__(kMaxBlock) k_update(StepArgs a) {
+  chain_wait();
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   if (kBatch && kMode <= kUpAverage && !a.batch_keep_dt) {
     for (int p = t0; p < a.n_problems; p += stride) {
@@ -1030,6 +1028,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_update(StepArgs a) {
       a.dt_p[p] = dt;
       a.time_p[p] += dt;
       a.dtmin_p[p] = kInfBits;
+      if (p == 0 && a.dt_trace) *a.dt_trace = dt;
     }
   }
   unsigned long long bits = kInfBits;
@@ -1150,17 +1149,10 @@ cudaError_t launch_geom_ghosts(const GeomArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_cfl(const StepArgs& a, cudaStream_t s, bool fill_ghosts) {
-  const int total = a.mesh.n + (fill_ghosts ? a.mesh.g : 0);
-  if (a.cell_problem)
-    k_cfl<true><<<grid_of(a.shapes.cfl, total), a.shapes.cfl.block, 0, s>>>(a, fill_ghosts ? 1 : 0);
-  else
-    k_cfl<false><<<grid_of(a.shapes.cfl, total), a.shapes.cfl.block, 0, s>>>(a, fill_ghosts ? 1 : 0);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ghost_fill(const StepArgs& a, cudaStream_t s) {
-  if (a.mesh.g > 0) k_ghost_fill<<<blocks(a.mesh.g), kBlock, 0, s>>>(a);
+cudaError_t launch_cfl(const StepArgs& a, cudaStream_t s) {
+  const LaunchShape sh = fit_shape(a.shapes.cfl, a.mesh.n);
+  const int nb = grid_of(sh, a.mesh.n);
+  a.cell_problem ? chain(s, nb, sh.block, k_cfl<true>, a) : chain(s, nb, sh.block, k_cfl<false>, a);
   return cudaGetLastError();
 }
 
@@ -1172,16 +1164,16 @@ cudaError_t launch_slopes(const StepArgs& a, cudaStream_t s) {
     // builds: 0 plain, 2 and 3 register-capped for 3 and 4 resident blocks of
     // up to 256 threads
     switch (sh.variant) {
-      case 2: b ? k_slopes<true, 3><<<nb, bs, 0, s>>>(a, nullptr) : k_slopes<false, 3><<<nb, bs, 0, s>>>(a, nullptr); break;
-      case 3: b ? k_slopes<true, 4><<<nb, bs, 0, s>>>(a, nullptr) : k_slopes<false, 4><<<nb, bs, 0, s>>>(a, nullptr); break;
-      default: b ? k_slopes<true><<<nb, bs, 0, s>>>(a, nullptr) : k_slopes<false><<<nb, bs, 0, s>>>(a, nullptr);
+      case 2: b ? chain(s, nb, bs, k_slopes<true, 3>, a, nullptr) : chain(s, nb, bs, k_slopes<false, 3>, a, nullptr); break;
+      case 3: b ? chain(s, nb, bs, k_slopes<true, 4>, a, nullptr) : chain(s, nb, bs, k_slopes<false, 4>, a, nullptr); break;
+      default: b ? chain(s, nb, bs, k_slopes<true>, a, nullptr) : chain(s, nb, bs, k_slopes<false>, a, nullptr);
     }
   }
   return cudaGetLastError();
 }
 
 cudaError_t launch_slopes_trace(const StepArgs& a, SlopeTrace* trace, cudaStream_t s) {
-  if (a.mesh.n > 0) k_slopes<false, 0, true><<<grid_of(kDefaultShape, 4LL * a.mesh.n), kDefaultShape.block, 0, s>>>(a, trace);
+  if (a.mesh.n > 0) chain(s, grid_of(kDefaultShape, 4LL * a.mesh.n), kDefaultShape.block, k_slopes<false, 0, true>, a, trace);
   return cudaGetLastError();
 }
 
@@ -1191,19 +1183,19 @@ cudaError_t launch_faces(const StepArgs& a, cudaStream_t s, bool scaled) {
   const int nb = grid_of(sh, a.mesh.e), bs = sh.block;
   const bool b = a.cell_problem != nullptr;
   if (a.n_rules > 0) {
-    scaled ? k_faces_cas<true><<<nb, bs, 0, s>>>(a) : k_faces_cas<false><<<nb, bs, 0, s>>>(a);
+    scaled ? chain(s, nb, bs, k_faces_cas<true>, a) : chain(s, nb, bs, k_faces_cas<false>, a);
     return cudaGetLastError();
   }
   if (a.order == 1) {
     if (scaled)
-      b ? k_faces<true, true, false><<<nb, bs, 0, s>>>(a) : k_faces<true, false, false><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_faces<true, true, false>, a) : chain(s, nb, bs, k_faces<true, false, false>, a);
     else
-      b ? k_faces<false, true, false><<<nb, bs, 0, s>>>(a) : k_faces<false, false, false><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_faces<false, true, false>, a) : chain(s, nb, bs, k_faces<false, false, false>, a);
   } else {
     if (scaled)
-      b ? k_faces<true, true, true><<<nb, bs, 0, s>>>(a) : k_faces<true, false, true><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_faces<true, true, true>, a) : chain(s, nb, bs, k_faces<true, false, true>, a);
     else
-      b ? k_faces<false, true, true><<<nb, bs, 0, s>>>(a) : k_faces<false, false, true><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_faces<false, true, true>, a) : chain(s, nb, bs, k_faces<false, false, true>, a);
   }
   return cudaGetLastError();
 }
@@ -1217,15 +1209,15 @@ cudaError_t launch_update(const StepArgs& a, cudaStream_t s, bool from_unscaled,
     if (extensive && cells) {
       // (the fused update reads scaled fluxes)
       if (a.ext_avg)
-        b ? k_update<true, kUpAverage><<<nb, bs, 0, s>>>(a) : k_update<false, kUpAverage><<<nb, bs, 0, s>>>(a);
+        b ? chain(s, nb, bs, k_update<true, kUpAverage>, a) : chain(s, nb, bs, k_update<false, kUpAverage>, a);
       else
-        b ? k_update<true, kUpFused><<<nb, bs, 0, s>>>(a) : k_update<false, kUpFused><<<nb, bs, 0, s>>>(a);
+        b ? chain(s, nb, bs, k_update<true, kUpFused>, a) : chain(s, nb, bs, k_update<false, kUpFused>, a);
     } else if (extensive && from_unscaled) {
-      b ? k_update<true, kUpUnscaled><<<nb, bs, 0, s>>>(a) : k_update<false, kUpUnscaled><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_update<true, kUpUnscaled>, a) : chain(s, nb, bs, k_update<false, kUpUnscaled>, a);
     } else if (extensive) {
-      b ? k_update<true, kUpScaled><<<nb, bs, 0, s>>>(a) : k_update<false, kUpScaled><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_update<true, kUpScaled>, a) : chain(s, nb, bs, k_update<false, kUpScaled>, a);
     } else {
-      b ? k_update<true, kUpCells><<<nb, bs, 0, s>>>(a) : k_update<false, kUpCells><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_update<true, kUpCells>, a) : chain(s, nb, bs, k_update<false, kUpCells>, a);
     }
   }
   return cudaGetLastError();

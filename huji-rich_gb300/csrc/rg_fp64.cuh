@@ -39,7 +39,18 @@ __device__ __forceinline__ double gamma_at(const StepArgs& a, int point) {
 template <bool kBatch>
 __device__ __forceinline__ double scaled_dt(const StepArgs& a, int point) {
   if (kBatch) return a.cfl * __longlong_as_double(static_cast<long long>(a.dtmin_p[a.cell_problem[point]]));
+  if (a.take_next_dt) return a.status->dt_next;  // (the first order's face kernel)
   return a.dt_from_device ? a.status->dt : a.dt_host;
+}
+
+// The step's dt, computed by the previous step's update, into place (one
+// thread): what the kernels after this one read, and the run's record of it
+__device__ __forceinline__ void take_next_dt(const StepArgs& a) {
+  if (a.take_next_dt && blockIdx.x == 0 && threadIdx.x == 0) {
+    const double dt = a.status->dt_next;
+    a.status->dt = dt;
+    if (a.dt_trace) *a.dt_trace = dt;
+  }
 }
 
 // Ghost state (LinearGaussImproved.cpp:543-550 new_cells[ghost]):
@@ -54,10 +65,6 @@ __device__ __forceinline__ Cell ghost_state(const StepArgs& a, int g) {
     c.vy -= u.y * s;
   }
   return c;
-}
-__device__ __forceinline__ void fill_ghost(const StepArgs& a, int g) {
-  const Cell c = ghost_state(a, g);
-  store4(a.cells, a.mesh.n + g, c.d, c.p, c.vx, c.vy);
 }
 // State of point p: a real cell's record, or a ghost's state formed from the
 // current state of its cell (the per-step kernels read no ghost records)

@@ -176,6 +176,8 @@ struct rg_handle {
   // launch (its grid barrier and problem 0's dt per step)
   int step_mode = 0;
   rgh::DevBuf barrier, dt_trace;
+  // where the step being enqueued keeps its dt (rg_run's record), or nullptr
+  double* step_trace = nullptr;
   // CUDA graph of one fused step
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;

@@ -159,9 +159,10 @@ constexpr int kMaxBlockWarps = 16;  // kMaxBlock / 32
 // Grid-wide minimum of non-negative doubles given as bit patterns (one value
 // per thread; every thread of the grid calls this once), then *out =
 // cfl * minimum, written by the last block to finish: SimpleCFL's
-// `cfl * min` (simple_cfl.cpp:58-71).  Leaves the reduction words reset.
+// `cfl * min` (simple_cfl.cpp:58-71), and to *trace where that is set.  Leaves
+// the reduction words reset.
 __device__ inline void grid_min_times(DevStatus* st, unsigned long long bits, double cfl, double* out,
-                                      float* out32 = nullptr) {
+                                      float* out32 = nullptr, double* trace = nullptr) {
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long ob = __shfl_xor_sync(0xffffffffu, bits, o);
     bits = ob < bits ? ob : bits;
@@ -184,6 +185,7 @@ __device__ inline void grid_min_times(DevStatus* st, unsigned long long bits, do
     const unsigned long long mb = atomicAdd(&st->dt_min_bits, 0ull);
     *out = cfl * __longlong_as_double(static_cast<long long>(mb));
     if (out32) *out32 = static_cast<float>(*out);
+    if (trace) *trace = *out;
     st->dt_min_bits = kInfBits;  // ready for the next reduction
     st->blocks_done = 0;
   }
@@ -256,7 +258,9 @@ struct StepArgs {
   int step;             // step number within an rg_run (error ordering)
   int cfl_next;         // the update also computes the next step's SimpleCFL dt (status->dt_next)
   int ev_zero;          // every face velocity is +-0: kernels read none
-  int take_next_dt;     // the slopes kernel first moves status->dt_next to status->dt
+  int take_next_dt;     // the slopes kernel (first order: the face kernel, which then scales by
+                        // dt_next itself) moves status->dt_next to status->dt
+  double* dt_trace;     // where the step's dt is kept (problem 0's of a batch), or nullptr
   int batch_keep_dt;    // batch: the update leaves the per-problem dt, time and minimum
                         // as they are (TimeAdvance2Heun's first half)
   // batch of independent problems (cell_problem == nullptr: one problem)
@@ -404,8 +408,7 @@ cudaError_t launch_problems(const MeshDev& m, const int* offsets, int P, int* ce
 cudaError_t launch_cell_order(const MeshDev& m, int* order, int* cflags, cudaStream_t s);
 cudaError_t launch_geometry(const GeomArgs& a, cudaStream_t s);
 cudaError_t launch_geom_ghosts(const GeomArgs& a, cudaStream_t s);  // the ghost part of launch_geometry
-cudaError_t launch_cfl(const StepArgs& a, cudaStream_t s, bool fill_ghosts);
-cudaError_t launch_ghost_fill(const StepArgs& a, cudaStream_t s);
+cudaError_t launch_cfl(const StepArgs& a, cudaStream_t s);
 cudaError_t launch_slopes(const StepArgs& a, cudaStream_t s);
 // the slopes with the adjoint's limiter trace (periodic meshes, one problem)
 struct SlopeTrace;

@@ -17,6 +17,7 @@
 // gather and the energy conversion), not by the flux arithmetic.
 #include <math.h>
 
+#include "rg_launch.cuh"
 #include "rg_adjoint.cuh"
 #include "rg_convert.cuh"
 #include "rg_div.cuh"
@@ -276,6 +277,7 @@ __global__ void __launch_bounds__(kBlock) k_cells_to32(const double* c64, float4
 }
 
 __global__ void __launch_bounds__(kBlock) k_cells_to64(const float4* c32, double* c64, int n) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 v = c32[i];
@@ -328,7 +330,6 @@ __device__ __forceinline__ float4 ghost_state32(const MixedArgs& a, int q) {
   }
   return c;
 }
-__device__ __forceinline__ void fill_ghost32(const MixedArgs& a, int q) { a.cells32[a.mesh.n + q] = ghost_state32(a, q); }
 // State of point p: a real cell's record, or a ghost's state formed from the
 // current state of its cell (the per-step kernels read no ghost records)
 __device__ __forceinline__ C4 point32(const MixedArgs& a, int p) {
@@ -364,19 +365,28 @@ __device__ __forceinline__ float cfl32_cell(const MixedArgs& a, int t) {
   return 1.0f / res;
 }
 
+// The step's dt, computed by the previous step's update, into place (one
+// thread): what the kernels after this one read, and the run's record of it
+__device__ __forceinline__ void take_next_dt32(const MixedArgs& a) {
+  if (a.take_next_dt && blockIdx.x == 0 && threadIdx.x == 0) {
+    const double dt = a.status->dt_next;
+    a.status->dt = dt;
+    a.status->dt32 = a.status->dt_next32;
+    if (a.dt_trace) *a.dt_trace = dt;
+  }
+}
+
 template <bool kBatch>
-__global__ void __launch_bounds__(kMaxBlock) k_cfl32(MixedArgs a, int fill_ghosts) {
+__global__ void __launch_bounds__(kMaxBlock) k_cfl32(MixedArgs a) {
+  chain_wait();
   const MeshDev& m = a.mesh;
-  const int total = fill_ghosts ? m.n + m.g : m.n;
   unsigned int bits = 0x7f800000u;  // this thread's minimum (+inf; non-negative floats order as integers)
   // warp-uniform trip count (see k_cfl)
-  for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
+  for (int base = blockIdx.x * blockDim.x; base < m.n; base += gridDim.x * blockDim.x) {
     const int t = base + threadIdx.x;
     float x = __int_as_float(0x7f800000);
     if (t < m.n) {
       x = cfl32_cell<kBatch>(a, t);
-    } else if (t < total) {
-      fill_ghost32(a, t - m.n);
     }
     if (kBatch)
       problem_min(a.dtmin_p, t < m.n ? a.cell_problem[t] : -1,
@@ -386,12 +396,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_cfl32(MixedArgs a, int fill_ghost
   }
   if (kBatch) return;
   grid_min_times(a.status, static_cast<unsigned long long>(__double_as_longlong(widen_exact(__uint_as_float(bits)))),
-                 a.cfl, &a.status->dt, &a.status->dt32);
-}
-
-__global__ void __launch_bounds__(kBlock) k_ghost_fill32(MixedArgs a) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < a.mesh.g) fill_ghost32(a, q);
+                 a.cfl, &a.status->dt, &a.status->dt32, a.dt_trace);
 }
 
 // The limiters' candidate of one neighbour, without branches: the candidate
@@ -424,6 +429,7 @@ __device__ __forceinline__ void shocked32(float dphi, float cv, float cellv, flo
 // as std::max / std::min do, and each psi is the smallest candidate taken in
 // edge order, which is what fminf over the candidates gives.
 __global__ void __launch_bounds__(kBlock) k_slopes32_trace(MixedArgs a, double* slopes64, SlopeTrace* trace) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
@@ -720,10 +726,8 @@ __device__ __forceinline__ void k_slopes32_pf_item(const MixedArgs& a, int i) {
 
 template <bool kBatch>
 __global__ void __launch_bounds__(kMaxBlock) k_slopes32_pf(MixedArgs a) {
-  if (a.take_next_dt && blockIdx.x == 0 && threadIdx.x == 0) {
-    a.status->dt = a.status->dt_next;
-    a.status->dt32 = a.status->dt_next32;
-  }
+  chain_wait();
+  take_next_dt32(a);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.mesh.n; i += gridDim.x * blockDim.x)
     k_slopes32_pf_item<kBatch>(a, i);
 }
@@ -731,11 +735,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_slopes32_pf(MixedArgs a) {
 template <bool kBatch, int kMinBlocks, int kUnroll>
 __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 1)
     k_slopes32(MixedArgs a) {
-  // the dt of this step, computed by the previous step's update
-  if (a.take_next_dt && blockIdx.x == 0 && threadIdx.x == 0) {
-    a.status->dt = a.status->dt_next;
-    a.status->dt32 = a.status->dt_next32;
-  }
+  chain_wait();
+  take_next_dt32(a);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.mesh.n; i += gridDim.x * blockDim.x)
     k_slopes32_item<kBatch, kUnroll>(a, i);
 }
@@ -811,7 +812,7 @@ __device__ __forceinline__ void write32(const MixedArgs& a, int e, int real_side
       s = narrow(a.cfl * __longlong_as_double(static_cast<long long>(
                                           a.dtmin_p[a.cell_problem[real_side]]))) * area;
     else
-      s = (a.dt32_from_device ? a.status->dt32 : a.dt32) * area;
+      s = (a.take_next_dt ? a.status->dt_next32 : (a.dt32_from_device ? a.status->dt32 : a.dt32)) * area;
   }
   a.flux32[e] = make_float4(c.m * s, c.en * s, c.mx * s, c.my * s);
   // the unscaled mass flux the tracer faces kernel upwinds with
@@ -863,6 +864,7 @@ __device__ __forceinline__ void k_faces32_lgi_item(const MixedArgs& a, int e) {
 
 template <bool kScaled, bool kBatch>
 __global__ void __launch_bounds__(kMaxBlock) k_faces32_lgi(MixedArgs a) {
+  chain_wait();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.mesh.e; e += gridDim.x * blockDim.x)
     k_faces32_lgi_item<kScaled, kBatch>(a, e);
 }
@@ -874,6 +876,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_faces32_lgi(MixedArgs a) {
 // k_faces32_lgi_item, so the fluxes are bit-identical to the one-thread build.
 template <bool kScaled, bool kBatch>
 __global__ void __launch_bounds__(kMaxBlock) k_faces32_lgi_pair(MixedArgs a) {
+  chain_wait();
   const int s = threadIdx.x & 1;
   const unsigned pair = 3u << (threadIdx.x & 30);
   const int stride = (gridDim.x * blockDim.x) >> 1;
@@ -934,6 +937,8 @@ __device__ __forceinline__ void k_faces32_pcm_item(const MixedArgs& a, int e) {
 
 template <bool kScaled, bool kBatch>
 __global__ void __launch_bounds__(kMaxBlock) k_faces32_pcm(MixedArgs a) {
+  chain_wait();
+  take_next_dt32(a);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.mesh.e; e += gridDim.x * blockDim.x)
     k_faces32_pcm_item<kScaled, kBatch>(a, e);
 }
@@ -1083,6 +1088,7 @@ __device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArg
 template <bool kBatch, int kMode, int kMinBlocks = 0>
 __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 1)
     k_update_mixed(MixedArgs a) {
+  chain_wait();
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   if (kBatch && kMode <= kUpAverage && !a.batch_keep_dt) {
     for (int p = t0; p < a.n_problems; p += stride) {
@@ -1090,6 +1096,7 @@ __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlo
       a.dt_p[p] = dt;
       a.time_p[p] += dt;
       a.dtmin_p[p] = kInfBits;
+      if (p == 0 && a.dt_trace) *a.dt_trace = dt;
     }
   }
   unsigned long long bits = kInfBits;
@@ -1210,7 +1217,7 @@ cudaError_t launch_cells_to32(const double* c64, float4* c32, int n, cudaStream_
   return cudaGetLastError();
 }
 cudaError_t launch_cells_to64(const float4* c32, double* c64, int n, cudaStream_t s) {
-  if (n > 0) k_cells_to64<<<blocks(n), kBlock, 0, s>>>(c32, c64, n);
+  if (n > 0) chain(s, blocks(n), kBlock, k_cells_to64, c32, c64, n);
   return cudaGetLastError();
 }
 cudaError_t launch_vec2_to32(const double* v64, float2* v32, int n, cudaStream_t s) {
@@ -1226,20 +1233,14 @@ cudaError_t launch_flux_to32(const double* f64, float4* f32, int n, cudaStream_t
   return cudaGetLastError();
 }
 
-cudaError_t launch_cfl32(const MixedArgs& a, cudaStream_t s, bool fill_ghosts) {
-  const int total = a.mesh.n + (fill_ghosts ? a.mesh.g : 0);
-  if (a.cell_problem)
-    k_cfl32<true><<<grid_of(a.shapes.cfl, total), a.shapes.cfl.block, 0, s>>>(a, fill_ghosts ? 1 : 0);
-  else
-    k_cfl32<false><<<grid_of(a.shapes.cfl, total), a.shapes.cfl.block, 0, s>>>(a, fill_ghosts ? 1 : 0);
-  return cudaGetLastError();
-}
-cudaError_t launch_ghost_fill32(const MixedArgs& a, cudaStream_t s) {
-  if (a.mesh.g > 0) k_ghost_fill32<<<blocks(a.mesh.g), kBlock, 0, s>>>(a);
+cudaError_t launch_cfl32(const MixedArgs& a, cudaStream_t s) {
+  const LaunchShape sh = fit_shape(a.shapes.cfl, a.mesh.n);
+  const int nb = grid_of(sh, a.mesh.n);
+  a.cell_problem ? chain(s, nb, sh.block, k_cfl32<true>, a) : chain(s, nb, sh.block, k_cfl32<false>, a);
   return cudaGetLastError();
 }
 cudaError_t launch_slopes32_trace(const MixedArgs& a, double* slopes64, SlopeTrace* trace, cudaStream_t s) {
-  if (a.mesh.n > 0) k_slopes32_trace<<<(a.mesh.n + kBlock - 1) / kBlock, kBlock, 0, s>>>(a, slopes64, trace);
+  if (a.mesh.n > 0) chain(s, (a.mesh.n + kBlock - 1) / kBlock, kBlock, k_slopes32_trace, a, slopes64, trace);
   return cudaGetLastError();
 }
 
@@ -1251,11 +1252,11 @@ cudaError_t launch_slopes32(const MixedArgs& a, cudaStream_t s) {
     // builds: 0 plain, 1 neighbour loops unrolled by 2, 2 and 3 register-capped
     // for 5 and 6 resident blocks of up to 256 threads, 4 neighbours prefetched
     switch (sh.variant) {
-      case 4: b ? k_slopes32_pf<true><<<nb, bs, 0, s>>>(a) : k_slopes32_pf<false><<<nb, bs, 0, s>>>(a); break;
-      case 1: b ? k_slopes32<true, 0, 2><<<nb, bs, 0, s>>>(a) : k_slopes32<false, 0, 2><<<nb, bs, 0, s>>>(a); break;
-      case 2: b ? k_slopes32<true, 5, 1><<<nb, bs, 0, s>>>(a) : k_slopes32<false, 5, 1><<<nb, bs, 0, s>>>(a); break;
-      case 3: b ? k_slopes32<true, 6, 1><<<nb, bs, 0, s>>>(a) : k_slopes32<false, 6, 1><<<nb, bs, 0, s>>>(a); break;
-      default: b ? k_slopes32<true, 0, 1><<<nb, bs, 0, s>>>(a) : k_slopes32<false, 0, 1><<<nb, bs, 0, s>>>(a);
+      case 4: b ? chain(s, nb, bs, k_slopes32_pf<true>, a) : chain(s, nb, bs, k_slopes32_pf<false>, a); break;
+      case 1: b ? chain(s, nb, bs, k_slopes32<true, 0, 2>, a) : chain(s, nb, bs, k_slopes32<false, 0, 2>, a); break;
+      case 2: b ? chain(s, nb, bs, k_slopes32<true, 5, 1>, a) : chain(s, nb, bs, k_slopes32<false, 5, 1>, a); break;
+      case 3: b ? chain(s, nb, bs, k_slopes32<true, 6, 1>, a) : chain(s, nb, bs, k_slopes32<false, 6, 1>, a); break;
+      default: b ? chain(s, nb, bs, k_slopes32<true, 0, 1>, a) : chain(s, nb, bs, k_slopes32<false, 0, 1>, a);
     }
   }
   return cudaGetLastError();
@@ -1266,21 +1267,21 @@ cudaError_t launch_faces32(const MixedArgs& a, cudaStream_t s, bool scaled) {
   const bool b = a.cell_problem != nullptr;
   if (a.order == 1) {
     if (scaled)
-      b ? k_faces32_pcm<true, true><<<nb, bs, 0, s>>>(a) : k_faces32_pcm<true, false><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_faces32_pcm<true, true>, a) : chain(s, nb, bs, k_faces32_pcm<true, false>, a);
     else
-      b ? k_faces32_pcm<false, true><<<nb, bs, 0, s>>>(a) : k_faces32_pcm<false, false><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_faces32_pcm<false, true>, a) : chain(s, nb, bs, k_faces32_pcm<false, false>, a);
   } else if (a.shapes.faces.variant == 1) {
     // two threads per face: the one-thread-per-item grid covers 2 e threads
     const int np = grid_of(a.shapes.faces, 2 * a.mesh.e);
     if (scaled)
-      b ? k_faces32_lgi_pair<true, true><<<np, bs, 0, s>>>(a) : k_faces32_lgi_pair<true, false><<<np, bs, 0, s>>>(a);
+      b ? chain(s, np, bs, k_faces32_lgi_pair<true, true>, a) : chain(s, np, bs, k_faces32_lgi_pair<true, false>, a);
     else
-      b ? k_faces32_lgi_pair<false, true><<<np, bs, 0, s>>>(a) : k_faces32_lgi_pair<false, false><<<np, bs, 0, s>>>(a);
+      b ? chain(s, np, bs, k_faces32_lgi_pair<false, true>, a) : chain(s, np, bs, k_faces32_lgi_pair<false, false>, a);
   } else {
     if (scaled)
-      b ? k_faces32_lgi<true, true><<<nb, bs, 0, s>>>(a) : k_faces32_lgi<true, false><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_faces32_lgi<true, true>, a) : chain(s, nb, bs, k_faces32_lgi<true, false>, a);
     else
-      b ? k_faces32_lgi<false, true><<<nb, bs, 0, s>>>(a) : k_faces32_lgi<false, false><<<nb, bs, 0, s>>>(a);
+      b ? chain(s, nb, bs, k_faces32_lgi<false, true>, a) : chain(s, nb, bs, k_faces32_lgi<false, false>, a);
   }
   return cudaGetLastError();
 }
@@ -1289,9 +1290,9 @@ static void update_mixed_build(const MixedArgs& a, const LaunchShape& sh, int nb
   // builds: 0 plain, 2 and 3 register-capped for 5 and 6 resident blocks of up
   // to 256 threads
   switch (sh.variant) {
-    case 2: k_update_mixed<kBatch, kMode, 5><<<nb, sh.block, 0, s>>>(a); break;
-    case 3: k_update_mixed<kBatch, kMode, 6><<<nb, sh.block, 0, s>>>(a); break;
-    default: k_update_mixed<kBatch, kMode><<<nb, sh.block, 0, s>>>(a);
+    case 2: chain(s, nb, sh.block, k_update_mixed<kBatch, kMode, 5>, a); break;
+    case 3: chain(s, nb, sh.block, k_update_mixed<kBatch, kMode, 6>, a); break;
+    default: chain(s, nb, sh.block, k_update_mixed<kBatch, kMode>, a);
   }
 }
 cudaError_t launch_update_mixed(const MixedArgs& a, cudaStream_t s, bool from_unscaled, bool extensive, bool cells) {

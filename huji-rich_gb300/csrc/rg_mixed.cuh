@@ -76,7 +76,9 @@ struct MixedArgs {
   int step;
   int cfl_next;          // the update also computes the next step's dt (status->dt_next)
   int ev_zero;          // every face velocity is +-0: kernels read none
-  int take_next_dt;      // the slopes kernel first moves status->dt_next to status->dt
+  int take_next_dt;      // the slopes kernel (first order: the face kernel, which then scales by
+                         // dt_next32 itself) moves status->dt_next to status->dt
+  double* dt_trace;      // where the step's dt is kept (problem 0's of a batch), or nullptr
   int batch_keep_dt;     // batch: the update leaves the per-problem dt, time and minimum
                          // as they are (TimeAdvance2Heun's first half)
   // batch of independent problems (cell_problem == nullptr: one problem)
@@ -113,12 +115,11 @@ cudaError_t launch_cells_to64(const float4* c32, double* c64, int n, cudaStream_
 cudaError_t launch_vec2_to32(const double* v64, float2* v32, int n, cudaStream_t s);
 cudaError_t launch_flux_to64(const float4* f32, double* f64, int n, cudaStream_t s);
 cudaError_t launch_flux_to32(const double* f64, float4* f32, int n, cudaStream_t s);
-cudaError_t launch_cfl32(const MixedArgs& a, cudaStream_t s, bool fill_ghosts);
+cudaError_t launch_cfl32(const MixedArgs& a, cudaStream_t s);
 // the FP32 slopes with the adjoint's limiter trace, slopes widened to FP64
 // (periodic meshes; rg_adjoint.cuh's SlopeTrace)
 struct SlopeTrace;
 cudaError_t launch_slopes32_trace(const MixedArgs& a, double* slopes64, SlopeTrace* trace, cudaStream_t s);
-cudaError_t launch_ghost_fill32(const MixedArgs& a, cudaStream_t s);
 cudaError_t launch_slopes32(const MixedArgs& a, cudaStream_t s);
 cudaError_t launch_faces32(const MixedArgs& a, cudaStream_t s, bool scaled);
 cudaError_t launch_update_mixed(const MixedArgs& a, cudaStream_t s, bool from_unscaled, bool extensive, bool cells);

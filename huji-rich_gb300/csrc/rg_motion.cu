@@ -18,6 +18,7 @@
 //                       through VoronoiMesh::CalcFaceVelocity (:146-151)
 #include <math.h>
 
+#include "rg_launch.cuh"
 #include "rg_convert.cuh"
 #include "rg_div.cuh"
 #include "rg_motion.cuh"
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(kMoBlock) k_cyl_geometry(MeshDev m, double* xa
 __device__ __forceinline__ double sound(double g, const double* c) { return root(quot(g * c[1], c[0])); }
 
 __global__ void __launch_bounds__(kMoBlock) k_point_velocities(StepArgs a, MotionArgs mo) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
@@ -163,6 +165,7 @@ __global__ void __launch_bounds__(kMoBlock) k_point_velocities(StepArgs a, Motio
 }
 
 __global__ void __launch_bounds__(kMoBlock) k_apply_fix(StepArgs a, MotionArgs mo) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
@@ -221,6 +224,7 @@ __global__ void __launch_bounds__(kMoBlock) k_apply_fix(StepArgs a, MotionArgs m
 }
 
 __global__ void __launch_bounds__(kMoBlock) k_edge_velocities(StepArgs a, MotionArgs mo) {
+  chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (e >= m.e) return;
@@ -250,6 +254,7 @@ __global__ void __launch_bounds__(kMoBlock) k_edge_velocities(StepArgs a, Motion
 // FP64 geometry).  The FP64 face velocities are formed when they are read
 // back (rg_get_edge_velocities).
 __global__ void __launch_bounds__(kMoBlock) k_edge_velocities32(StepArgs a, MotionArgs mo, float2* ev32) {
+  chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (e >= m.e) return;
@@ -294,23 +299,23 @@ cudaError_t launch_cyl_geometry(const MeshDev& m, double* xarea, double* cd_volu
 }
 
 cudaError_t launch_point_velocities(const StepArgs& a, const MotionArgs& mo, cudaStream_t s) {
-  if (a.mesh.n > 0) k_point_velocities<<<mo_blocks(a.mesh.n), kMoBlock, 0, s>>>(a, mo);
+  if (a.mesh.n > 0) chain(s, mo_blocks(a.mesh.n), kMoBlock, k_point_velocities, a, mo);
   return cudaGetLastError();
 }
 
 cudaError_t launch_apply_fix(const StepArgs& a, const MotionArgs& mo, cudaStream_t s) {
   if (a.mesh.n > 0 && mo.kind == RG_MOTION_ROUND_CELLS && (mo.cold || mo.fix))
-    k_apply_fix<<<mo_blocks(a.mesh.n), kMoBlock, 0, s>>>(a, mo);
+    chain(s, mo_blocks(a.mesh.n), kMoBlock, k_apply_fix, a, mo);
   return cudaGetLastError();
 }
 
 cudaError_t launch_edge_velocities(const StepArgs& a, const MotionArgs& mo, cudaStream_t s) {
-  if (a.mesh.e > 0) k_edge_velocities<<<mo_blocks(a.mesh.e), kMoBlock, 0, s>>>(a, mo);
+  if (a.mesh.e > 0) chain(s, mo_blocks(a.mesh.e), kMoBlock, k_edge_velocities, a, mo);
   return cudaGetLastError();
 }
 
 cudaError_t launch_edge_velocities32(const StepArgs& a, const MotionArgs& mo, float2* ev32, cudaStream_t s) {
-  if (a.mesh.e > 0) k_edge_velocities32<<<mo_blocks(a.mesh.e), kMoBlock, 0, s>>>(a, mo, ev32);
+  if (a.mesh.e > 0) chain(s, mo_blocks(a.mesh.e), kMoBlock, k_edge_velocities32, a, mo, ev32);
   return cudaGetLastError();
 }
 

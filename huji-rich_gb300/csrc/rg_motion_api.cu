@@ -180,10 +180,10 @@ rg_status rg_advance_begin(rg_handle* h, double* dt_out, double* pv_out) {
   }
   const bool o2 = h->cfg.order == 2;
   if (h->mixed) {
-    RG_CUDA(h, rg::launch_cfl32(mixed_args(h), h->stream, false));
+    RG_CUDA(h, rg::launch_cfl32(mixed_args(h), h->stream));
   } else {
     rg::StepArgs ac = step_args(h);
-    RG_CUDA(h, rg::launch_cfl(ac, h->stream, false));
+    RG_CUDA(h, rg::launch_cfl(ac, h->stream));
   }
   if (h->motion.kind == RG_MOTION_ROUND_CELLS && (h->motion.cold || h->motion.correct_overshoot)) {
     // ApplyFix with the device dt, face velocities again (the other motions'
@@ -202,7 +202,6 @@ rg_status rg_advance_begin(rg_handle* h, double* dt_out, double* pv_out) {
     a64.dt_from_device = 1;
     const rg::TracerArgs ta = tracer_args(h);
     if (o2) {
-      RG_CUDA(h, rg::launch_ghost_fill32(m, h->stream));
       RG_CUDA(h, rg::launch_slopes32(m, h->stream));
       if (tr) RG_CUDA(h, rg::launch_tr_slopes(a64, ta, h->stream));
     }
@@ -216,7 +215,6 @@ rg_status rg_advance_begin(rg_handle* h, double* dt_out, double* pv_out) {
     const bool tr = h->tcfg.n_tracers > 0;
     const rg::TracerArgs ta = tracer_args(h);
     if (o2) {
-      RG_CUDA(h, rg::launch_ghost_fill(a, h->stream));
       RG_CUDA(h, rg::launch_slopes(a, h->stream));
       if (tr) RG_CUDA(h, rg::launch_tr_slopes(a, ta, h->stream));
     }

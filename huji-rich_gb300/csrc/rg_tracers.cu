@@ -22,6 +22,7 @@
 // registers and no FP64 work is spent on absent tracers.
 #include <math.h>
 
+#include "rg_launch.cuh"
 #include "rg_lgi.cuh"
 
 namespace rg {
@@ -35,6 +36,7 @@ constexpr int kTrBlock = 256;
 // per-tile neighbour-count order.  Tracers share only the geometry and the
 // shock decision, which the hydro pass kept.
 __global__ void __launch_bounds__(kTrBlock) k_tr_slopes(StepArgs a, TracerArgs t) {
+  chain_wait();
   const long long id = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const MeshDev& m = a.mesh;
   const int nt = t.nt;
@@ -93,6 +95,7 @@ __device__ __forceinline__ double tr_scale(const StepArgs& a, int e) {
 // gradient at rigid walls, RigidWallGenerator.cpp:39-54).
 template <bool kScaled>
 __global__ void __launch_bounds__(kTrBlock) k_tr_faces_lgi(StepArgs a, TracerArgs t) {
+  chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (e >= m.e) return;
@@ -123,6 +126,7 @@ __global__ void __launch_bounds__(kTrBlock) k_tr_faces_lgi(StepArgs a, TracerArg
 // k_tr_faces_lgi forms it.  Faces with no action carry none.
 template <bool kScaled>
 __global__ void __launch_bounds__(kTrBlock) k_tr_faces_cas(StepArgs a, TracerArgs t) {
+  chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (e >= m.e) return;
@@ -165,6 +169,7 @@ __global__ void __launch_bounds__(kTrBlock) k_tr_faces_cas(StepArgs a, TracerArg
 // or Mass is 0; a periodic ghost reads its source cell, as the hydro state does.
 template <bool kScaled>
 __global__ void __launch_bounds__(kTrBlock) k_tr_faces_pcm(StepArgs a, TracerArgs t) {
+  chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (e >= m.e) return;
@@ -192,6 +197,7 @@ __global__ void __launch_bounds__(kTrBlock) k_tr_faces_pcm(StepArgs a, TracerArg
 // that is off still take the FP64 unit where the compiler predicates them.
 template <int NT, bool kUnscaled, bool kAverage>
 __global__ void __launch_bounds__(kTrBlock) k_tr_update(StepArgs a, TracerArgs t, int do_ext, int do_cells) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
@@ -276,7 +282,7 @@ inline int tr_blocks(int n) { return (n + kTrBlock - 1) / kTrBlock; }
 
 // k_tr_update for NT = t.nt
 #define RG_TR_CASE(NT, U, A, grid, s, ...) \
-  case NT: k_tr_update<NT, U, A><<<grid, kTrBlock, 0, s>>>(__VA_ARGS__); break;
+  case NT: chain(s, grid, kTrBlock, k_tr_update<NT, U, A>, __VA_ARGS__); break;
 #define RG_TR_DISPATCH(U, A, grid, s, ...)  \
   switch (t.nt) {                           \
     RG_TR_CASE(1, U, A, grid, s, __VA_ARGS__) \
@@ -293,7 +299,7 @@ inline int tr_blocks(int n) { return (n + kTrBlock - 1) / kTrBlock; }
 cudaError_t launch_tr_slopes(const StepArgs& a, const TracerArgs& t, cudaStream_t s) {
   if (a.mesh.n > 0 && t.nt > 0 && t.nt <= kMaxTracers) {
     const long long lanes = static_cast<long long>(a.mesh.n) * t.nt;
-    k_tr_slopes<<<static_cast<unsigned>((lanes + kTrBlock - 1) / kTrBlock), kTrBlock, 0, s>>>(a, t);
+    chain(s, static_cast<unsigned>((lanes + kTrBlock - 1) / kTrBlock), kTrBlock, k_tr_slopes, a, t);
   }
   return cudaGetLastError();
 }
@@ -302,11 +308,11 @@ cudaError_t launch_tr_faces(const StepArgs& a, const TracerArgs& t, cudaStream_t
   if (a.mesh.e == 0 || t.nt == 0) return cudaSuccess;
   const int nb = tr_blocks(a.mesh.e);
   if (a.n_rules > 0)
-    scaled ? k_tr_faces_cas<true><<<nb, kTrBlock, 0, s>>>(a, t) : k_tr_faces_cas<false><<<nb, kTrBlock, 0, s>>>(a, t);
+    scaled ? chain(s, nb, kTrBlock, k_tr_faces_cas<true>, a, t) : chain(s, nb, kTrBlock, k_tr_faces_cas<false>, a, t);
   else if (a.order == 1)
-    scaled ? k_tr_faces_pcm<true><<<nb, kTrBlock, 0, s>>>(a, t) : k_tr_faces_pcm<false><<<nb, kTrBlock, 0, s>>>(a, t);
+    scaled ? chain(s, nb, kTrBlock, k_tr_faces_pcm<true>, a, t) : chain(s, nb, kTrBlock, k_tr_faces_pcm<false>, a, t);
   else
-    scaled ? k_tr_faces_lgi<true><<<nb, kTrBlock, 0, s>>>(a, t) : k_tr_faces_lgi<false><<<nb, kTrBlock, 0, s>>>(a, t);
+    scaled ? chain(s, nb, kTrBlock, k_tr_faces_lgi<true>, a, t) : chain(s, nb, kTrBlock, k_tr_faces_lgi<false>, a, t);
   return cudaGetLastError();
 }
 

@@ -57,7 +57,7 @@ rg_status launch_one(rg_handle* h, int k, const rg::LaunchShape& sh, void* ext_s
     *slot(a.shapes, k) = sh;
     a.dt32_from_device = 1;
     switch (k) {
-      case RG_KERNEL_CFL: RG_CUDA(h, rg::launch_cfl32(a, h->stream, o2)); break;
+      case RG_KERNEL_CFL: RG_CUDA(h, rg::launch_cfl32(a, h->stream)); break;
       case RG_KERNEL_SLOPES: if (o2) RG_CUDA(h, rg::launch_slopes32(a, h->stream)); break;
       case RG_KERNEL_FACES: RG_CUDA(h, rg::launch_faces32(a, h->stream, true)); break;
       default:
@@ -70,7 +70,7 @@ rg_status launch_one(rg_handle* h, int k, const rg::LaunchShape& sh, void* ext_s
     *slot(a.shapes, k) = sh;
     a.dt_from_device = 1;
     switch (k) {
-      case RG_KERNEL_CFL: RG_CUDA(h, rg::launch_cfl(a, h->stream, o2)); break;
+      case RG_KERNEL_CFL: RG_CUDA(h, rg::launch_cfl(a, h->stream)); break;
       case RG_KERNEL_SLOPES: if (o2) RG_CUDA(h, rg::launch_slopes(a, h->stream)); break;
       case RG_KERNEL_FACES: RG_CUDA(h, rg::launch_faces(a, h->stream, true)); break;
       default:
