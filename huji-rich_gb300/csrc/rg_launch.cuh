@@ -4,10 +4,13 @@
 // before it wrote, and the gap between two of them (the drain of one grid, the
 // launch of the next: 2.2 to 2.8 us) was a tenth of a 512^2 FP32-mixed step and
 // half of an 8,000-cell one.  chain() launches with programmatic stream
-// serialization: the next grid's blocks are set up while the last blocks of the
-// one before run, and every such kernel starts with chain_wait(), which returns
-// when the grids before it in the stream have completed and their writes are
-// visible.  Nothing else changes: the kernels still run one after another.
+// serialization: the next grid is set up as the one before ends, and every such
+// kernel starts with chain_wait(), which returns when the grids before it in the
+// stream have completed and their writes are visible.  Nothing else changes: the
+// kernels still run one after another.  No kernel triggers the next one's launch
+// itself: blocks set up earlier go to whichever SMs have room then, and the
+// uneven spread cost more than the last half microsecond saved (FP64 adjoint at
+// 256^2 8.28 against 7.56 ms, Sedov 512^2 FP64 3.89 against 3.69 ms).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -17,11 +20,9 @@ namespace rg {
 
 #ifdef __CUDACC__
 // First statement of every kernel that chain() launches (a no-op in a launch
-// without the attribute): wait for the grids before this one, then let the next
-// one's blocks be set up.
+// without the attribute): wait for the grids before this one.
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <class... P>
