@@ -9,6 +9,7 @@
 // energy, px, py}, I hdsim's init_extensives, C SimpleCellUpdater and G the
 // dt*area-scaled flux gather of one step.
 #pragma once
+#include "rg_div.cuh"
 #include "rg_internal.cuh"
 
 namespace rg {
@@ -35,6 +36,7 @@ struct AdjArgs {
   MeshDev mesh;
   GeomDev geom;
   double gamma, dt, delta_v, theta, delta_p;
+  Divisor gm1;           // gamma - 1 as a divisor
   int slf;
   const double* cells;   // W_k: 4 doubles per point (only real records are read)
   const double* ext;     // U_k: 4*n

@@ -92,6 +92,7 @@ rg::AdjArgs adj_args(rg_handle* h) {
   a.mesh = s->mesh;
   a.geom = s->geom;
   a.gamma = h->cfg.gamma;
+  a.gm1 = rg::divisor(h->cfg.gamma - 1, rg::RcpSeedHost{});
   a.dt = A->dt;
   a.delta_v = h->cfg.delta_v;
   a.theta = h->cfg.theta;

@@ -29,6 +29,7 @@
 #include "rg_launch.cuh"
 #include "rg_adjoint.cuh"
 #include "rg_div.cuh"
+#include "rg_face.cuh"
 
 #ifndef RG_ADJ_REAL
 #define RG_ADJ_REAL double
@@ -39,6 +40,7 @@ namespace rg {
 namespace {
 
 constexpr int kBlock = 256;
+constexpr int kFaceBlock = 128;  // FP64 k_adj_faces
 
 __device__ __forceinline__ void load_raw(const double* c, int i, double o[4]) {
   const double2 a = reinterpret_cast<const double2*>(c)[2 * i];
@@ -129,6 +131,173 @@ __global__ void __launch_bounds__(kBlock) k_adj_seed(AdjArgs a, const double* wb
 
 #endif  // RG_ADJ_FP64
 
+#if RG_ADJ_FP64
+template <class O>
+__device__ __forceinline__ double scaled(O& o, double x, double s) { return o.mul(x, s); }
+#else
+__device__ __forceinline__ double scaled(int&, double x, double s) { return x * s; }
+#endif
+
+#if RG_ADJ_FP64
+// The operations of the reverse in plain arithmetic, for operands outside the
+// integer forms' range (FaceOps clears ok there).
+struct PlainOps {
+  static constexpr bool ok = true;
+  __device__ __forceinline__ double by(double b) { return b; }
+  __device__ __forceinline__ double by(const Divisor&, double b) { return b; }
+  __device__ __forceinline__ double div(double a, double b) { return a / b; }
+  __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
+  __device__ __forceinline__ double mul(double a, double b) { return a * b; }
+  __device__ __forceinline__ double half(double x) { return 0.5 * x; }
+  __device__ __forceinline__ void finite(double, double, double, double) {}
+  static __device__ __forceinline__ double pick(bool first, double a, double b) { return first ? a : b; }
+};
+struct RevOps : FaceOps {
+  using FaceOps::by;
+  __device__ __forceinline__ Divisor by(const Divisor& D, double) {
+    ok = ok && D.ok;
+    return D;
+  }
+  __device__ __forceinline__ double half(double x) { return half_of(x); }
+  __device__ __forceinline__ void finite(double a, double b, double c, double d) {
+    ok = ok && max(max(mag_hi(a), mag_hi(b)), max(mag_hi(c), mag_hi(d))) < 0x7ff00000u;
+  }
+  static __device__ __forceinline__ Divisor pick(bool first, const Divisor& a, const Divisor& b) {
+    return rg::pick(first, a, b);
+  }
+};
+__device__ __forceinline__ bool positive(double x) { return !sign_bit(x) && !is_zero(x); }
+__device__ __forceinline__ bool negative(double x) { return sign_bit(x) && !is_zero(x); }
+// a + b where only few warps need it, not computed ahead of its branch
+__device__ __forceinline__ double add_here(double a, double b) {
+  double r;
+  asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+
+// Reverse of primitive conversion, rotation into the face frame, Hllc
+// (hllc.cpp:97-154, massflux, face at rest) and the rotation back: from fb
+// (adjoint of {mass, energy, px, py}) to the adjoints of the two states.
+//
+// Hllc's flux is written the way it is cheapest to reverse.  With J = d (S_K - u)
+// the mass flux through the outer wave and z the contact speed S*, the flux
+// F_K + S_K (U* - U_K) equals
+//     {m, E' m + p* z, p* + m z, m v_t},   m = d* z,   d* = J/(S_K - z),
+//     p* = p + J A,   E' = |v|^2/2 + e + A B,   A = z - u,   B = z + p/J,
+// and the flux of an undisturbed side is the same with z = u, d* = d, p* = p, A = 0.
+// The reverse of this form takes 80 FP64 additions or multiply-adds where the
+// reverse of the former takes 240 FP64 operations, and is as accurate or
+// better (20,000 random faces against 80-bit arithmetic: mean error 2.4e-16 of
+// the largest adjoint against 4.3e-16, worst 3.1e-15 against 1.6e-14).
+template <class O>
+__device__ __forceinline__ void hllc_reverse(O& o, double g, const Divisor& gm1, rv2 n, double na, rv2 p, double pa,
+                                             const double L[4], const double R[4], const double fb[4], double lb[4],
+                                             double rb[4]) {
+  // forward values
+  const double dL = L[0], pL = L[1], dR = R[0], pR = R[1];
+  const auto qdL = o.by(dL), qdR = o.by(dR), qna = o.by(na), qpa = o.by(pa), qgm1 = o.by(gm1, g - 1.0);
+  const double cL = o.sqrt(o.div(o.mul(g, pL), qdL)), cR = o.sqrt(o.div(o.mul(g, pR), qdR));
+  const double lu = o.div(o.mul(L[2], n.x) + L[3] * n.y, qna), ru = o.div(o.mul(R[2], n.x) + R[3] * n.y, qna);
+  const double a1 = lu - cL, b1 = ru - cR, a2 = lu + cL, b2 = ru + cR;
+  const bool sl_right = less_finite(b1, a1), sr_right = less_finite(a2, b2);
+  const double sl = sl_right ? b1 : a1, sr = sr_right ? b2 : a2;
+  o.finite(a1, b1, a2, b2);  // the tests on signs and bit patterns are for finite speeds
+  const double tl = sl - lu, tr = sr - ru;
+  const double JL = o.mul(dL, tl), JR = o.mul(dR, tr);
+  const auto qden = o.by(JL - JR);
+  const double ss = o.div((pR - pL) + JL * lu - JR * ru, qden);
+  const bool left = positive(sl) || !negative(ss);
+  const bool star = left ? !positive(sl) : !negative(sr);
+  // the upwind side
+  const double qd = left ? dL : dR, qp = left ? pL : pR, qu = left ? lu : ru, sk = left ? sl : sr;
+  const double K = left ? tl : tr, J = left ? JL : JR;
+  const auto by_d = O::pick(left, qdL, qdR);
+  const double qv = o.div(o.mul(left ? L[2] : R[2], p.x) + (left ? L[3] : R[3]) * p.y, qpa);
+  const double e = o.div(o.div(qp, by_d), qgm1);
+  double E = 0.5 * (qu * qu + o.mul(qv, qv)) + e;
+  // adjoint of the face-frame flux {fm, fmx, fmy, fen}
+  const double bfm = fb[0], bfen = fb[1];
+  const double bfmx = o.div(n.x * fb[2] + o.mul(n.y, fb[3]), qna);
+  const double bfmy = o.div(p.x * fb[2] + o.mul(p.y, fb[3]), qpa);
+  double bd, bp, bu, bv;
+  if (!star) {
+    const double m = o.mul(qd, qu), w = o.mul(m, bfen);
+    const double G = bfm + bfmx * qu + bfmy * qv + bfen * E;
+    bv = o.mul(m, bfmy + bfen * qv);
+    const double y = o.div(w, by_d);
+    bd = o.mul(qu, G) - y * e;
+    bu = qd * G + m * bfmx + bfen * qp + w * qu;
+    bp = bfmx + bfen * qu + o.div(y, qgm1);
+    const double xu = o.div(bu, qna), xv = o.div(bv, qpa);
+    const double x = xu * n.x + o.mul(xv, p.x), yy = xu * n.y + o.mul(xv, p.y);
+    lb[0] = left ? bd : 0.0, lb[1] = left ? bp : 0.0, lb[2] = left ? x : 0.0, lb[3] = left ? yy : 0.0;
+    rb[0] = left ? 0.0 : bd, rb[1] = left ? 0.0 : bp, rb[2] = left ? 0.0 : x, rb[3] = left ? 0.0 : yy;
+    return;
+  }
+  double bss, bsk;
+  {
+    const auto qD = o.by(sk - ss), qJ = o.by(J);
+    const double ds = o.div(J, qD), A = ss - qu, Q = o.div(qp, qJ), B = ss + Q;
+    E += A * B;
+    const double ps = qp + J * A, m = o.mul(ds, ss), w = o.mul(m, bfen);
+    const double H = bfmx + bfen * ss, G = bfm + bfmx * ss + bfmy * qv + bfen * E;
+    bv = o.mul(m, bfmy + bfen * qv);
+    const double X = o.div(o.mul(ss, G), qD), wA = o.mul(w, A), Y = o.div(wA, qJ);
+    const double S = X + H * A - Y * Q;
+    const double y = o.div(w, by_d);
+    bp = H + Y + o.div(y, qgm1);
+    bd = o.mul(K, S) - y * e;
+    const double qS = o.mul(qd, S), bA = o.mul(H, J) + w * B;
+    bss = ds * G + m * bfmx + bfen * ps + bA + wA + ds * X;
+    bu = w * qu - bA - qS;
+    bsk = qS - ds * X;
+  }
+  // the wave speeds: ss = num/den, sl = min(lu - cL, ru - cR), sr = max(lu + cL, ru + cR)
+  const double bnum = o.div(bss, qden);
+  const double aL = o.mul(bnum, lu - ss), aR = o.mul(bnum, ru - ss);
+  double bdL = tl * aL + (left ? bd : 0.0), bdR = (left ? 0.0 : bd) - tr * aR;
+  double buL = dL * (bnum * tl - aL) + (left ? bu : 0.0), buR = (left ? 0.0 : bu) - dR * (bnum * tr - aR);
+  double bpL = (left ? bp : 0.0) - bnum, bpR = (left ? 0.0 : bp) + bnum;
+  const double bsl = aL * dL + (left ? bsk : 0.0), bsr = (left ? 0.0 : bsk) - aR * dR;
+  double bcL, bcR;
+  if (!sl_right && sr_right) {
+    buL += bsl;
+    buR += bsr;
+    bcL = -bsl;
+    bcR = bsr;
+  } else if (sl_right && sr_right) {  // both waves from the right side, or the left, or crossed
+    buR = add_here(add_here(buR, bsl), bsr);
+    bcL = 0.0;
+    bcR = add_here(bsr, -bsl);
+  } else if (!sl_right) {
+    buL = add_here(add_here(buL, bsl), bsr);
+    bcL = add_here(bsr, -bsl);
+    bcR = 0.0;
+  } else {
+    buR = add_here(buR, bsl);
+    buL = add_here(buL, bsr);
+    bcL = bsr;
+    bcR = -bsl;
+  }
+  // c = sqrt(gamma p/d)
+  const double hL = o.half(o.div(bcL, qdL)), hR = o.half(o.div(bcR, qdR));
+  bdL -= hL * cL;
+  bdR -= hR * cR;
+  bpL += o.div(o.mul(hL, g), o.by(cL));
+  bpR += o.div(o.mul(hR, g), o.by(cR));
+  // rotation into the face frame: u = v.n/|n|, v_t = v.par/|par|
+  const double xL = o.div(buL, qna), xR = o.div(buR, qna), xv = o.div(bv, qpa);
+  const double vx = o.mul(xv, p.x), vy = o.mul(xv, p.y);
+  lb[0] = bdL;
+  lb[1] = bpL;
+  lb[2] = xL * n.x + (left ? vx : 0.0);
+  lb[3] = xL * n.y + (left ? vy : 0.0);
+  rb[0] = bdR;
+  rb[1] = bpR;
+  rb[2] = xR * n.x + (left ? 0.0 : vx);
+  rb[3] = xR * n.y + (left ? 0.0 : vy);
+}
+#else
 // Reverse of primitive conversion, rotation into the face frame, Hllc
 // (hllc.cpp:97-154, massflux, face at rest) and the rotation back: from fb
 // (adjoint of {mass, energy, px, py}) to the adjoints of the two states.
@@ -251,6 +420,8 @@ __device__ void hllc_reverse(real g, rv2 n, real na, rv2 p, real pa, const real 
   rb[3] = quot(buR * n.y, na) + quot(bvR * p.y, pa);
 }
 
+#endif  // RG_ADJ_FP64
+
 __device__ __forceinline__ void face_state(const AdjArgs& a, int pid, rv2 dm, real c[4]) {
   const int sid = source_of(a.mesh, pid);
   real gx[4], gy[4];
@@ -261,21 +432,15 @@ __device__ __forceinline__ void face_state(const AdjArgs& a, int pid, rv2 dm, re
   for (int q = 0; q < 4; ++q) c[q] = c[q] + gx[q] * dm.x + gy[q] * dm.y;
 }
 
-__global__ void __launch_bounds__(kBlock) k_adj_faces(AdjArgs a, const double* ubar) {
-  chain_wait();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+// One face; false (nothing stored) where its operands are outside O's range.
+template <class O>
+__device__ __forceinline__ bool face_reverse(O& o, const AdjArgs& a, const double* ubar, int e) {
   const MeshDev& m = a.mesh;
-  if (e >= m.e) return;
   const int2 fc = m.face_cells[e];
   // the transposed gather of the extensive update stays in FP64
   const double s = a.dt * a.geom.area[e];
   double fbd[4] = {0, 0, 0, 0};
-  if (fc.y < m.n) {
-    double u[4];
-    load_raw(ubar, fc.y, u);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) fbd[q] += u[q];
-  }
+  if (fc.y < m.n) load_raw(ubar, fc.y, fbd);
   if (fc.x < m.n) {
     double u[4];
     load_raw(ubar, fc.x, u);
@@ -284,15 +449,49 @@ __global__ void __launch_bounds__(kBlock) k_adj_faces(AdjArgs a, const double* u
   }
   real fb[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) fb[q] = to_real(fbd[q] * s);
+  for (int q = 0; q < 4; ++q) fb[q] = to_real(scaled(o, fbd[q], s));
   real L[4], R[4], lb[4], rb[4];
   face_state(a, fc.x, r2(a.geom.dm0[e]), L);
   face_state(a, fc.y, r2(a.geom.dm1[e]), R);
+#if RG_ADJ_FP64
+  hllc_reverse(o, a.gamma, a.gm1, r2(a.geom.nrm[e]), a.geom.nabs[e], r2(a.geom.par[e]), a.geom.area[e], L, R, fb, lb,
+               rb);
+  if (!o.ok) return false;
+#else
   hllc_reverse(to_real(a.gamma), r2(a.geom.nrm[e]), to_real(a.geom.nabs[e]), r2(a.geom.par[e]),
                to_real(a.geom.area[e]), L, R, fb, lb, rb);
+#endif
   store_r(a.side_bar, 2 * e, lb);
   store_r(a.side_bar, 2 * e + 1, rb);
+  return true;
 }
+
+#if RG_ADJ_FP64
+static __device__ __noinline__ void face_reverse_plain(const AdjArgs& a, const double* ubar, int e) {
+  PlainOps o;
+  face_reverse(o, a, ubar, e);
+}
+// One thread per face.  Bound by the FP64 unit (80 operations a warp) with the
+// products and quotients on the integer pipes beside it.  Six blocks of 128 per
+// SM (80 registers, 400 bytes spilt) hold most of a 256^2 mesh's faces at once:
+// 48 us, against 51 with five, 50 with four and 52-58 in blocks of 256 and 512.
+// 256^2 (132,000 faces) 123 -> 48 us.
+__global__ void __launch_bounds__(kFaceBlock, 6) k_adj_faces(AdjArgs a, const double* ubar) {
+  chain_wait();
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= a.mesh.e) return;
+  RevOps o;
+  if (!face_reverse(o, a, ubar, e)) face_reverse_plain(a, ubar, e);
+}
+#else
+__global__ void __launch_bounds__(kBlock) k_adj_faces(AdjArgs a, const double* ubar) {
+  chain_wait();
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= a.mesh.e) return;
+  int none = 0;
+  face_reverse(none, a, ubar, e);
+}
+#endif
 
 __global__ void __launch_bounds__(kBlock) k_adj_cell(AdjArgs a) {
   chain_wait();
@@ -439,7 +638,7 @@ cudaError_t adj_launch_update(const AdjArgs& a, const double* ubar_in, double* u
 
 cudaError_t adj_launch_reverse(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
                                cudaStream_t s) {
-  chain(s, blocks(a.mesh.e), kBlock, k_adj_faces, a, ubar_in);
+  chain(s, (a.mesh.e + kFaceBlock - 1) / kFaceBlock, kFaceBlock, k_adj_faces, a, ubar_in);
   chain(s, blocks(a.mesh.n), kBlock, k_adj_cell, a);
   return adj_launch_update(a, ubar_in, ubar_out, grad, s);
 }
