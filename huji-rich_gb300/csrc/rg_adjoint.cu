@@ -53,6 +53,12 @@ __device__ __forceinline__ T constant(double x);
 template <>
 __device__ __forceinline__ Dual constant<Dual>(double x) { return Dual{x, 0.0}; }
 
+// the recorded step's FP64 records
+__host__ __device__ __forceinline__ const double* cells64(const AdjArgs& a) {
+  return static_cast<const double*>(a.cells);
+}
+__host__ __device__ __forceinline__ double* slopes64(const AdjArgs& a) { return static_cast<double*>(a.slopes); }
+
 // {density, pressure, vx, vy}
 template <class T>
 struct V4 {
@@ -98,14 +104,14 @@ __device__ __forceinline__ int entry_source(const AdjArgs& a, int k) {
 template <class T>
 __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
   const MeshDev& m = a.mesh;
-  const V4<T> cell = load4<T>(a.cells, a.dcells, i);
+  const V4<T> cell = load4<T>(cells64(a), a.dcells, i);
   const int b = m.cell_off[i], nn = m.cell_off[i + 1] - b;
   const dbl4 mi = a.geom.minv[i];
   V4<T> vx, vy;
 #pragma unroll
   for (int q = 0; q < 4; ++q) vx.v[q] = vy.v[q] = constant<T>(0.0);
   for (int k = 0; k < nn; ++k) {
-    const V4<T> nb = load4<T>(a.cells, a.dcells, entry_source(a, b + k));
+    const V4<T> nb = load4<T>(cells64(a), a.dcells, entry_source(a, b + k));
     const double2 h = a.geom.hr[b + k];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -137,7 +143,7 @@ __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
     bool shock = lhs < (-a.delta_v) * root(quot(a.gamma * cq_[1], cq_[0]));
     if (!shock && nn == 0) shock = 1.0 < a.delta_p;
     for (int k = 0; k < nn && !shock; ++k) {
-      const double np_ = a.cells[4 * entry_source(a, b + k) + 1];
+      const double np_ = cells64(a)[4 * entry_source(a, b + k) + 1];
       const double num = cq_[1] > np_ ? np_ : cq_[1];
       const double den = cq_[1] > np_ ? cq_[1] : np_;
       shock = quot(num, den) < a.delta_p;
@@ -149,7 +155,7 @@ __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
     for (int q = 0; q < 4; ++q) cmax[q] = cmin[q] = cq_[q];
     for (int k = 0; k < nn; ++k) {
       double nv[4];
-      load_raw(a.cells, entry_source(a, b + k), nv);
+      load_raw(cells64(a), entry_source(a, b + k), nv);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         if (cmax[q] < nv[q]) {
@@ -170,8 +176,8 @@ __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
       const double thr = f * smax(fabs(maxd), fabs(mind));
       // the numerators as functions of the state: neighbour (or cell) minus cell
       T nmax = constant<T>(0.0), nmin = constant<T>(0.0);
-      if (amax[q] >= 0) nmax = load4<T>(a.cells, a.dcells, entry_source(a, b + amax[q])).v[q] - cell.v[q];
-      if (amin[q] >= 0) nmin = load4<T>(a.cells, a.dcells, entry_source(a, b + amin[q])).v[q] - cell.v[q];
+      if (amax[q] >= 0) nmax = load4<T>(cells64(a), a.dcells, entry_source(a, b + amax[q])).v[q] - cell.v[q];
+      if (amin[q] >= 0) nmin = load4<T>(cells64(a), a.dcells, entry_source(a, b + amin[q])).v[q] - cell.v[q];
       for (int k = 0; k < nn; ++k) {
         const int e = m.cell_faces[b + k];
         const double2 dm = (a.geom.nbr[b + k] & kNbrFirst) ? a.geom.dm0[e] : a.geom.dm1[e];
@@ -190,7 +196,7 @@ __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
             if (val(cand) < val(psi[q])) psi[q] = cand;
           }
         } else if (fabs(dv) > 1e-9 * cq) {
-          const T nb = load4<T>(a.cells, a.dcells, entry_source(a, b + k)).v[q];
+          const T nb = load4<T>(cells64(a), a.dcells, entry_source(a, b + k)).v[q];
           const T cand = quot(a.theta * (nb - cell.v[q]), dphi);
           const bool clamp = val(cand) < 0.0;  // std::max(cand, 0)
           const T x = clamp ? constant<T>(0.0) : cand;
@@ -208,8 +214,8 @@ __device__ void lgi_slope(const AdjArgs& a, int i, V4<T>& sx, V4<T>& sy) {
 
 template <class T>
 __device__ __forceinline__ void store_slope(const AdjArgs& a, int i, const V4<T>& sx, const V4<T>& sy) {
-  store_raw(a.slopes, 2 * i, val(sx.v[0]), val(sx.v[1]), val(sx.v[2]), val(sx.v[3]));
-  store_raw(a.slopes, 2 * i + 1, val(sy.v[0]), val(sy.v[1]), val(sy.v[2]), val(sy.v[3]));
+  store_raw(slopes64(a), 2 * i, val(sx.v[0]), val(sx.v[1]), val(sx.v[2]), val(sx.v[3]));
+  store_raw(slopes64(a), 2 * i + 1, val(sy.v[0]), val(sy.v[1]), val(sy.v[2]), val(sy.v[3]));
   if (a.dslopes) {
     store_raw(a.dslopes, 2 * i, tan_of(sx.v[0]), tan_of(sx.v[1]), tan_of(sx.v[2]), tan_of(sx.v[3]));
     store_raw(a.dslopes, 2 * i + 1, tan_of(sy.v[0]), tan_of(sy.v[1]), tan_of(sy.v[2]), tan_of(sy.v[3]));
@@ -285,8 +291,8 @@ __device__ bool face_flux(const AdjArgs& a, int e, const V4<T>& L, const V4<T>& 
 // times (face centroid - centre of mass of the side's point)
 __device__ __forceinline__ V4<Dual> face_state(const AdjArgs& a, int pid, double2 dm) {
   const int sid = source_of(a.mesh, pid);
-  V4<Dual> c = load4<Dual>(a.cells, a.dcells, sid);
-  const V4<Dual> gx = load4<Dual>(a.slopes, a.dslopes, 2 * sid), gy = load4<Dual>(a.slopes, a.dslopes, 2 * sid + 1);
+  V4<Dual> c = load4<Dual>(cells64(a), a.dcells, sid);
+  const V4<Dual> gx = load4<Dual>(slopes64(a), a.dslopes, 2 * sid), gy = load4<Dual>(slopes64(a), a.dslopes, 2 * sid + 1);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     c.v[q] = c.v[q] + gx.v[q] * dm.x;
@@ -365,7 +371,7 @@ __global__ void __launch_bounds__(kBlock) k_tl_init(AdjArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.mesh.n) return;
   double c[4], t[4];
-  load_raw(a.cells, i, c);
+  load_raw(cells64(a), i, c);
   load_raw(a.dcells, i, t);
   const double V = a.mesh.cd_volume[i];
   const double mass = V * c[0];
@@ -392,10 +398,10 @@ cudaError_t adj_launch_record_slopes(const AdjArgs& a, cudaStream_t s) {
   t.delta_v = a.delta_v;
   t.theta = a.theta;
   t.delta_p = a.delta_p;
-  t.cells = const_cast<double*>(a.cells);
-  t.slopes = a.slopes;
+  t.cells = const_cast<double*>(cells64(a));
+  t.slopes = slopes64(a);
   t.status = a.status;
-  return launch_slopes_trace(t, a.trace, s);
+  return launch_slopes_trace(t, static_cast<SlopeTrace*>(a.trace), s);
 }
 
 cudaError_t tl_launch_init(const AdjArgs& a, cudaStream_t s) {

@@ -11,6 +11,7 @@
 #pragma once
 #include "rg_div.cuh"
 #include "rg_internal.cuh"
+#include "rg_mixed.cuh"
 
 namespace rg {
 
@@ -24,10 +25,12 @@ namespace rg {
 //                         and clamped to 0), bits 16-23 the entry whose
 //                         neighbour gave the numerator, plus one (0: the
 //                         numerator is identically zero)
-struct __align__(16) SlopeTrace {
-  double naive[8];
-  double psi[4];
-  double dphi[4];
+// SlopeTrace32: the same of the FP32 slopes.
+template <class R>
+struct __align__(16) SlopeTraceOf {
+  R naive[8];
+  R psi[4];
+  R dphi[4];
   int code[4];
 };
 constexpr int kTraceNone = 0xff;
@@ -38,10 +41,13 @@ struct AdjArgs {
   double gamma, dt, delta_v, theta, delta_p;
   Divisor gm1;           // gamma - 1 as a divisor
   int slf;
-  const double* cells;   // W_k: 4 doubles per point (only real records are read)
+  MixedGeom g32;         // FP32-mixed reverse: the geometry as its step uses it
+  // the recorded step and the reverse's work arrays below: records of doubles
+  // (SlopeTrace) or, for the FP32-mixed reverse, of floats (SlopeTrace32)
+  const void* cells;     // W_k: 4 per point (only real records are read)
   const double* ext;     // U_k: 4*n
-  double* slopes;        // 8*n (forward: written; reverse: read)
-  SlopeTrace* trace;     // n
+  void* slopes;          // 8*n (forward: written; reverse: read)
+  void* trace;           // n
   DevStatus* status;
   // tangent-linear forward: tangents beside the values
   const double* dcells;  // 4*n
@@ -53,9 +59,9 @@ struct AdjArgs {
   double* cells_out;     // 4*n
   double* dcells_out;    // 4*n
   // reverse sweep work arrays
-  double* side_bar;      // 8*e: adjoint of each face's two reconstructed states
-  double* self_bar;      // 4*n: a cell's own share of its state adjoint
-  double* entry_bar;     // 4*m: per CSR entry, the share of that neighbour's source
+  void* side_bar;        // 8*e: adjoint of each face's two reconstructed states
+  void* self_bar;        // 4*n: a cell's own share of its state adjoint
+  void* entry_bar;       // 4*m: per CSR entry, the share of that neighbour's source
   // reverse adjacency (ascending, built once per mesh)
   const int* side_off;   // n+1
   const int* sides;      // 2*e: side s = 2*face + (0 first, 1 second) whose source is the cell
@@ -75,9 +81,6 @@ cudaError_t adj_launch_seed(const AdjArgs& a, const double* wbar, double* ubar, 
 // for the first step (grad != nullptr), to the gradient with respect to W_0.
 cudaError_t adj_launch_reverse(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
                                cudaStream_t s);
-// the transposed cell update and gather alone (shared by both precisions)
-cudaError_t adj_launch_update(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
-                              cudaStream_t s);
 // rg_adjoint_rev32.cu: the same reverse step with the face and cell kernels in FP32
 cudaError_t adj_launch_reverse32(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
                                  cudaStream_t s);

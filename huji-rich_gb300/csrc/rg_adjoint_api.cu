@@ -46,12 +46,10 @@ struct rg_adjoint_state {
   // reverse sweep and tangent work arrays
   DevBuf ubar0, ubar1, side_bar, self_bar, entry_bar, io;
   DevBuf dcells, dslopes, dflux, dext;
-  // FP32-mixed recomputation: the interval's running FP32 primitives and extensives
-  DevBuf w_cells32;
   void release() {
     for (DevBuf* b : {&side_off, &sides, &target_off, &targets, &ckpt_cells, &ckpt_ext, &final_ext, &seg_cells,
                       &seg_ext, &seg_slopes, &seg_trace, &ubar0, &ubar1, &side_bar, &self_bar, &entry_bar, &io,
-                      &dcells, &dslopes, &dflux, &dext, &w_cells32})
+                      &dcells, &dslopes, &dflux, &dext})
       b->release();
     adjacency = have_forward = false;
   }
@@ -99,9 +97,10 @@ rg::AdjArgs adj_args(rg_handle* h) {
   a.delta_p = h->cfg.delta_p;
   a.slf = h->cfg.slope_limiter;
   a.status = h->d_status;
-  a.side_bar = ptr<double>(A->side_bar);
-  a.self_bar = ptr<double>(A->self_bar);
-  a.entry_bar = ptr<double>(A->entry_bar);
+  a.g32 = s->g32;
+  a.side_bar = A->side_bar.p;
+  a.self_bar = A->self_bar.p;
+  a.entry_bar = A->entry_bar.p;
   a.side_off = ptr<int>(A->side_off);
   a.sides = ptr<int>(A->sides);
   a.target_off = ptr<int>(A->target_off);
@@ -162,9 +161,10 @@ rg_status ensure_adjacency(rg_handle* h) {
   RG_CUDA(h, A->ubar0.ensure(32 * static_cast<size_t>(n)));
   RG_CUDA(h, A->ubar1.ensure(32 * static_cast<size_t>(n)));
   RG_CUDA(h, A->io.ensure(32 * static_cast<size_t>(n)));
-  RG_CUDA(h, A->side_bar.ensure(64 * ne));
-  RG_CUDA(h, A->self_bar.ensure(32 * static_cast<size_t>(n)));
-  RG_CUDA(h, A->entry_bar.ensure(32 * nm));
+  const size_t rec = h->mixed ? 16 : 32;
+  RG_CUDA(h, A->side_bar.ensure(2 * rec * ne));
+  RG_CUDA(h, A->self_bar.ensure(rec * static_cast<size_t>(n)));
+  RG_CUDA(h, A->entry_bar.ensure(rec * nm));
   RG_CUDA(h, A->final_ext.ensure(32 * static_cast<size_t>(n)));
   // the mesh must be one the adjoint covers
   RG_TRY(reset_status(h, h->d_status, h->stream));
@@ -234,10 +234,11 @@ rg_status rg_step_fwd(rg_handle* h, int32_t n_steps, double dt, int32_t every) {
   RG_CUDA(h, A->ckpt_cells.ensure(32 * n * static_cast<size_t>(n_ckpt)));
   RG_CUDA(h, A->ckpt_ext.ensure(32 * n * static_cast<size_t>(n_ckpt)));
   const size_t seg = static_cast<size_t>(std::min(every, n_steps));
-  RG_CUDA(h, A->seg_cells.ensure(32 * np * seg));
+  // (FP32 records where the steps are FP32-mixed)
+  RG_CUDA(h, A->seg_cells.ensure((h->mixed ? 16 : 32) * np * seg));
   RG_CUDA(h, A->seg_ext.ensure(32 * n * seg));
-  RG_CUDA(h, A->seg_slopes.ensure(64 * n * seg));
-  RG_CUDA(h, A->seg_trace.ensure(sizeof(rg::SlopeTrace) * n * seg));
+  RG_CUDA(h, A->seg_slopes.ensure((h->mixed ? 32 : 64) * n * seg));
+  RG_CUDA(h, A->seg_trace.ensure((h->mixed ? sizeof(rg::SlopeTrace32) : sizeof(rg::SlopeTrace)) * n * seg));
   RG_TRY(reset_status(h, h->d_status, h->stream));
   rg::StepArgs a = step_args(h);
   a.dt_host = dt;
@@ -305,43 +306,38 @@ rg_status rg_step_bwd(rg_handle* h, const double* cells_bar, double* cells0_bar)
   RG_CUDA(h, rg::adj_launch_seed(base, ptr<double>(A->io), cur, h->stream));
   rg::StepArgs a = step_args(h);
   a.dt_host = A->dt;
-  if (h->mixed) {
-    RG_CUDA(h, A->w_cells32.ensure(16 * np));
-  }
   for (int c = A->n_ckpt - 1; c >= 0 && h->mixed; --c) {
     // FP32-mixed: recompute the interval with the mixed kernels, recording
     // each step's state (widened), extensives, FP32 slopes and their trace
     const int start = c * A->every;
     const int len = std::min(A->every, A->n_steps - start);
-    RG_CUDA(h, cudaMemcpyAsync(A->w_cells32.p, ptr<double>(A->ckpt_cells, 4 * n * static_cast<size_t>(c)), 16 * n,
+    RG_CUDA(h, cudaMemcpyAsync(A->seg_cells.p, ptr<double>(A->ckpt_cells, 4 * n * static_cast<size_t>(c)), 16 * n,
                                cudaMemcpyDeviceToDevice, h->stream));
     RG_CUDA(h, cudaMemcpyAsync(A->seg_ext.p, ptr<double>(A->ckpt_ext, 4 * n * static_cast<size_t>(c)), 32 * n,
                                cudaMemcpyDeviceToDevice, h->stream));
     rg::MixedArgs mx = mixed_fixed_dt(h, A->dt);
-    mx.cells32 = static_cast<float4*>(A->w_cells32.p);
     for (int j = 0; j < len; ++j) {
       const size_t J = static_cast<size_t>(j);
-      // each step's update writes its extensives into the next step's record
+      // each step's update writes into the next step's record
+      mx.cells32 = ptr<float4>(A->seg_cells, np * J);
+      mx.cells32_out = ptr<float4>(A->seg_cells, np * (J + 1));
+      mx.slopes32 = ptr<float4>(A->seg_slopes, 2 * n * J);
       mx.ext = ptr<double>(A->seg_ext, 4 * n * J);
       mx.ext_out = ptr<double>(A->seg_ext, 4 * n * (J + 1));
-      RG_CUDA(h, rg::launch_cells_to64(mx.cells32, ptr<double>(A->seg_cells, 4 * np * J), s->n, h->stream));
-      RG_CUDA(h, rg::launch_slopes32_trace(mx, ptr<double>(A->seg_slopes, 8 * n * J),
-                                           ptr<rg::SlopeTrace>(A->seg_trace, n * J), h->stream));
+      mx.step = std::min(start + j, 0x1fff);
+      RG_CUDA(h, rg::launch_slopes32_trace(mx, ptr<rg::SlopeTrace32>(A->seg_trace, n * J), h->stream));
       if (j + 1 < len) {
-        // the rest of the step: the trace kernel has left the FP32 slopes
-        rg::MixedArgs mj = mx;
-        mj.step = std::min(start + j, 0x1fff);
-        RG_CUDA(h, rg::launch_faces32(mj, h->stream, true));
-        RG_CUDA(h, rg::launch_update_mixed(mj, h->stream, false, true, true));
+        RG_CUDA(h, rg::launch_faces32(mx, h->stream, true));
+        RG_CUDA(h, rg::launch_update_mixed(mx, h->stream, false, true, true));
       }
     }
     for (int j = len - 1; j >= 0; --j) {
       const size_t J = static_cast<size_t>(j);
       rg::AdjArgs r = base;
-      r.cells = ptr<double>(A->seg_cells, 4 * np * J);
+      r.cells = ptr<float4>(A->seg_cells, np * J);
       r.ext = ptr<double>(A->seg_ext, 4 * n * J);
-      r.slopes = ptr<double>(A->seg_slopes, 8 * n * J);
-      r.trace = ptr<rg::SlopeTrace>(A->seg_trace, n * J);
+      r.slopes = ptr<float4>(A->seg_slopes, 2 * n * J);
+      r.trace = ptr<rg::SlopeTrace32>(A->seg_trace, n * J);
       const bool first = start + j == 0;
       RG_CUDA(h, rg::adj_launch_reverse32(r, cur, nxt, first ? ptr<double>(A->io) : nullptr, h->stream));
       std::swap(cur, nxt);

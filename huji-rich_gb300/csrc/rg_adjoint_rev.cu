@@ -40,7 +40,7 @@ namespace rg {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kFaceBlock = 128;  // FP64 k_adj_faces
+constexpr int kFaceBlock = 128;  // k_adj_faces
 
 __device__ __forceinline__ void load_raw(const double* c, int i, double o[4]) {
   const double2 a = reinterpret_cast<const double2*>(c)[2 * i];
@@ -58,14 +58,13 @@ __device__ __forceinline__ int source_of(const MeshDev& m, int p) { return p < m
 
 // Working precision of the face and cell reverse kernels: double here;
 // rg_adjoint_rev32.cu compiles them again with float (the FP32-mixed
-// adjoint), loading and storing the same FP64 arrays.
+// adjoint).  The recorded steps and the arrays between the kernels are of the
+// same precision (kept in FP64, the FP32 faces took 26 us where they take 16,
+// the trace slopes 18 where they take 15, at 256^2).
 using real = RG_ADJ_REAL;
 struct rv2 {
   real x, y;
 };
-// double <-> real; float on the integer pipes (rg_convert.cuh): the hardware
-// conversions take the FP64 unit, which bound the FP32 build (68-78 % active:
-// 256^2 faces 28.6 us, cells 19.7 us)
 __device__ __forceinline__ real to_real(double x) {
 #if RG_ADJ_FP64
   return x;
@@ -73,34 +72,56 @@ __device__ __forceinline__ real to_real(double x) {
   return narrow(x);
 #endif
 }
-__device__ __forceinline__ double from_real(real x) {
 #if RG_ADJ_FP64
-  return x;
+using Trace = SlopeTrace;
+__device__ __forceinline__ void load_r(const void* c, int i, real o[4]) { load_raw(static_cast<const double*>(c), i, o); }
+__device__ __forceinline__ void store_r(void* c, int i, const real v[4]) { store_raw(static_cast<double*>(c), i, v); }
+__device__ __forceinline__ void load_wide(const void* c, int i, double o[4]) { load_r(c, i, o); }
+// the geometry
+__device__ __forceinline__ rv2 r2(double2 v) { return rv2{v.x, v.y}; }
+__device__ __forceinline__ rv2 side_dm(const AdjArgs& a, int e, bool first) {
+  return r2(first ? a.geom.dm0[e] : a.geom.dm1[e]);
+}
+__device__ __forceinline__ rv2 entry_dm(const AdjArgs& a, int k) {
+  return side_dm(a, a.mesh.cell_faces[k], a.geom.nbr[k] & kNbrFirst);
+}
+__device__ __forceinline__ rv2 entry_h(const AdjArgs& a, int k) { return r2(a.geom.hr[k]); }
+__device__ __forceinline__ void load_minv(const AdjArgs& a, int i, real mi[4]) {
+  const dbl4 v = a.geom.minv[i];
+  mi[0] = v.x, mi[1] = v.y, mi[2] = v.z, mi[3] = v.w;
+}
 #else
-  return widen_exact(x);
-#endif
+using Trace = SlopeTrace32;
+__device__ __forceinline__ void load_r(const void* c, int i, real o[4]) {
+  const float4 v = static_cast<const float4*>(c)[i];
+  o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w;
 }
-__device__ __forceinline__ rv2 r2(double2 v) { return rv2{to_real(v.x), to_real(v.y)}; }
-__device__ __forceinline__ void load_r(const double* c, int i, real o[4]) {
-  double t[4];
-  load_raw(c, i, t);
+__device__ __forceinline__ void store_r(void* c, int i, const real v[4]) {
+  static_cast<float4*>(c)[i] = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void load_wide(const void* c, int i, double o[4]) {
+  real v[4];
+  load_r(c, i, v);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) o[q] = to_real(t[q]);
+  for (int q = 0; q < 4; ++q) o[q] = widen_exact(v[q]);
 }
-__device__ __forceinline__ void store_r(double* c, int i, const real v[4]) {
-  const double t[4] = {from_real(v[0]), from_real(v[1]), from_real(v[2]), from_real(v[3])};
-  store_raw(c, i, t);
+// the geometry: the handle's FP32 copies (roundings of the FP64 arrays)
+__device__ __forceinline__ rv2 r2(float2 v) { return rv2{v.x, v.y}; }
+__device__ __forceinline__ rv2 side_dm(const AdjArgs& a, int e, bool first) {
+  return r2(first ? a.g32.dm0[e] : a.g32.dm1[e]);
 }
-
-#if RG_ADJ_FP64
-// Periodic meshes only: every ghost has a source, no CSR entry is a
-// self-mirror and no cell uses the boundary slope.
-__global__ void __launch_bounds__(kBlock) k_adj_check(AdjArgs a) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < a.mesh.m && (a.geom.nbr[t] & kNbrMirror)) record_error(a.status, 0, RG_ERR_INVALID_ARGUMENT, 0, t, 0.0);
-  if (t < a.mesh.n && (a.geom.cflags[t] & kCellBoundarySlope))
-    record_error(a.status, 0, RG_ERR_INVALID_ARGUMENT, 1, t, 0.0);
+__device__ __forceinline__ rv2 entry_dm(const AdjArgs& a, int k) {
+  const float4 v = a.g32.ent[k];
+  return rv2{v.z, v.w};
 }
+__device__ __forceinline__ rv2 entry_h(const AdjArgs& a, int k) {
+  return r2(*reinterpret_cast<const float2*>(a.g32.ent + k));
+}
+__device__ __forceinline__ void load_minv(const AdjArgs& a, int i, real mi[4]) {
+  const float4 v = a.g32.minv[i];
+  mi[0] = v.x, mi[1] = v.y, mi[2] = v.z, mi[3] = v.w;
+}
+#endif
 
 // C'(U)^T w for SimpleCellUpdater (d = m/V, v = P/m, e = E/m - |v|^2/2,
 // p = (gamma-1) e d), added to ub.
@@ -116,6 +137,16 @@ __device__ __forceinline__ void cell_update_transpose(double gamma, double V, co
   ub[1] += quot(be, mass);
   ub[2] += quot(bvx, mass);
   ub[3] += quot(bvy, mass);
+}
+
+#if RG_ADJ_FP64
+// Periodic meshes only: every ghost has a source, no CSR entry is a
+// self-mirror and no cell uses the boundary slope.
+__global__ void __launch_bounds__(kBlock) k_adj_check(AdjArgs a) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < a.mesh.m && (a.geom.nbr[t] & kNbrMirror)) record_error(a.status, 0, RG_ERR_INVALID_ARGUMENT, 0, t, 0.0);
+  if (t < a.mesh.n && (a.geom.cflags[t] & kCellBoundarySlope))
+    record_error(a.status, 0, RG_ERR_INVALID_ARGUMENT, 1, t, 0.0);
 }
 
 __global__ void __launch_bounds__(kBlock) k_adj_seed(AdjArgs a, const double* wbar, double* ubar) {
@@ -301,8 +332,11 @@ __device__ __forceinline__ void hllc_reverse(O& o, double g, const Divisor& gm1,
 // Reverse of primitive conversion, rotation into the face frame, Hllc
 // (hllc.cpp:97-154, massflux, face at rest) and the rotation back: from fb
 // (adjoint of {mass, energy, px, py}) to the adjoints of the two states.
-__device__ void hllc_reverse(real g, rv2 n, real na, rv2 p, real pa, const real L[4], const real R[4],
-                             const real fb[4], real lb[4], real rb[4]) {
+// A call of its own: inlined, the compiler contracts other pairs of these
+// products, and the FP32 gradients differ in the last bits from what they were
+// (16.4 us a call, 14.9 inlined, at 256^2; 15.9 in blocks of 128).
+__device__ __noinline__ void hllc_reverse(real g, rv2 n, real na, rv2 p, real pa, const real L[4], const real R[4],
+                                          const real fb[4], real lb[4], real rb[4]) {
   // forward values
   const real dL = L[0], pL = L[1], dR = R[0], pR = R[1];
   const real eL = quot(quot(pL, dL), g - real(1)), cL = root(quot(g * pL, dL));
@@ -451,15 +485,14 @@ __device__ __forceinline__ bool face_reverse(O& o, const AdjArgs& a, const doubl
 #pragma unroll
   for (int q = 0; q < 4; ++q) fb[q] = to_real(scaled(o, fbd[q], s));
   real L[4], R[4], lb[4], rb[4];
-  face_state(a, fc.x, r2(a.geom.dm0[e]), L);
-  face_state(a, fc.y, r2(a.geom.dm1[e]), R);
+  face_state(a, fc.x, side_dm(a, e, true), L);
+  face_state(a, fc.y, side_dm(a, e, false), R);
 #if RG_ADJ_FP64
   hllc_reverse(o, a.gamma, a.gm1, r2(a.geom.nrm[e]), a.geom.nabs[e], r2(a.geom.par[e]), a.geom.area[e], L, R, fb, lb,
                rb);
   if (!o.ok) return false;
 #else
-  hllc_reverse(to_real(a.gamma), r2(a.geom.nrm[e]), to_real(a.geom.nabs[e]), r2(a.geom.par[e]),
-               to_real(a.geom.area[e]), L, R, fb, lb, rb);
+  hllc_reverse(to_real(a.gamma), r2(a.g32.nrm[e]), a.g32.nabs[e], r2(a.g32.par[e]), a.g32.area[e], L, R, fb, lb, rb);
 #endif
   store_r(a.side_bar, 2 * e, lb);
   store_r(a.side_bar, 2 * e + 1, rb);
@@ -484,7 +517,7 @@ __global__ void __launch_bounds__(kFaceBlock, 6) k_adj_faces(AdjArgs a, const do
   if (!face_reverse(o, a, ubar, e)) face_reverse_plain(a, ubar, e);
 }
 #else
-__global__ void __launch_bounds__(kBlock) k_adj_faces(AdjArgs a, const double* ubar) {
+__global__ void __launch_bounds__(kFaceBlock) k_adj_faces(AdjArgs a, const double* ubar) {
   chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.mesh.e) return;
@@ -493,88 +526,84 @@ __global__ void __launch_bounds__(kBlock) k_adj_faces(AdjArgs a, const double* u
 }
 #endif
 
+// a b + c d, the product that is rounded by itself fixed
+__device__ __forceinline__ real dot2(real a, real b, real c, real d) {
+#if RG_ADJ_FP64
+  return fma(a, b, c * d);
+#else
+  return fmaf(a, b, __fmul_rn(c, d));
+#endif
+}
+// Four lanes per cell, one component each: nothing passes between them, a
+// quad's loads and stores are its cell's records, and a 256^2 mesh gives every
+// SM 54 warps where a thread per cell gave 13 and waited for memory.  An entry
+// that also takes the limiter's share is stored again after the loop: an add
+// under the loop's test would cost the FP64 unit its clocks on every entry.
+// 256^2: FP64 48 -> 35 us (its unit 80 % busy before), FP32 20 -> 8.3 us.
 __global__ void __launch_bounds__(kBlock) k_adj_cell(AdjArgs a) {
   chain_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t >> 2, q = t & 3;
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
+  const Trace& tr = static_cast<const Trace*>(a.trace)[i];
+  const int b = m.cell_off[i], nn = m.cell_off[i + 1] - b;
+  const int code = tr.code[q];
   // face-state adjoints -> state adjoint w and slope adjoints bx, by
-  real w[4] = {0, 0, 0, 0}, bx[4] = {0, 0, 0, 0}, by[4] = {0, 0, 0, 0};
-  for (int k = a.side_off[i]; k < a.side_off[i + 1]; ++k) {
+  real w = 0, bx = 0, by = 0;
+  for (int k = a.side_off[i], end = a.side_off[i + 1]; k < end; ++k) {
     const int s = a.sides[k];
-    const int e = s >> 1;
-    const rv2 dm = r2((s & 1) ? a.geom.dm1[e] : a.geom.dm0[e]);
-    real sb[4];
-    load_r(a.side_bar, s, sb);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      w[q] += sb[q];
-      bx[q] += sb[q] * dm.x;
-      by[q] += sb[q] * dm.y;
-    }
+    const rv2 dm = side_dm(a, s >> 1, !(s & 1));
+    const real sb = static_cast<const real*>(a.side_bar)[4 * static_cast<size_t>(s) + q];
+    w += sb;
+    bx += sb * dm.x;
+    by += sb * dm.y;
   }
   // limiter: s = naive*psi
-  const SlopeTrace& tr = a.trace[i];
-  const int b = m.cell_off[i], nn = m.cell_off[i + 1] - b;
-  real bnx[4], bny[4], extra[4];
-  int ex_at[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int code = tr.code[q];
-    const int k = code & 0xff;
-    bnx[q] = bx[q];
-    bny[q] = by[q];
-    extra[q] = 0;
-    ex_at[q] = -1;
-    if (k == kTraceNone) continue;
-    const int kind = (code >> 8) & 3;
-    const real psi = to_real(tr.psi[q]);
-    bnx[q] = bx[q] * psi;
-    bny[q] = by[q] * psi;
-    if (kind == 3) continue;  // clamped to zero: no dependence
-    // psi = N/D with D = naive_x dm.x + naive_y dm.y (the centroid difference)
-    // and N = coef*(W[neighbour] - W[cell])
-    const real nx = to_real(tr.naive[q]), ny = to_real(tr.naive[4 + q]);
-    const real bpsi = bx[q] * nx + by[q] * ny;
-    const real D = to_real(tr.dphi[q]);
-    const real bN = quot(bpsi, D), bD = quot(-bpsi * psi, D);
-    const int e = m.cell_faces[b + k];
-    const rv2 dm = r2((a.geom.nbr[b + k] & kNbrFirst) ? a.geom.dm0[e] : a.geom.dm1[e]);
-    bnx[q] += bD * dm.x;
-    bny[q] += bD * dm.y;
-    const int ex = (code >> 16) - 1;
-    if (ex >= 0) {
-      extra[q] = (kind == 2 ? to_real(a.theta) : real(1)) * bN;
-      ex_at[q] = ex;
-      w[q] -= extra[q];
+  real bnx = bx, bny = by, extra = 0;
+  int ex_at = -1;
+  if ((code & 0xff) != kTraceNone) {
+    const int k = code & 0xff, kind = (code >> 8) & 3;
+    const real psi = tr.psi[q];
+    bnx = bx * psi;
+    bny = by * psi;
+    if (kind != 3) {  // else clamped to zero: no dependence
+      // psi = N/D with D = naive_x dm.x + naive_y dm.y (the centroid difference)
+      // and N = coef*(W[neighbour] - W[cell])
+      const real nx = tr.naive[q], ny = tr.naive[4 + q];
+      const real bpsi = dot2(bx, nx, by, ny);
+      const real D = tr.dphi[q];
+      const real bN = quot(bpsi, D), bD = quot(-bpsi * psi, D);
+      const rv2 dm = entry_dm(a, b + k);
+      bnx = dot2(bD, dm.x, bx, psi);
+      bny = dot2(bD, dm.y, by, psi);
+      ex_at = (code >> 16) - 1;
+      if (ex_at >= 0) {
+        const real coef = kind == 2 ? to_real(a.theta) : real(1);
+        extra = coef * bN;
+        w -= extra;
+      }
     }
   }
   // naive slope: nx = vx*mi.x + vy*mi.y, ny = vx*mi.z + vy*mi.w,
   // v = sum_k h_k (W[cell] + W[neighbour k])
-  const dbl4 mid = a.geom.minv[i];
-  const real mix = to_real(mid.x), miy = to_real(mid.y), miz = to_real(mid.z),
-             miw = to_real(mid.w);
-  real bvx[4], bvy[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    bvx[q] = bnx[q] * mix + bny[q] * miz;
-    bvy[q] = bnx[q] * miy + bny[q] * miw;
-  }
+  real mi[4];
+  load_minv(a, i, mi);
+  const real bvx = dot2(bnx, mi[0], bny, mi[2]), bvy = dot2(bnx, mi[1], bny, mi[3]);
+  real* out = static_cast<real*>(a.entry_bar) + 4 * static_cast<size_t>(b) + q;
+  real at = 0;
   for (int k = 0; k < nn; ++k) {
-    const rv2 h = r2(a.geom.hr[b + k]);
-    real c[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      c[q] = bvx[q] * h.x + bvy[q] * h.y;
-      w[q] += c[q];
-      if (ex_at[q] == k) c[q] += extra[q];
-    }
-    store_r(a.entry_bar, b + k, c);
+    const rv2 h = entry_h(a, b + k);
+    const real c = dot2(bvx, h.x, bvy, h.y);
+    w += c;
+    if (ex_at == k) at = c;
+    out[4 * k] = c;
   }
-  store_r(a.self_bar, i, w);
+  if (ex_at >= 0) out[4 * ex_at] = at + extra;
+  static_cast<real*>(a.self_bar)[t] = w;
 }
 
-#if RG_ADJ_FP64
+// (all in FP64; the shares and the state are records of the working precision)
 __global__ void __launch_bounds__(kBlock) k_adj_update(AdjArgs a, const double* ubar_in, double* ubar_out,
                                                        double* grad) {
   chain_wait();
@@ -582,10 +611,10 @@ __global__ void __launch_bounds__(kBlock) k_adj_update(AdjArgs a, const double* 
   const MeshDev& m = a.mesh;
   if (i >= m.n) return;
   double w[4];
-  load_raw(a.self_bar, i, w);
+  load_wide(a.self_bar, i, w);
   for (int k = a.target_off[i]; k < a.target_off[i + 1]; ++k) {
     double c[4];
-    load_raw(a.entry_bar, a.targets[k], c);
+    load_wide(a.entry_bar, a.targets[k], c);
 #pragma unroll
     for (int q = 0; q < 4; ++q) w[q] += c[q];
   }
@@ -595,7 +624,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_update(AdjArgs a, const double* 
   if (grad) {
     // U_0 = I(W_0): mass = V d, E = V p/(gamma-1) + V d |v|^2/2, P = mass v
     double c[4];
-    load_raw(a.cells, i, c);
+    load_wide(a.cells, i, c);
     const double k2 = c[2] * c[2] + c[3] * c[3];
     const double mass = V * c[0];
     double g[4];
@@ -612,16 +641,14 @@ __global__ void __launch_bounds__(kBlock) k_adj_update(AdjArgs a, const double* 
   store_raw(ubar_out, i, ub);
 }
 
-#endif  // RG_ADJ_FP64
-
-inline int blocks(int n) { return (n + kBlock - 1) / kBlock; }
+inline long long blocks(long long n) { return (n + kBlock - 1) / kBlock; }
 
 }  // namespace
 
 #if RG_ADJ_FP64
 cudaError_t adj_launch_check(const AdjArgs& a, cudaStream_t s) {
   const int n = a.mesh.m > a.mesh.n ? a.mesh.m : a.mesh.n;
-  k_adj_check<<<blocks(n), kBlock, 0, s>>>(a);
+  k_adj_check<<<static_cast<unsigned>(blocks(n)), kBlock, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -630,24 +657,20 @@ cudaError_t adj_launch_seed(const AdjArgs& a, const double* wbar, double* ubar, 
   return cudaGetLastError();
 }
 
-cudaError_t adj_launch_update(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
-                              cudaStream_t s) {
-  chain(s, blocks(a.mesh.n), kBlock, k_adj_update, a, ubar_in, ubar_out, grad);
-  return cudaGetLastError();
-}
-
 cudaError_t adj_launch_reverse(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
                                cudaStream_t s) {
   chain(s, (a.mesh.e + kFaceBlock - 1) / kFaceBlock, kFaceBlock, k_adj_faces, a, ubar_in);
-  chain(s, blocks(a.mesh.n), kBlock, k_adj_cell, a);
-  return adj_launch_update(a, ubar_in, ubar_out, grad, s);
+  chain(s, blocks(4 * static_cast<long long>(a.mesh.n)), kBlock, k_adj_cell, a);
+  chain(s, blocks(a.mesh.n), kBlock, k_adj_update, a, ubar_in, ubar_out, grad);
+  return cudaGetLastError();
 }
 #else
 cudaError_t adj_launch_reverse32(const AdjArgs& a, const double* ubar_in, double* ubar_out, double* grad,
                                  cudaStream_t s) {
-  chain(s, blocks(a.mesh.e), kBlock, k_adj_faces, a, ubar_in);
-  chain(s, blocks(a.mesh.n), kBlock, k_adj_cell, a);
-  return adj_launch_update(a, ubar_in, ubar_out, grad, s);
+  chain(s, (a.mesh.e + kFaceBlock - 1) / kFaceBlock, kFaceBlock, k_adj_faces, a, ubar_in);
+  chain(s, blocks(4 * static_cast<long long>(a.mesh.n)), kBlock, k_adj_cell, a);
+  chain(s, blocks(a.mesh.n), kBlock, k_adj_update, a, ubar_in, ubar_out, grad);
+  return cudaGetLastError();
 }
 #endif
 

@@ -411,7 +411,10 @@ cudaError_t launch_geom_ghosts(const GeomArgs& a, cudaStream_t s);  // the ghost
 cudaError_t launch_cfl(const StepArgs& a, cudaStream_t s);
 cudaError_t launch_slopes(const StepArgs& a, cudaStream_t s);
 // the slopes with the adjoint's limiter trace (periodic meshes, one problem)
-struct SlopeTrace;
+template <class R>
+struct SlopeTraceOf;
+using SlopeTrace = SlopeTraceOf<double>;
+using SlopeTrace32 = SlopeTraceOf<float>;
 cudaError_t launch_slopes_trace(const StepArgs& a, SlopeTrace* trace, cudaStream_t s);
 cudaError_t launch_faces(const StepArgs& a, cudaStream_t s, bool scaled);
 cudaError_t launch_update(const StepArgs& a, cudaStream_t s, bool from_unscaled, bool extensive, bool cells);

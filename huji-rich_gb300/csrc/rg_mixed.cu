@@ -423,12 +423,12 @@ __device__ __forceinline__ void shocked32(float dphi, float cv, float cellv, flo
 // The FP32 slopes of a periodic mesh (no self-mirror neighbour, no boundary
 // slope), written widened and as the FP32 slopes the face kernel reads, with
 // the limiter trace the adjoint's reverse slope kernel reads
-// (SlopeTrace: the unlimited slope, each component's factor, the centroid
+// (SlopeTrace32: the unlimited slope, each component's factor, the centroid
 // difference and neighbour of its active candidate).  The arithmetic is
 // k_slopes32_item's; the arg max / min follow the first strict improvement
 // as std::max / std::min do, and each psi is the smallest candidate taken in
 // edge order, which is what fminf over the candidates gives.
-__global__ void __launch_bounds__(kBlock) k_slopes32_trace(MixedArgs a, double* slopes64, SlopeTrace* trace) {
+__global__ void __launch_bounds__(kBlock) k_slopes32_trace(MixedArgs a, SlopeTrace32* trace) {
   chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(kBlock) k_slopes32_trace(MixedArgs a, double* 
   naive_slope(false, vx, vy, mi, nx, ny);
   float sx[4] = {nx.d, nx.p, nx.vx, nx.vy};
   float sy[4] = {ny.d, ny.p, ny.vx, ny.vy};
-  SlopeTrace& tr = trace[i];
+  SlopeTrace32& tr = trace[i];
   const float cq[4] = {cell.d, cell.p, cell.vx, cell.vy};
   float psi[4] = {1, 1, 1, 1};
 #pragma unroll
@@ -516,18 +516,12 @@ __global__ void __launch_bounds__(kBlock) k_slopes32_trace(MixedArgs a, double* 
       }
     }
   }
-  double2* o = reinterpret_cast<double2*>(slopes64) + 4 * i;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     tr.psi[q] = psi[q];
     sx[q] *= psi[q];
     sy[q] *= psi[q];
   }
-  o[0] = make_double2(sx[0], sx[1]);
-  o[1] = make_double2(sx[2], sx[3]);
-  o[2] = make_double2(sy[0], sy[1]);
-  o[3] = make_double2(sy[2], sy[3]);
-  // the same slopes for the face kernel of the recomputed step
   a.slopes32[2 * i] = make_float4(sx[0], sx[1], sx[2], sx[3]);
   a.slopes32[2 * i + 1] = make_float4(sy[0], sy[1], sy[2], sy[3]);
 }
@@ -1239,8 +1233,8 @@ cudaError_t launch_cfl32(const MixedArgs& a, cudaStream_t s) {
   a.cell_problem ? chain(s, nb, sh.block, k_cfl32<true>, a) : chain(s, nb, sh.block, k_cfl32<false>, a);
   return cudaGetLastError();
 }
-cudaError_t launch_slopes32_trace(const MixedArgs& a, double* slopes64, SlopeTrace* trace, cudaStream_t s) {
-  if (a.mesh.n > 0) chain(s, (a.mesh.n + kBlock - 1) / kBlock, kBlock, k_slopes32_trace, a, slopes64, trace);
+cudaError_t launch_slopes32_trace(const MixedArgs& a, SlopeTrace32* trace, cudaStream_t s) {
+  if (a.mesh.n > 0) chain(s, (a.mesh.n + kBlock - 1) / kBlock, kBlock, k_slopes32_trace, a, trace);
   return cudaGetLastError();
 }
 
