@@ -1,9 +1,6 @@
 // rg_adjoint.cu -- forward side of the differentiated step (FP64, compiled
 // without FMA contraction like rg_fp64.cu):
 //
-//   adj_launch_record_slopes  LinearGaussImproved slopes of W_k with the
-//                    limiter trace the reverse slope kernel needs
-//                    (SlopeTrace): rg_fp64.cu's slopes kernel, its trace build
 //   k_tl_*           tangent-linear model: the same formulas on dual numbers
 //                    (value, tangent).  The value parts follow the production
 //                    kernels' operation order, so a tangent run reproduces the
@@ -386,23 +383,6 @@ __global__ void __launch_bounds__(kBlock) k_tl_init(AdjArgs a) {
 inline int blocks(int n) { return (n + kBlock - 1) / kBlock; }
 
 }  // namespace
-
-cudaError_t adj_launch_record_slopes(const AdjArgs& a, cudaStream_t s) {
-  StepArgs t{};
-  t.mesh = a.mesh;
-  t.geom = a.geom;
-  t.gamma = a.gamma;
-  t.order = 2;
-  t.ghost_kind = RG_GHOST_PERIODIC;
-  t.slf = a.slf;
-  t.delta_v = a.delta_v;
-  t.theta = a.theta;
-  t.delta_p = a.delta_p;
-  t.cells = const_cast<double*>(cells64(a));
-  t.slopes = slopes64(a);
-  t.status = a.status;
-  return launch_slopes_trace(t, static_cast<SlopeTrace*>(a.trace), s);
-}
 
 cudaError_t tl_launch_init(const AdjArgs& a, cudaStream_t s) {
   k_tl_init<<<blocks(a.mesh.n), kBlock, 0, s>>>(a);

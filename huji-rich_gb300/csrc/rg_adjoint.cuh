@@ -70,7 +70,6 @@ struct AdjArgs {
 };
 
 // rg_adjoint.cu (plain FP64: the values equal the production path bit for bit)
-cudaError_t adj_launch_record_slopes(const AdjArgs& a, cudaStream_t s);
 cudaError_t tl_launch_init(const AdjArgs& a, cudaStream_t s);
 cudaError_t tl_launch_step(const AdjArgs& a, cudaStream_t s);
 

@@ -2,23 +2,28 @@
 // rg_step_fwd / rg_step_bwd (adjoint pair with checkpointing) and
 // rg_step_tlm (tangent-linear run).
 //
-// Forward: the plain FP64 kernels of rg_fp64.cu with the fixed dt (ghost
-// fill, slopes, dt*area-scaled fluxes, update), W and U copied to a
-// checkpoint every `every` steps.
+// Forward: the plain FP64 kernels of rg_fp64.cu with the fixed dt (slopes,
+// dt*area-scaled fluxes, update), W and U copied to a checkpoint every `every`
+// steps; the steps of the last interval are recorded as they run.
 // Backward: per checkpoint interval, last first: the interval is recomputed
-// from its checkpoint into per-step buffers (W_k with ghost records, U_k, the
-// slopes and the limiter trace of k_record_slopes, which yields the same
-// slopes as the plain path), then the reverse steps run from the interval's
-// last step to its first.  Memory: (n_steps/every) checkpoints of 64 bytes
-// per cell plus `every` recomputed steps of about 240 bytes per cell.
+// from its checkpoint into per-step records (W_k, U_k, the slopes and their
+// limiter trace, by the trace build of the slopes kernel, which yields the
+// same slopes as the plain one), then the reverse steps run from the
+// interval's last step to its first.  The last interval's records are the
+// forward's own; a second backward recomputes it where there are others.
+// Memory: (n_steps/every) checkpoints of 64 bytes per cell plus `every`
+// recorded steps of about 270 bytes per cell (FP32-mixed 150).
+// (Recomputing the last interval as well took a quarter of the time of a run
+// of one interval: 20 FP64 steps at 256^2 5.79 ms against 4.09, 40 FP32-mixed
+// steps in two intervals 3.38 against 3.05.)
 // The reverse adjacency (which face sides and CSR entries read each cell)
 // is built once per mesh on the host, in ascending order, so every reverse
 // gather is deterministic.
 // FP32-mixed handles differentiate the FP32-mixed step: the forward and the
-// recomputation run the FP32-mixed kernels, the recomputation records the
-// limiter trace of the FP32 slopes (k_slopes32_trace), and the reverse runs
-// the face and cell kernels in FP32 with the FP64 transposed gather and cell
-// update (adj_launch_reverse32).  Checkpoints hold the FP32 primitives.
+// recomputation run the FP32-mixed kernels, with the limiter trace of the FP32
+// slopes (k_slopes32_trace), and the reverse runs the face and cell kernels in
+// FP32 with the FP64 transposed gather and cell update (adj_launch_reverse32).
+// Checkpoints and records hold the FP32 primitives.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,6 +44,7 @@ struct rg_adjoint_state {
   // forward record
   bool have_forward = false;
   int n_steps = 0, every = 0, n_ckpt = 0;
+  int recorded = -1;  // the interval whose steps the records below hold (-1: none)
   double dt = 0;
   DevBuf ckpt_cells, ckpt_ext, final_ext;
   // recomputed interval
@@ -181,17 +187,6 @@ rg_status ensure_adjacency(rg_handle* h) {
   return RG_OK;
 }
 
-// The plain FP64 step with a fixed dt, from a.cells / a.ext into
-// a.cells_out / a.ext_out (nullptr: in place).
-rg_status enqueue_plain_step(rg_handle* h, const rg::StepArgs& a, bool faces_and_update = true) {
-  RG_CUDA(h, rg::launch_slopes(a, h->stream));
-  if (faces_and_update) {
-    RG_CUDA(h, rg::launch_faces(a, h->stream, true));
-    RG_CUDA(h, rg::launch_update(a, h->stream, false, true, true));
-  }
-  return RG_OK;
-}
-
 rg_status check_run(rg_handle* h, int32_t n_steps, double dt, bool allow_mixed = true) {
   if (rg_status st = require(h, true, false, false, false)) return st;
   if (rg_status st = check_config(h, allow_mixed)) return st;
@@ -200,20 +195,86 @@ rg_status check_run(rg_handle* h, int32_t n_steps, double dt, bool allow_mixed =
   return ensure_adjacency(h);
 }
 
-// One FP32-mixed step with a fixed dt on the FP32 primitives and FP64
-// extensives of `m` (in place).
-rg_status enqueue_mixed_step(rg_handle* h, const rg::MixedArgs& m) {
+rg::MixedArgs mixed_fixed_dt(rg_handle* h, double dt) {
+  rg::MixedArgs m = mixed_args(h);
+  m.dt32 = static_cast<float>(dt);
+  m.dt32_from_device = 0;
+  return m;
+}
+rg::StepArgs fixed_dt(rg_handle* h, double dt) {
+  rg::StepArgs a = step_args(h);
+  a.dt_host = dt;
+  return a;
+}
+
+// One step with a fixed dt: the handle's state in place, or from a record
+// into the next one (a.cells_out / a.ext_out); with a trace its slopes and
+// their limiter trace are kept.
+rg_status fixed_step(rg_handle* h, rg::StepArgs a, int step) {
+  a.step = std::min(step, 0x1fff);
+  RG_CUDA(h, rg::launch_slopes(a, h->stream));
+  RG_CUDA(h, rg::launch_faces(a, h->stream, true));
+  RG_CUDA(h, rg::launch_update(a, h->stream, false, true, true));
+  return RG_OK;
+}
+rg_status fixed_step(rg_handle* h, rg::MixedArgs m, int step) {
+  m.step = std::min(step, 0x1fff);
   RG_CUDA(h, rg::launch_slopes32(m, h->stream));
   RG_CUDA(h, rg::launch_faces32(m, h->stream, true));
   RG_CUDA(h, rg::launch_update_mixed(m, h->stream, false, true, true));
   return RG_OK;
 }
 
-rg::MixedArgs mixed_fixed_dt(rg_handle* h, double dt) {
-  rg::MixedArgs m = mixed_args(h);
-  m.dt32 = static_cast<float>(dt);
-  m.dt32_from_device = 0;
-  return m;
+// The steps start .. start + len - 1 into the interval's records, whose first
+// state and extensives are there: each step's update writes the next step's
+// record.  The last step ends with its slopes, or (finish) goes on into the
+// handle's cells and extensives.
+rg_status record_steps(rg_handle* h, int start, int len, bool finish) {
+  rg_adjoint_state* A = h->adj;
+  const MeshSlot* s = active_slot(h);
+  const size_t n = static_cast<size_t>(s->n), np = n + static_cast<size_t>(s->g);
+  const rg::AdjArgs base = adj_args(h);
+  const rg::StepArgs a = fixed_dt(h, A->dt);
+  for (int j = 0; j < len; ++j) {
+    const size_t J = static_cast<size_t>(j);
+    const bool last = j + 1 == len;
+    double* ext = ptr<double>(A->seg_ext, 4 * n * J);
+    double* ext_out = last ? static_cast<double*>(h->ext.p) : ext + 4 * n;
+    if (h->mixed) {
+      rg::MixedArgs m = mixed_fixed_dt(h, A->dt);
+      m.step = std::min(start + j, 0x1fff);
+      m.cells32 = ptr<float4>(A->seg_cells, np * J);
+      m.cells32_out = last ? static_cast<float4*>(h->cells32.p) : m.cells32 + np;
+      m.slopes32 = ptr<float4>(A->seg_slopes, 2 * n * J);
+      m.ext = ext;
+      m.ext_out = ext_out;
+      RG_CUDA(h, rg::launch_slopes32_trace(m, ptr<rg::SlopeTrace32>(A->seg_trace, n * J), h->stream));
+      if (last && !finish) break;
+      RG_CUDA(h, rg::launch_faces32(m, h->stream, true));
+      RG_CUDA(h, rg::launch_update_mixed(m, h->stream, false, true, true));
+    } else {
+      rg::StepArgs aj = a;
+      aj.step = std::min(start + j, 0x1fff);
+      aj.cells = ptr<double>(A->seg_cells, 4 * np * J);
+      aj.cells_out = last ? static_cast<double*>(h->cells.p) : aj.cells + 4 * np;
+      aj.slopes = ptr<double>(A->seg_slopes, 8 * n * J);
+      aj.ext = ext;
+      aj.ext_out = ext_out;
+      RG_CUDA(h, rg::launch_slopes_trace(aj, ptr<rg::SlopeTrace>(A->seg_trace, n * J), h->stream));
+      if (last && !finish) break;
+      RG_CUDA(h, rg::launch_faces(aj, h->stream, true));
+      RG_CUDA(h, rg::launch_update(aj, h->stream, false, true, true));
+    }
+  }
+  return RG_OK;
+}
+
+// {cells, extensives} of checkpoint c (32 or, FP32-mixed, 16 bytes a cell)
+rg_status copy_state(rg_handle* h, void* cells, void* ext, const void* from_cells, const void* from_ext) {
+  const size_t n = static_cast<size_t>(active_slot(h)->n);
+  RG_CUDA(h, cudaMemcpyAsync(cells, from_cells, (h->mixed ? 16 : 32) * n, cudaMemcpyDeviceToDevice, h->stream));
+  RG_CUDA(h, cudaMemcpyAsync(ext, from_ext, 32 * n, cudaMemcpyDeviceToDevice, h->stream));
+  return RG_OK;
 }
 
 }  // namespace
@@ -240,39 +301,36 @@ rg_status rg_step_fwd(rg_handle* h, int32_t n_steps, double dt, int32_t every) {
   RG_CUDA(h, A->seg_slopes.ensure((h->mixed ? 32 : 64) * n * seg));
   RG_CUDA(h, A->seg_trace.ensure((h->mixed ? sizeof(rg::SlopeTrace32) : sizeof(rg::SlopeTrace)) * n * seg));
   RG_TRY(reset_status(h, h->d_status, h->stream));
-  rg::StepArgs a = step_args(h);
-  a.dt_host = dt;
+  A->dt = dt;
+  A->recorded = -1;
+  const rg::StepArgs a = fixed_dt(h, dt);
   if (h->mixed) {
     // U_0 from the FP32 primitives the mixed steps start from
     RG_CUDA(h, rg::launch_cells_to64(static_cast<const float4*>(h->cells32.p), static_cast<double*>(h->cells.p),
                                      s->n, h->stream));
-    RG_CUDA(h, rg::launch_init_extensives(a, h->stream));
-    const rg::MixedArgs mx = mixed_fixed_dt(h, dt);
-    for (int k = 0; k < n_steps; ++k) {
-      if (k % every == 0) {
-        const size_t c = static_cast<size_t>(k / every);
-        RG_CUDA(h, cudaMemcpyAsync(ptr<double>(A->ckpt_cells, 4 * n * c), h->cells32.p, 16 * n,
-                                   cudaMemcpyDeviceToDevice, h->stream));
-        RG_CUDA(h, cudaMemcpyAsync(ptr<double>(A->ckpt_ext, 4 * n * c), h->ext.p, 32 * n, cudaMemcpyDeviceToDevice,
-                                   h->stream));
-      }
-      rg::MixedArgs mk = mx;
-      mk.step = std::min(k, 0x1fff);
-      RG_TRY(enqueue_mixed_step(h, mk));
-    }
-  } else {
-    RG_CUDA(h, rg::launch_init_extensives(a, h->stream));
   }
-  for (int k = 0; k < (h->mixed ? 0 : n_steps); ++k) {
+  RG_CUDA(h, rg::launch_init_extensives(a, h->stream));
+  const rg::MixedArgs mx = h->mixed ? mixed_fixed_dt(h, dt) : rg::MixedArgs{};
+  const void* cells = h->mixed ? h->cells32.p : h->cells.p;
+  // the last interval is recorded as it runs, the others leave a checkpoint
+  const int tail = (n_ckpt - 1) * every;
+  for (int k = 0; k < tail; ++k) {
     if (k % every == 0) {
       const size_t c = static_cast<size_t>(k / every);
-      RG_CUDA(h, cudaMemcpyAsync(ptr<double>(A->ckpt_cells, 4 * n * c), h->cells.p, 32 * n, cudaMemcpyDeviceToDevice,
-                                 h->stream));
-      RG_CUDA(h, cudaMemcpyAsync(ptr<double>(A->ckpt_ext, 4 * n * c), h->ext.p, 32 * n, cudaMemcpyDeviceToDevice,
-                                 h->stream));
+      RG_TRY(copy_state(h, ptr<double>(A->ckpt_cells, 4 * n * c), ptr<double>(A->ckpt_ext, 4 * n * c), cells,
+                        h->ext.p));
     }
-    a.step = std::min(k, 0x1fff);
-    RG_TRY(enqueue_plain_step(h, a));
+    if (h->mixed)
+      RG_TRY(fixed_step(h, mx, k));
+    else
+      RG_TRY(fixed_step(h, a, k));
+  }
+  {
+    const size_t c = static_cast<size_t>(n_ckpt - 1);
+    RG_TRY(copy_state(h, ptr<double>(A->ckpt_cells, 4 * n * c), ptr<double>(A->ckpt_ext, 4 * n * c), cells, h->ext.p));
+    RG_TRY(copy_state(h, A->seg_cells.p, A->seg_ext.p, cells, h->ext.p));
+    RG_TRY(record_steps(h, tail, n_steps - tail, true));
+    A->recorded = n_ckpt - 1;
   }
   RG_CUDA(h, cudaMemcpyAsync(A->final_ext.p, h->ext.p, 32 * n, cudaMemcpyDeviceToDevice, h->stream));
   h->have_ext = true;
@@ -282,7 +340,6 @@ rg_status rg_step_fwd(rg_handle* h, int32_t n_steps, double dt, int32_t every) {
   A->n_steps = n_steps;
   A->every = every;
   A->n_ckpt = n_ckpt;
-  A->dt = dt;
   A->have_forward = true;
   return RG_OK;
 }
@@ -304,82 +361,34 @@ rg_status rg_step_bwd(rg_handle* h, const double* cells_bar, double* cells0_bar)
   double* cur = ptr<double>(A->ubar0);
   double* nxt = ptr<double>(A->ubar1);
   RG_CUDA(h, rg::adj_launch_seed(base, ptr<double>(A->io), cur, h->stream));
-  rg::StepArgs a = step_args(h);
-  a.dt_host = A->dt;
-  for (int c = A->n_ckpt - 1; c >= 0 && h->mixed; --c) {
-    // FP32-mixed: recompute the interval with the mixed kernels, recording
-    // each step's state (widened), extensives, FP32 slopes and their trace
+  for (int c = A->n_ckpt - 1; c >= 0; --c) {
     const int start = c * A->every;
     const int len = std::min(A->every, A->n_steps - start);
-    RG_CUDA(h, cudaMemcpyAsync(A->seg_cells.p, ptr<double>(A->ckpt_cells, 4 * n * static_cast<size_t>(c)), 16 * n,
-                               cudaMemcpyDeviceToDevice, h->stream));
-    RG_CUDA(h, cudaMemcpyAsync(A->seg_ext.p, ptr<double>(A->ckpt_ext, 4 * n * static_cast<size_t>(c)), 32 * n,
-                               cudaMemcpyDeviceToDevice, h->stream));
-    rg::MixedArgs mx = mixed_fixed_dt(h, A->dt);
-    for (int j = 0; j < len; ++j) {
-      const size_t J = static_cast<size_t>(j);
-      // each step's update writes into the next step's record
-      mx.cells32 = ptr<float4>(A->seg_cells, np * J);
-      mx.cells32_out = ptr<float4>(A->seg_cells, np * (J + 1));
-      mx.slopes32 = ptr<float4>(A->seg_slopes, 2 * n * J);
-      mx.ext = ptr<double>(A->seg_ext, 4 * n * J);
-      mx.ext_out = ptr<double>(A->seg_ext, 4 * n * (J + 1));
-      mx.step = std::min(start + j, 0x1fff);
-      RG_CUDA(h, rg::launch_slopes32_trace(mx, ptr<rg::SlopeTrace32>(A->seg_trace, n * J), h->stream));
-      if (j + 1 < len) {
-        RG_CUDA(h, rg::launch_faces32(mx, h->stream, true));
-        RG_CUDA(h, rg::launch_update_mixed(mx, h->stream, false, true, true));
-      }
-    }
-    for (int j = len - 1; j >= 0; --j) {
-      const size_t J = static_cast<size_t>(j);
-      rg::AdjArgs r = base;
-      r.cells = ptr<float4>(A->seg_cells, np * J);
-      r.ext = ptr<double>(A->seg_ext, 4 * n * J);
-      r.slopes = ptr<float4>(A->seg_slopes, 2 * n * J);
-      r.trace = ptr<rg::SlopeTrace32>(A->seg_trace, n * J);
-      const bool first = start + j == 0;
-      RG_CUDA(h, rg::adj_launch_reverse32(r, cur, nxt, first ? ptr<double>(A->io) : nullptr, h->stream));
-      std::swap(cur, nxt);
-    }
-  }
-  for (int c = h->mixed ? -1 : A->n_ckpt - 1; c >= 0; --c) {
-    const int start = c * A->every;
-    const int len = std::min(A->every, A->n_steps - start);
-    RG_CUDA(h, cudaMemcpyAsync(A->seg_cells.p, ptr<double>(A->ckpt_cells, 4 * n * static_cast<size_t>(c)), 32 * n,
-                               cudaMemcpyDeviceToDevice, h->stream));
-    RG_CUDA(h, cudaMemcpyAsync(A->seg_ext.p, ptr<double>(A->ckpt_ext, 4 * n * static_cast<size_t>(c)), 32 * n,
-                               cudaMemcpyDeviceToDevice, h->stream));
-    // recompute the interval: W_j, U_j, slopes and trace of every step in it
-    for (int j = 0; j < len; ++j) {
-      const size_t J = static_cast<size_t>(j);
-      rg::StepArgs aj = a;
-      aj.step = std::min(start + j, 0x1fff);
-      aj.cells = ptr<double>(A->seg_cells, 4 * np * J);
-      aj.ext = ptr<double>(A->seg_ext, 4 * n * J);
-      aj.slopes = ptr<double>(A->seg_slopes, 8 * n * J);
-      aj.cells_out = ptr<double>(A->seg_cells, 4 * np * (J + 1));
-      aj.ext_out = ptr<double>(A->seg_ext, 4 * n * (J + 1));
-      rg::AdjArgs r = base;
-      r.cells = aj.cells;
-      r.slopes = aj.slopes;
-      r.trace = ptr<rg::SlopeTrace>(A->seg_trace, n * J);
-      RG_CUDA(h, rg::adj_launch_record_slopes(r, h->stream));
-      if (j + 1 < len) {
-        RG_CUDA(h, rg::launch_faces(aj, h->stream, true));
-        RG_CUDA(h, rg::launch_update(aj, h->stream, false, true, true));
-      }
+    if (A->recorded != c) {
+      A->recorded = -1;
+      const size_t C = static_cast<size_t>(c);
+      RG_TRY(copy_state(h, A->seg_cells.p, A->seg_ext.p, ptr<double>(A->ckpt_cells, 4 * n * C),
+                        ptr<double>(A->ckpt_ext, 4 * n * C)));
+      RG_TRY(record_steps(h, start, len, false));
+      A->recorded = c;
     }
     // reverse steps
     for (int j = len - 1; j >= 0; --j) {
       const size_t J = static_cast<size_t>(j);
       rg::AdjArgs r = base;
-      r.cells = ptr<double>(A->seg_cells, 4 * np * J);
       r.ext = ptr<double>(A->seg_ext, 4 * n * J);
-      r.slopes = ptr<double>(A->seg_slopes, 8 * n * J);
-      r.trace = ptr<rg::SlopeTrace>(A->seg_trace, n * J);
-      const bool first = start + j == 0;
-      RG_CUDA(h, rg::adj_launch_reverse(r, cur, nxt, first ? ptr<double>(A->io) : nullptr, h->stream));
+      double* grad = start + j == 0 ? ptr<double>(A->io) : nullptr;
+      if (h->mixed) {
+        r.cells = ptr<float4>(A->seg_cells, np * J);
+        r.slopes = ptr<float4>(A->seg_slopes, 2 * n * J);
+        r.trace = ptr<rg::SlopeTrace32>(A->seg_trace, n * J);
+        RG_CUDA(h, rg::adj_launch_reverse32(r, cur, nxt, grad, h->stream));
+      } else {
+        r.cells = ptr<double>(A->seg_cells, 4 * np * J);
+        r.slopes = ptr<double>(A->seg_slopes, 8 * n * J);
+        r.trace = ptr<rg::SlopeTrace>(A->seg_trace, n * J);
+        RG_CUDA(h, rg::adj_launch_reverse(r, cur, nxt, grad, h->stream));
+      }
       std::swap(cur, nxt);
     }
   }
