@@ -39,7 +39,9 @@
 namespace rg {
 namespace {
 
-constexpr int kBlock = 256;
+// (per cell: small blocks spread a 256^2 mesh's 1 to 4 warps per SM sub-partition
+// evenly; cells 34.9 us in blocks of 256, 33.5 of 64, update 12.7 and 12.1)
+constexpr int kBlock = 64;
 constexpr int kFaceBlock = 128;  // k_adj_faces
 
 __device__ __forceinline__ void load_raw(const double* c, int i, double o[4]) {
@@ -539,7 +541,7 @@ __device__ __forceinline__ real dot2(real a, real b, real c, real d) {
 // SM 54 warps where a thread per cell gave 13 and waited for memory.  An entry
 // that also takes the limiter's share is stored again after the loop: an add
 // under the loop's test would cost the FP64 unit its clocks on every entry.
-// 256^2: FP64 48 -> 35 us (its unit 80 % busy before), FP32 20 -> 8.3 us.
+// 256^2: FP64 48 -> 34 us (its unit 80 % busy before), FP32 20 -> 8.3 us.
 __global__ void __launch_bounds__(kBlock) k_adj_cell(AdjArgs a) {
   chain_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
