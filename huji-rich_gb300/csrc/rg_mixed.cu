@@ -21,6 +21,7 @@
 #include "rg_adjoint.cuh"
 #include "rg_convert.cuh"
 #include "rg_div.cuh"
+#include "rg_limit32.cuh"
 #include "rg_mixed.cuh"
 
 namespace rg {
@@ -399,27 +400,6 @@ __global__ void __launch_bounds__(kMaxBlock) k_cfl32(MixedArgs a) {
                  a.cfl, &a.status->dt, &a.status->dt32, a.dt_trace);
 }
 
-// The limiters' candidate of one neighbour, without branches: the candidate
-// quotient is always formed and taken only where the limiter takes it, so
-// psi is the same bits as with the limiter's if / else-if, and a warp's
-// lanes never diverge here.
-__device__ __forceinline__ void limit32(float dphi, float cv, float cellv, float thr, float maxd, float mind,
-                                        bool use_abs, float& psi) {
-  const bool active = fabsf(dphi) > thr || cv * cellv < 0.0f;
-  const float t = use_abs ? fabsf(1e-9f * cellv) : 1e-9f * cellv;
-  const float nt = use_abs ? -fabsf(1e-9f * cellv) : -1e-9f * cellv;
-  const bool up = dphi > t;
-  const float cand = __fdividef(up ? maxd : mind, dphi);
-  psi = active && (up || dphi < nt) ? fminf(psi, cand) : psi;
-}
-
-__device__ __forceinline__ void shocked32(float dphi, float cv, float cellv, float thr, float nbv, float theta,
-                                          float& psi) {
-  const bool active = (fabsf(dphi) > thr || cv * cellv < 0.0f) && fabsf(dphi) > 1e-9f * cellv;
-  const float cand = fmaxf(__fdividef(theta * (nbv - cellv), dphi), 0.0f);
-  psi = active ? fminf(psi, cand) : psi;
-}
-
 // The FP32 slopes of a periodic mesh (no self-mirror neighbour, no boundary
 // slope), written widened and as the FP32 slopes the face kernel reads, with
 // the limiter trace the adjoint's reverse slope kernel reads
@@ -526,85 +506,105 @@ __global__ void __launch_bounds__(kBlock) k_slopes32_trace(MixedArgs a, SlopeTra
   a.slopes32[2 * i + 1] = make_float4(sy[0], sy[1], sy[2], sy[3]);
 }
 
+__device__ __forceinline__ void widen_range(const C4& v, C4& hi, C4& lo) {
+  hi = C4{fmaxf(hi.d, v.d), fmaxf(hi.p, v.p), fmaxf(hi.vx, v.vx), fmaxf(hi.vy, v.vy)};
+  lo = C4{fminf(lo.d, v.d), fminf(lo.p, v.p), fminf(lo.vx, v.vx), fminf(lo.vy, v.vy)};
+}
+
 // LinearGaussImproved::calc_slope (LinearGaussImproved.cpp:425-494) in FP32.
-template <bool kBatch, int kUnroll>
-__device__ __forceinline__ void k_slopes32_item(const MixedArgs& a, int i) {
-  const MeshDev& m = a.mesh;
-  const C4 cell = ld4(a.cells32, i);
-  const int b = m.cell_off[i], nn = m.cell_off[i + 1] - b;
+// en(k), word(k), state(k): stencil record, neighbour word and state of
+// neighbour k, again(k) the state a second time.
+template <bool kBatch, int kUnroll, class En, class Word, class State, class Again>
+__device__ __forceinline__ void slopes32_cell(const MixedArgs& a, int i, const C4& cell, int nn, const En& en,
+                                              const Word& word, const State& state, const Again& again) {
   const float4 mi = a.g32.minv[i];
   const bool boundary = a.geom.cflags[i] & kCellBoundarySlope;
-  // one pass over the neighbours: the gradient's sums, the neighbour
-  // max / min over all neighbours and over those that are not self-mirror
-  // ghosts (the unshocked limiter skips those, LinearGaussImproved.cpp:194-195)
-  // and the pressure-ratio shock test
+  // neighbours with LinearGaussImproved's skip_key sticker stay out of the
+  // extrema (:192-193, :314-315)
+  const bool skips = a.skip_mask != 0;
+  // boundary cells: least squares on differences (:401-422); others: the
+  // Green-Gauss sum of 0.5 r_ij (cell + neighbour) (:80-133)
+  const float sign = boundary ? -1.0f : 1.0f;
   C4 vx{0, 0, 0, 0}, vy{0, 0, 0, 0};
-  C4 amax = cell, amin = cell, nmax = cell, nmin = cell;
-  bool ratio_shock = false;
+  C4 amax = cell, amin = cell;
 #pragma unroll(kUnroll)
   for (int k = 0; k < nn; ++k) {
-    const uint32_t w = a.geom.nbr[b + k];
-    const C4 nb = point32(a, static_cast<int>(w & kNbrIdMask));
-    const float4 en = a.g32.ent[b + k];
-    // boundary cells: least squares on differences (:401-422); others: the
-    // Green-Gauss sum of 0.5 r_ij (cell + neighbour) (:80-133)
-    const C4 s = boundary ? C4{nb.d - cell.d, nb.p - cell.p, nb.vx - cell.vx, nb.vy - cell.vy}
-                          : C4{cell.d + nb.d, cell.p + nb.p, cell.vx + nb.vx, cell.vy + nb.vy};
-    addm(vx, s, en.x);
-    addm(vy, s, en.y);
-    // neighbours with LinearGaussImproved's skip_key sticker stay out of
-    // both extrema (:192-193, :314-315)
-    if (!skipped32(a, static_cast<int>(w & kNbrIdMask))) {
-      amax = C4{fmaxf(amax.d, nb.d), fmaxf(amax.p, nb.p), fmaxf(amax.vx, nb.vx), fmaxf(amax.vy, nb.vy)};
-      amin = C4{fminf(amin.d, nb.d), fminf(amin.p, nb.p), fminf(amin.vx, nb.vx), fminf(amin.vy, nb.vy)};
-      if (boundary && !(w & kNbrMirror)) {
-        nmax = C4{fmaxf(nmax.d, nb.d), fmaxf(nmax.p, nb.p), fmaxf(nmax.vx, nb.vx), fmaxf(nmax.vy, nb.vy)};
-        nmin = C4{fminf(nmin.d, nb.d), fminf(nmin.p, nb.p), fminf(nmin.vx, nb.vx), fminf(nmin.vy, nb.vy)};
-      }
-    }
-    // min(p, p_k) / max(p, p_k) < delta_p without the division
-    ratio_shock = ratio_shock || fminf(cell.p, nb.p) < a.delta_p * fmaxf(cell.p, nb.p);
-  }
-  if (!boundary) {
-    // a cell with a self-mirror neighbour takes the boundary slope: every
-    // other cell's neighbours count in both extrema
-    nmax = amax;
-    nmin = amin;
+    const C4 nb = state(k);
+    const float4 e = en(k);
+    const C4 s{fmaf(sign, cell.d, nb.d), fmaf(sign, cell.p, nb.p), fmaf(sign, cell.vx, nb.vx),
+               fmaf(sign, cell.vy, nb.vy)};
+    addm(vx, s, e.x);
+    addm(vy, s, e.y);
+    if (!skips || !skipped32(a, static_cast<int>(word(k) & kNbrIdMask))) widen_range(nb, amax, amin);
   }
   // boundary cells: vx, vy hold sum(df*dx), sum(df*dy)
   C4 sx, sy;
   naive_slope(boundary, vx, vy, mi, sx, sy);
   if (a.slf) {
     const float cs = sqrtf(gamma32<kBatch>(a, i) * cell.p / cell.d);
+    // some min(p, p_k) < delta_p * max(p, p_k) (without the division): of the
+    // neighbours above the cell the largest decides, of those below the smallest
+    bool ratio_shock = nn > 0 && (cell.p < a.delta_p * amax.p || amin.p < a.delta_p * cell.p);
+    if (skips || !(a.delta_p >= 0.0f) || !(cell.p >= 0.0f)) {
+      // extrema that leave neighbours out, or an order that does not carry over
+      ratio_shock = false;
+      for (int k = 0; k < nn; ++k) {
+        const float q = again(k).p;
+        ratio_shock = ratio_shock || fminf(cell.p, q) < a.delta_p * fmaxf(cell.p, q);
+      }
+    }
     const bool shock = (sx.vx + sy.vy) * a.g32.width[i] < (-a.delta_v) * cs || ratio_shock;
     if (a.shock) a.shock[i] = shock ? 1 : 0;  // read by the tracer slopes
-    const C4 cmax = shock ? amax : nmax, cmin = shock ? amin : nmin;
+    C4 cmax = amax, cmin = amin;
+    if (boundary && !shock) {
+      // the unshocked limiter's extrema leave out self-mirror ghosts too
+      // (:194-195); a cell without one takes no boundary slope
+      cmax = cmin = cell;
+      for (int k = 0; k < nn; ++k) {
+        const uint32_t w = word(k);
+        if (!(w & kNbrMirror) && !skipped32(a, static_cast<int>(w & kNbrIdMask))) widen_range(again(k), cmax, cmin);
+      }
+    }
     const C4 maxd{cmax.d - cell.d, cmax.p - cell.p, cmax.vx - cell.vx, cmax.vy - cell.vy};
     const C4 mind{cmin.d - cell.d, cmin.p - cell.p, cmin.vx - cell.vx, cmin.vy - cell.vy};
     const float f = shock ? 0.1f : 0.05f;
     const C4 thr{f * fmaxf(fabsf(maxd.d), fabsf(mind.d)), f * fmaxf(fabsf(maxd.p), fabsf(mind.p)),
                  f * fmaxf(fabsf(maxd.vx), fabsf(mind.vx)), f * fmaxf(fabsf(maxd.vy), fabsf(mind.vy))};
     float psi0 = 1, psi1 = 1, psi2 = 1, psi3 = 1;
+    if (!shock && cell.d >= 0.0f && cell.p >= 0.0f) {
+      C4 hi = cell, lo = cell;
 #pragma unroll(kUnroll)
-    for (int k = 0; k < nn; ++k) {
-      const float4 en = a.g32.ent[b + k];
-      C4 cv = cell;
-      addm(cv, sx, en.z);
-      addm(cv, sy, en.w);
-      const C4 dphi{cv.d - cell.d, cv.p - cell.p, cv.vx - cell.vx, cv.vy - cell.vy};
-      if (!shock) {
-        limit32(dphi.d, cv.d, cell.d, thr.d, maxd.d, mind.d, false, psi0);
-        limit32(dphi.p, cv.p, cell.p, thr.p, maxd.p, mind.p, false, psi1);
-        limit32(dphi.vx, cv.vx, cell.vx, thr.vx, maxd.vx, mind.vx, true, psi2);
-        limit32(dphi.vy, cv.vy, cell.vy, thr.vy, maxd.vy, mind.vy, true, psi3);
-      } else {
-        const int p = static_cast<int>(a.geom.nbr[b + k] & kNbrIdMask);
-        if (skipped32(a, p)) continue;  // :339-340
-        const C4 nb = point32(a, p);
-        shocked32(dphi.d, cv.d, cell.d, thr.d, nb.d, a.theta, psi0);
-        shocked32(dphi.p, cv.p, cell.p, thr.p, nb.p, a.theta, psi1);
-        shocked32(dphi.vx, cv.vx, cell.vx, thr.vx, nb.vx, a.theta, psi2);
-        shocked32(dphi.vy, cv.vy, cell.vy, thr.vy, nb.vy, a.theta, psi3);
+      for (int k = 0; k < nn; ++k) {
+        const float4 e = en(k);
+        C4 cv = cell;
+        addm(cv, sx, e.z);
+        addm(cv, sy, e.w);
+        widen_range(cv, hi, lo);
+      }
+      psi0 = limit32_range(hi.d, lo.d, cell.d, thr.d, maxd.d, mind.d, false);
+      psi1 = limit32_range(hi.p, lo.p, cell.p, thr.p, maxd.p, mind.p, false);
+      psi2 = limit32_range(hi.vx, lo.vx, cell.vx, thr.vx, maxd.vx, mind.vx, true);
+      psi3 = limit32_range(hi.vy, lo.vy, cell.vy, thr.vy, maxd.vy, mind.vy, true);
+    } else {
+      for (int k = 0; k < nn; ++k) {
+        const float4 e = en(k);
+        C4 cv = cell;
+        addm(cv, sx, e.z);
+        addm(cv, sy, e.w);
+        const C4 dphi{cv.d - cell.d, cv.p - cell.p, cv.vx - cell.vx, cv.vy - cell.vy};
+        if (!shock) {  // a negative (or NaN) density or pressure: face by face
+          limit32(dphi.d, cv.d, cell.d, thr.d, maxd.d, mind.d, false, psi0);
+          limit32(dphi.p, cv.p, cell.p, thr.p, maxd.p, mind.p, false, psi1);
+          limit32(dphi.vx, cv.vx, cell.vx, thr.vx, maxd.vx, mind.vx, true, psi2);
+          limit32(dphi.vy, cv.vy, cell.vy, thr.vy, maxd.vy, mind.vy, true, psi3);
+        } else {
+          if (skipped32(a, static_cast<int>(word(k) & kNbrIdMask))) continue;  // :339-340
+          const C4 nb = again(k);
+          shocked32(dphi.d, cv.d, cell.d, thr.d, nb.d, a.theta, psi0);
+          shocked32(dphi.p, cv.p, cell.p, thr.p, nb.p, a.theta, psi1);
+          shocked32(dphi.vx, cv.vx, cell.vx, thr.vx, nb.vx, a.theta, psi2);
+          shocked32(dphi.vy, cv.vy, cell.vy, thr.vy, nb.vy, a.theta, psi3);
+        }
       }
     }
     sx.d *= psi0; sy.d *= psi0;
@@ -616,23 +616,35 @@ __device__ __forceinline__ void k_slopes32_item(const MixedArgs& a, int i) {
   a.slopes32[2 * i + 1] = make_float4(sy.d, sy.p, sy.vx, sy.vy);
 }
 
+// One thread per cell.  Bound by memory latency: 24 warps per SM, half of
+// their time waiting for neighbour states, the DRAM 39 % busy.  The limiter
+// over the range of reconstructed values, the ratio test on the extrema, the
+// boundary cells' own extrema in a pass of their own and the sign of the
+// Green-Gauss sums as a factor took a third of the instructions out: 1024^2
+// 72 -> 62 us, 512^2 21.5 -> 20.6, 96 Riemann problems 70 -> 60.  Copying a
+// warp's CSR records to shared memory first did not help (61 us), nor did more
+// resident warps (48 registers 62, 40 registers 64: the states leave L1).
+template <bool kBatch, int kUnroll>
+__device__ __forceinline__ void k_slopes32_item(const MixedArgs& a, int i) {
+  const int b = a.mesh.cell_off[i], nn = a.mesh.cell_off[i + 1] - b;
+  const auto word = [&](int k) { return a.geom.nbr[b + k]; };
+  const auto state = [&](int k) { return point32(a, static_cast<int>(word(k) & kNbrIdMask)); };
+  slopes32_cell<kBatch, kUnroll>(a, i, ld4(a.cells32, i), nn, [&](int k) { return a.g32.ent[b + k]; }, word, state,
+                                 state);
+}
+
 // The same slope with the neighbour states and stencil records of cells
 // with at most kPrefetch neighbours loaded up front, all independent, so
-// their latencies overlap; the arithmetic runs over them in the order of
-// k_slopes32_item and gives the same bits.  Cells with more neighbours take
-// k_slopes32_item.
+// their latencies overlap; the same arithmetic in the same order.  Cells with
+// more neighbours take k_slopes32_item.
 constexpr int kPrefetch = 8;
 template <bool kBatch>
 __device__ __forceinline__ void k_slopes32_pf_item(const MixedArgs& a, int i) {
-  const MeshDev& m = a.mesh;
-  const int b = m.cell_off[i], nn = m.cell_off[i + 1] - b;
+  const int b = a.mesh.cell_off[i], nn = a.mesh.cell_off[i + 1] - b;
   if (nn > kPrefetch) {
     k_slopes32_item<kBatch, 1>(a, i);
     return;
   }
-  const C4 cell = ld4(a.cells32, i);
-  const float4 mi = a.g32.minv[i];
-  const bool boundary = a.geom.cflags[i] & kCellBoundarySlope;
   C4 nbk[kPrefetch];
   float4 enk[kPrefetch];
   uint32_t wk[kPrefetch];
@@ -646,76 +658,17 @@ __device__ __forceinline__ void k_slopes32_pf_item(const MixedArgs& a, int i) {
 #pragma unroll
   for (int k = 0; k < kPrefetch; ++k)
     if (k < nn) nbk[k] = point32(a, static_cast<int>(wk[k] & kNbrIdMask));
-  C4 vx{0, 0, 0, 0}, vy{0, 0, 0, 0};
-  C4 amax = cell, amin = cell, nmax = cell, nmin = cell;
-  bool ratio_shock = false;
+  // (the shared loops run over k: a select per record, not an index)
+  const auto pick = [](const auto& v, int k) {
+    auto r = v[0];
 #pragma unroll
-  for (int k = 0; k < kPrefetch; ++k) {
-    if (k >= nn) break;
-    const C4& nb = nbk[k];
-    const float4 en = enk[k];
-    const C4 s = boundary ? C4{nb.d - cell.d, nb.p - cell.p, nb.vx - cell.vx, nb.vy - cell.vy}
-                          : C4{cell.d + nb.d, cell.p + nb.p, cell.vx + nb.vx, cell.vy + nb.vy};
-    addm(vx, s, en.x);
-    addm(vy, s, en.y);
-    if (!skipped32(a, static_cast<int>(wk[k] & kNbrIdMask))) {
-      amax = C4{fmaxf(amax.d, nb.d), fmaxf(amax.p, nb.p), fmaxf(amax.vx, nb.vx), fmaxf(amax.vy, nb.vy)};
-      amin = C4{fminf(amin.d, nb.d), fminf(amin.p, nb.p), fminf(amin.vx, nb.vx), fminf(amin.vy, nb.vy)};
-      if (boundary && !(wk[k] & kNbrMirror)) {
-        nmax = C4{fmaxf(nmax.d, nb.d), fmaxf(nmax.p, nb.p), fmaxf(nmax.vx, nb.vx), fmaxf(nmax.vy, nb.vy)};
-        nmin = C4{fminf(nmin.d, nb.d), fminf(nmin.p, nb.p), fminf(nmin.vx, nb.vx), fminf(nmin.vy, nb.vy)};
-      }
-    }
-    ratio_shock = ratio_shock || fminf(cell.p, nb.p) < a.delta_p * fmaxf(cell.p, nb.p);
-  }
-  if (!boundary) {
-    // a cell with a self-mirror neighbour takes the boundary slope: every
-    // other cell's neighbours count in both extrema
-    nmax = amax;
-    nmin = amin;
-  }
-  C4 sx, sy;
-  naive_slope(boundary, vx, vy, mi, sx, sy);
-  if (a.slf) {
-    const float cs = sqrtf(gamma32<kBatch>(a, i) * cell.p / cell.d);
-    const bool shock = (sx.vx + sy.vy) * a.g32.width[i] < (-a.delta_v) * cs || ratio_shock;
-    if (a.shock) a.shock[i] = shock ? 1 : 0;  // read by the tracer slopes
-    const C4 cmax = shock ? amax : nmax, cmin = shock ? amin : nmin;
-    const C4 maxd{cmax.d - cell.d, cmax.p - cell.p, cmax.vx - cell.vx, cmax.vy - cell.vy};
-    const C4 mind{cmin.d - cell.d, cmin.p - cell.p, cmin.vx - cell.vx, cmin.vy - cell.vy};
-    const float f = shock ? 0.1f : 0.05f;
-    const C4 thr{f * fmaxf(fabsf(maxd.d), fabsf(mind.d)), f * fmaxf(fabsf(maxd.p), fabsf(mind.p)),
-                 f * fmaxf(fabsf(maxd.vx), fabsf(mind.vx)), f * fmaxf(fabsf(maxd.vy), fabsf(mind.vy))};
-    float psi0 = 1, psi1 = 1, psi2 = 1, psi3 = 1;
-#pragma unroll
-    for (int k = 0; k < kPrefetch; ++k) {
-      if (k >= nn) break;
-      const float4 en = enk[k];
-      C4 cv = cell;
-      addm(cv, sx, en.z);
-      addm(cv, sy, en.w);
-      const C4 dphi{cv.d - cell.d, cv.p - cell.p, cv.vx - cell.vx, cv.vy - cell.vy};
-      if (!shock) {
-        limit32(dphi.d, cv.d, cell.d, thr.d, maxd.d, mind.d, false, psi0);
-        limit32(dphi.p, cv.p, cell.p, thr.p, maxd.p, mind.p, false, psi1);
-        limit32(dphi.vx, cv.vx, cell.vx, thr.vx, maxd.vx, mind.vx, true, psi2);
-        limit32(dphi.vy, cv.vy, cell.vy, thr.vy, maxd.vy, mind.vy, true, psi3);
-      } else {
-        if (skipped32(a, static_cast<int>(wk[k] & kNbrIdMask))) continue;
-        const C4& nb = nbk[k];
-        shocked32(dphi.d, cv.d, cell.d, thr.d, nb.d, a.theta, psi0);
-        shocked32(dphi.p, cv.p, cell.p, thr.p, nb.p, a.theta, psi1);
-        shocked32(dphi.vx, cv.vx, cell.vx, thr.vx, nb.vx, a.theta, psi2);
-        shocked32(dphi.vy, cv.vy, cell.vy, thr.vy, nb.vy, a.theta, psi3);
-      }
-    }
-    sx.d *= psi0; sy.d *= psi0;
-    sx.p *= psi1; sy.p *= psi1;
-    sx.vx *= psi2; sy.vx *= psi2;
-    sx.vy *= psi3; sy.vy *= psi3;
-  }
-  a.slopes32[2 * i] = make_float4(sx.d, sx.p, sx.vx, sx.vy);
-  a.slopes32[2 * i + 1] = make_float4(sy.d, sy.p, sy.vx, sy.vy);
+    for (int j = 1; j < kPrefetch; ++j)
+      if (j == k) r = v[j];
+    return r;
+  };
+  slopes32_cell<kBatch, kPrefetch>(
+      a, i, ld4(a.cells32, i), nn, [&](int k) { return pick(enk, k); }, [&](int k) { return pick(wk, k); },
+      [&](int k) { return pick(nbk, k); }, [&](int k) { return point32(a, static_cast<int>(a.geom.nbr[b + k] & kNbrIdMask)); });
 }
 
 template <bool kBatch>
