@@ -664,10 +664,11 @@ rg_status rg_create(const rg_config* cfg, rg_handle** out) {
   h->shapes64.slopes = rg::LaunchShape{256, 0, 3};
   // the FP64 faces in blocks of 512 (k_faces)
   h->shapes64.faces = rg::LaunchShape{512, 0, 0};
-  // the FP32-mixed slopes in blocks of 128 (1024^2: 72 us, 76 us in blocks of
-  // 256), the update as the build for six resident blocks (1024^2: 68 us, 84 us
+  // the FP32-mixed slopes and faces in blocks of 128 (1024^2: slopes 62 us, 67 us
+  // in blocks of 256; faces 50.0 and 51.5 us), the update as the build for six resident blocks (1024^2: 68 us, 84 us
   // as the plain build)
   h->shapes32.slopes = rg::LaunchShape{128, 0, 0};
+  h->shapes32.faces = rg::LaunchShape{128, 0, 0};
   h->shapes32.update = rg::LaunchShape{256, 0, 3};
   h->heun = cfg->time_integrator == RG_TIME_ADVANCE_HEUN;
   auto fail = [&](cudaError_t e) {

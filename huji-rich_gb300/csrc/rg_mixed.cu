@@ -321,15 +321,16 @@ __device__ __forceinline__ float inv_gm1_32(const MixedArgs& a, int point) {
 }
 
 // Ghost state: RigidWallGenerator.cpp:5-15 reflection / PeriodicGhostGenerator copy.
-__device__ __forceinline__ float4 ghost_state32(const MixedArgs& a, int q) {
-  float4 c = a.cells32[a.geom.ghost_real[q]];
-  if (a.ghost_kind != RG_GHOST_PERIODIC) {
-    const float2 u = a.g32.ghost_unit[q];
-    const float s = 2.0f * (c.z * u.x + c.w * u.y);
-    c.z -= u.x * s;
-    c.w -= u.y * s;
-  }
+__device__ __forceinline__ float4 reflected32(const MixedArgs& a, int q, float4 c) {
+  const float2 u = a.g32.ghost_unit[q];
+  const float s = 2.0f * (c.z * u.x + c.w * u.y);
+  c.z -= u.x * s;
+  c.w -= u.y * s;
   return c;
+}
+__device__ __forceinline__ float4 ghost_state32(const MixedArgs& a, int q) {
+  const float4 c = a.cells32[a.geom.ghost_real[q]];
+  return a.ghost_kind != RG_GHOST_PERIODIC ? reflected32(a, q, c) : c;
 }
 // State of point p: a real cell's record, or a ghost's state formed from the
 // current state of its cell (the per-step kernels read no ghost records)
@@ -766,51 +767,81 @@ __device__ __forceinline__ void write32(const MixedArgs& a, int e, int real_side
   if (a.mflux) a.mflux[e] = static_cast<double>(c.m);
 }
 
-// LinearGaussImproved's face value of point pid at offset dm from its CM
-__device__ __forceinline__ C4 side32(const MixedArgs& a, int pid, float2 dm) {
+// The records of one side of a face: its point's state and slopes, loaded
+// without a branch on what the point is, so that both sides' loads and the
+// face's own are in flight together.
+struct Side32 {
+  bool ghost;  // a reflected ghost: the state still to be reflected, no slope
+  C4 c, gx, gy;
+};
+__device__ __forceinline__ Side32 load_side32(const MixedArgs& a, int pid) {
   const MeshDev& m = a.mesh;
-  C4 c = point32(a, pid);
-  int sid = pid;
-  bool zero = false;
+  int cell = pid, slope = pid;
+  bool ghost = false;
   if (pid >= m.n) {
+    cell = slope = a.geom.ghost_real[pid - m.n];
     if (a.ghost_kind == RG_GHOST_PERIODIC)
-      sid = m.ghost_source[pid - m.n];
+      slope = m.ghost_source[pid - m.n];
     else
-      zero = true;
+      ghost = true;
   }
-  if (!zero) {
-    const C4 gx = ld4(a.slopes32, 2 * sid), gy = ld4(a.slopes32, 2 * sid + 1);
-    addm(c, gx, dm.x);
-    addm(c, gy, dm.y);
+  return Side32{ghost, ld4(a.cells32, cell), ld4(a.slopes32, 2 * slope), ld4(a.slopes32, 2 * slope + 1)};
+}
+// LinearGaussImproved's face value of point pid at offset dm from its CM
+__device__ __forceinline__ C4 side32(const MixedArgs& a, int pid, const Side32& r, float2 dm) {
+  C4 c = r.c;
+  if (r.ghost) {
+    const float4 v = reflected32(a, pid - a.mesh.n, make_float4(c.d, c.p, c.vx, c.vy));
+    c = C4{v.x, v.y, v.z, v.w};
+  } else {
+    addm(c, r.gx, dm.x);
+    addm(c, r.gy, dm.y);
   }
   return c;
 }
 
+// A face's own records
+struct Face32 {
+  float2 w, n, p;
+  float na, pa, xa;
+};
+__device__ __forceinline__ Face32 load_face32(const MixedArgs& a, int e) {
+  return Face32{a.ev_zero ? make_float2(0.0f, 0.0f) : a.ev32[e], a.g32.nrm[e], a.g32.par[e],
+                a.g32.nabs[e], a.g32.area[e], a.g32.xarea[e]};
+}
+
 // Hllc on face e's two face values, scaled and written
 template <bool kScaled, bool kBatch>
-__device__ __forceinline__ void face32_solve(const MixedArgs& a, int e, int2 fc, const C4& s0, const C4& s1) {
+__device__ __forceinline__ void face32_solve(const MixedArgs& a, int e, int2 fc, const Face32& f, const C4& s0,
+                                             const C4& s1) {
   const MeshDev& m = a.mesh;
-  const float2 w = a.ev_zero ? make_float2(0.0f, 0.0f) : a.ev32[e];
-  const float2 n = a.g32.nrm[e], p = a.g32.par[e];
-  const float na = a.g32.nabs[e], pa = a.g32.area[e];
-  const float vel = (n.x * w.x + n.y * w.y) / na;
+  const float vel = (f.n.x * f.w.x + f.n.y * f.w.y) / f.na;
   const int real_side = fc.x < m.n ? fc.x : fc.y;
   const float g = gamma32<kBatch>(a, real_side), igm = inv_gm1_32<kBatch>(a, real_side);
   F4 c;
-  if (!solve32(prim32(g, igm, s0), prim32(g, igm, s1), vel, n, na, p, pa, c, a, e)) return;
-  write32<kBatch>(a, e, real_side, c, kScaled, a.g32.xarea[e]);
+  if (!solve32(prim32(g, igm, s0), prim32(g, igm, s1), vel, f.n, f.na, f.p, f.pa, c, a, e)) return;
+  write32<kBatch>(a, e, real_side, c, kScaled, f.xa);
 }
 
 template <bool kScaled, bool kBatch>
 __device__ __forceinline__ void k_faces32_lgi_item(const MixedArgs& a, int e) {
   const int2 fc = a.mesh.face_cells[e];
-  const C4 s0 = side32(a, fc.x, a.g32.dm0[e]);
-  const C4 s1 = side32(a, fc.y, a.g32.dm1[e]);
-  face32_solve<kScaled, kBatch>(a, e, fc, s0, s1);
+  const float2 dm0 = a.g32.dm0[e], dm1 = a.g32.dm1[e];
+  const Face32 f = load_face32(a, e);
+  const Side32 r0 = load_side32(a, fc.x), r1 = load_side32(a, fc.y);
+  asm volatile("" ::: "memory");  // every load above is issued before the first use
+  const C4 s0 = side32(a, fc.x, r0, dm0), s1 = side32(a, fc.y, r1, dm1);
+  face32_solve<kScaled, kBatch>(a, e, fc, f, s0, s1);
 }
 
+// Bound by memory: 56 bytes of geometry a face and the two sides' records.  All
+// of a face's loads are issued before the first use, in 48 registers (5
+// resident blocks of 256); with the sides' loads behind the branch on what a
+// point is, as the compiler placed them in 32 registers, they waited for one
+// another.  1024^2 (3.1 M faces, blocks of 128) 55.7 -> 50.0 us, 512^2 15.2 ->
+// 14.4; 52.6 us in 56 registers, 59.3 in 44 (spilt); blocks of 256 51.5 us.
 template <bool kScaled, bool kBatch>
-__global__ void __launch_bounds__(kMaxBlock) k_faces32_lgi(MixedArgs a) {
+__global__ void __maxnreg__(48) k_faces32_lgi(MixedArgs a) {
   chain_wait();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.mesh.e; e += gridDim.x * blockDim.x)
     k_faces32_lgi_item<kScaled, kBatch>(a, e);
@@ -829,13 +860,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_faces32_lgi_pair(MixedArgs a) {
   const int stride = (gridDim.x * blockDim.x) >> 1;
   for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 1; e < a.mesh.e; e += stride) {
     const int2 fc = a.mesh.face_cells[e];
-    const C4 mine = side32(a, s ? fc.y : fc.x, s ? a.g32.dm1[e] : a.g32.dm0[e]);
+    const int pid = s ? fc.y : fc.x;
+    const C4 mine = side32(a, pid, load_side32(a, pid), s ? a.g32.dm1[e] : a.g32.dm0[e]);
     C4 other;
     other.d = __shfl_xor_sync(pair, mine.d, 1);
     other.p = __shfl_xor_sync(pair, mine.p, 1);
     other.vx = __shfl_xor_sync(pair, mine.vx, 1);
     other.vy = __shfl_xor_sync(pair, mine.vy, 1);
-    if (s == 0) face32_solve<kScaled, kBatch>(a, e, fc, mine, other);
+    if (s == 0) face32_solve<kScaled, kBatch>(a, e, fc, load_face32(a, e), mine, other);
   }
 }
 
