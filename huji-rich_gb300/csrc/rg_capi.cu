@@ -665,11 +665,12 @@ rg_status rg_create(const rg_config* cfg, rg_handle** out) {
   // the FP64 faces in blocks of 512 (k_faces)
   h->shapes64.faces = rg::LaunchShape{512, 0, 0};
   // the FP32-mixed slopes and faces in blocks of 128 (1024^2: slopes 62 us, 67 us
-  // in blocks of 256; faces 50.0 and 51.5 us), the update as the build for six resident blocks (1024^2: 68 us, 84 us
-  // as the plain build)
+  // in blocks of 256; faces 50.0 and 51.5 us), the update too, as the build for
+  // six resident blocks of 256 (1024^2: 54 us, 56 us in blocks of 256, 69 us as
+  // the plain build)
   h->shapes32.slopes = rg::LaunchShape{128, 0, 0};
   h->shapes32.faces = rg::LaunchShape{128, 0, 0};
-  h->shapes32.update = rg::LaunchShape{256, 0, 3};
+  h->shapes32.update = rg::LaunchShape{128, 0, 3};
   h->heun = cfg->time_integrator == RG_TIME_ADVANCE_HEUN;
   auto fail = [&](cudaError_t e) {
     rg_destroy(h);
