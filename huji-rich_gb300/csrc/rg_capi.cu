@@ -321,10 +321,14 @@ rg_status mesh_error(rg_handle* h) {
 
 namespace {
 
-// Fused steps (the update computes the next step's dt): one problem, no caller
-// access to the device buffers.  The dt is moved into place by the slopes
-// kernel, or by the face kernel at first order.
-bool fusable(const rg_handle* h) { return h->n_problems == 0 && !h->external_state; }
+// Fused steps (the update computes the next step's dt): no caller access to
+// the device buffers.  The dt is moved into place by the slopes kernel, or for
+// one problem at first order by the face kernel.  A batch is fused on the
+// FP32-mixed path (a CFL pass of its own took 18 us of a step's 185, 96 Riemann
+// problems; in the update 7); the FP64 update screens one minimum, not many.
+bool fusable(const rg_handle* h) {
+  return !h->external_state && (h->n_problems == 0 || (h->mixed && h->cfg.order == 2 && !h->heun));
+}
 
 // hdsim::TimeAdvance2Heun on a fixed mesh (hdsim2d.cpp:323-449): dt once;
 // pass 1 on the cells writes the mid extensives and mid cells; pass 2 on the
@@ -426,6 +430,7 @@ rg_status enqueue_step(rg_handle* h, int step, cudaEvent_t* ev = nullptr) {
     a.dt32_from_device = 1;
     a.step = step;
     const bool fuse = fusable(h), have_dt = fuse && h->dt_next_ready;
+    if (fuse && h->n_problems > 0) a.dtnext_p = a.dtmin_p + h->n_problems;
     // tracers: the FP64 tracer passes after each FP32 hydro pass, reading
     // its shock decisions and mass fluxes (the dt from the device)
     const bool tr = h->tcfg.n_tracers > 0;
@@ -1311,7 +1316,7 @@ rg_status rg_set_problems(rg_handle* h, int32_t P, const int32_t* offsets, const
   RG_CUDA(h, h->gamma_p.ensure(8 * static_cast<size_t>(P)));
   RG_CUDA(h, h->gamma32_p.ensure(4 * static_cast<size_t>(P)));
   RG_CUDA(h, h->inv_gm1_32_p.ensure(4 * static_cast<size_t>(P)));
-  RG_CUDA(h, h->dtmin_p.ensure(8 * static_cast<size_t>(P)));
+  RG_CUDA(h, h->dtmin_p.ensure(16 * static_cast<size_t>(P)));  // this step's and the next one's
   RG_CUDA(h, h->time_p.ensure(8 * static_cast<size_t>(P)));
   RG_CUDA(h, h->dt_p.ensure(8 * static_cast<size_t>(P)));
   std::vector<float> g32(static_cast<size_t>(P)), igm(static_cast<size_t>(P));

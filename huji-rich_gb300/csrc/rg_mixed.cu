@@ -367,9 +367,19 @@ __device__ __forceinline__ float cfl32_cell(const MixedArgs& a, int t) {
   return 1.0f / res;
 }
 
-// The step's dt, computed by the previous step's update, into place (one
-// thread): what the kernels after this one read, and the run's record of it
+// The step's dt, computed by the previous step's update, into place: what the
+// kernels after this one read, and the run's record of it
+template <bool kBatch>
 __device__ __forceinline__ void take_next_dt32(const MixedArgs& a) {
+  if (kBatch) {
+    // each problem's minimum into place, the next step's record emptied
+    if (!a.dtnext_p) return;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n_problems; p += gridDim.x * blockDim.x) {
+      if (a.take_next_dt) a.dtmin_p[p] = a.dtnext_p[p];
+      a.dtnext_p[p] = kInfBits;
+    }
+    return;
+  }
   if (a.take_next_dt && blockIdx.x == 0 && threadIdx.x == 0) {
     const double dt = a.status->dt_next;
     a.status->dt = dt;
@@ -675,7 +685,7 @@ __device__ __forceinline__ void k_slopes32_pf_item(const MixedArgs& a, int i) {
 template <bool kBatch>
 __global__ void __launch_bounds__(kMaxBlock) k_slopes32_pf(MixedArgs a) {
   chain_wait();
-  take_next_dt32(a);
+  take_next_dt32<kBatch>(a);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.mesh.n; i += gridDim.x * blockDim.x)
     k_slopes32_pf_item<kBatch>(a, i);
 }
@@ -684,7 +694,7 @@ template <bool kBatch, int kMinBlocks, int kUnroll>
 __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 1)
     k_slopes32(MixedArgs a) {
   chain_wait();
-  take_next_dt32(a);
+  take_next_dt32<kBatch>(a);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.mesh.n; i += gridDim.x * blockDim.x)
     k_slopes32_item<kBatch, kUnroll>(a, i);
 }
@@ -917,7 +927,7 @@ __device__ __forceinline__ void k_faces32_pcm_item(const MixedArgs& a, int e) {
 template <bool kScaled, bool kBatch>
 __global__ void __launch_bounds__(kMaxBlock) k_faces32_pcm(MixedArgs a) {
   chain_wait();
-  take_next_dt32(a);
+  take_next_dt32<kBatch>(a);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.mesh.e; e += gridDim.x * blockDim.x)
     k_faces32_pcm_item<kScaled, kBatch>(a, e);
 }
@@ -1088,6 +1098,16 @@ __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlo
       a.dtmin_p[p] = kInfBits;
       if (p == 0 && a.dt_trace) *a.dt_trace = dt;
     }
+  }
+  if (kBatch && a.cfl_next) {
+    // (whole warps stay in the loop: problem_min's shuffles)
+    for (int base = t0 - (threadIdx.x & 31); base < a.mesh.n; base += stride) {
+      const int i = base + (threadIdx.x & 31);
+      const bool in = i < a.mesh.n;
+      const unsigned long long b = in ? k_update_mixed_item<kBatch, kMode>(a, i) : kInfBits;
+      problem_min(a.dtnext_p, in ? a.cell_problem[i] : -1, b);
+    }
+    return;
   }
   unsigned long long bits = kInfBits;
   for (int i = t0; i < a.mesh.n; i += stride) {

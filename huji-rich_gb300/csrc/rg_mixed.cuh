@@ -85,7 +85,10 @@ struct MixedArgs {
   const int* cell_problem;
   const float* gamma_p;     // per problem
   const float* inv_gm1_p;   // per problem 1/(gamma-1)
-  unsigned long long* dtmin_p;
+  unsigned long long* dtmin_p;  // the step's CFL minima
+  // fused steps (nullptr: not): the next step's minima, which the update forms
+  // (cfl_next) and the next step's slopes kernel moves to dtmin_p (take_next_dt)
+  unsigned long long* dtnext_p;
   double* time_p;
   double* dt_p;
   int n_problems;
