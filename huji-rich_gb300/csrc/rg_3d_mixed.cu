@@ -113,7 +113,10 @@ __global__ void __launch_bounds__(kBlock) k3m_flux_to64(const float4* f32, const
 
 // cell i's CFL bound, as the bit pattern of its FP64 value
 __device__ __forceinline__ unsigned long long cfl3m_bits(const Mixed3Args& a, int i, const C3& c) {
-  const float b = a.width32[i] / (fabs3(c.v) + sqrtf(a.gamma * c.p / c.d));
+  // |v| written out: in the update and in the pass of its own the compiler
+  // contracts other pairs of the sum's products
+  const float speed = sqrtf(fmaf(c.v.z, c.v.z, fmaf(c.v.x, c.v.x, __fmul_rn(c.v.y, c.v.y))));
+  const float b = a.width32[i] / (speed + sqrtf(a.gamma * c.p / c.d));
   return static_cast<unsigned long long>(__double_as_longlong(widen_exact(b)));
 }
 
