@@ -149,8 +149,7 @@ namespace rgh {
 
 rg_status reset_status(rg_handle* h, DevStatus* st, cudaStream_t s) {
   // error part only: err_key = ~0, err_status = lock = 0
-  RG_CUDA(h, cudaMemsetAsync(&st->err_key, 0xff, sizeof(unsigned long long), s));
-  RG_CUDA(h, cudaMemsetAsync(&st->err_status, 0, 2 * sizeof(int), s));
+  RG_CUDA(h, rg::launch_reset_status(st, 1, s));
   return RG_OK;
 }
 
@@ -686,7 +685,10 @@ rg_status rg_create(const rg_config* cfg, rg_handle** out) {
   if ((e = cudaSetDevice(cfg->device)) != cudaSuccess) return fail(e);
   if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
   if ((e = cudaStreamCreateWithFlags(&h->upload_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
+  if ((e = cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
   if ((e = cudaEventCreateWithFlags(&h->ev_uploaded, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
+  for (cudaEvent_t* ev : {&h->ev_topology, &h->ev_places, &h->ev_motion, &h->ev_pv})
+    if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
   if ((e = cudaStreamCreateWithFlags(&h->download_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
   if ((e = cudaEventCreateWithFlags(&h->ev_state, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
   if ((e = cudaEventCreateWithFlags(&h->ev_downloaded, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
@@ -712,6 +714,7 @@ rg_status rg_destroy(rg_handle* h) {
   if (!h) return RG_OK;
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->upload_stream) cudaStreamSynchronize(h->upload_stream);
+  if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
   if (h->download_stream) cudaStreamSynchronize(h->download_stream);
   for (auto& s : h->slots) {
     s.buf.release();
@@ -749,10 +752,13 @@ rg_status rg_destroy(rg_handle* h) {
   for (auto& k : h->ev_k)
     if (k) cudaEventDestroy(k);
   if (h->ev_uploaded) cudaEventDestroy(h->ev_uploaded);
+  for (cudaEvent_t ev : {h->ev_topology, h->ev_places, h->ev_motion, h->ev_pv})
+    if (ev) cudaEventDestroy(ev);
   if (h->ev_state) cudaEventDestroy(h->ev_state);
   if (h->ev_downloaded) cudaEventDestroy(h->ev_downloaded);
   if (h->stream) cudaStreamDestroy(h->stream);
   if (h->upload_stream) cudaStreamDestroy(h->upload_stream);
+  if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
   if (h->download_stream) cudaStreamDestroy(h->download_stream);
   cudaGetLastError();
   delete h;
@@ -781,6 +787,7 @@ rg_status rg_upload_mesh(rg_handle* h, const rg_mesh_view* v, uint32_t flags) {
   RG_CUDA(h, cudaStreamWaitEvent(h->upload_stream, s.last_use, 0));
   s.lay.compute(n, g, e, m, h->mixed, h->pgeo.kind == RG_GEOMETRY_CYLINDRICAL);
   RG_CUDA(h, cudaStreamSynchronize(h->upload_stream));
+  RG_CUDA(h, cudaStreamSynchronize(h->copy_stream));  // (idle, but after an upload that failed half-way)
   RG_CUDA(h, s.buf.ensure(s.lay.total));
   RG_CUDA(h, h->staging.ensure(s.lay.input_end));
   s.n = n;
@@ -796,39 +803,47 @@ rg_status rg_upload_mesh(rg_handle* h, const rg_mesh_view* v, uint32_t flags) {
     size_t off;
     const void* src;
     size_t bytes;
-  } parts[10] = {{s.lay.points, v->point_xy, 16 * np},
-                 {s.lay.cms, v->cm_xy, 16 * np},
-                 {s.lay.volume, v->volume, 8 * static_cast<size_t>(n)},
-                 {s.lay.cd_volume, v->cd_volume, 8 * static_cast<size_t>(n)},
-                 {s.lay.ghost_source, v->ghost_source, 4 * static_cast<size_t>(g)},
-                 {s.lay.ghost_face, v->ghost_face, 4 * static_cast<size_t>(g)},
-                 {s.lay.face_cells, v->face_cells, 8 * static_cast<size_t>(e)},
-                 {s.lay.face_vertices, v->face_vertices, 32 * static_cast<size_t>(e)},
-                 {s.lay.cell_off, v->cell_face_offset, 4 * (static_cast<size_t>(n) + 1)},
-                 {s.lay.cell_faces, v->cell_faces, 4 * static_cast<size_t>(m)}};
-  for (const Part& p : parts) {
-    if (p.bytes == 0 || p.src == nullptr) continue;  // device geometry: computed below
-    if (is_pinned(p.src)) {
-      RG_CUDA(h, cudaMemcpyAsync(static_cast<char*>(s.buf.p) + p.off, p.src, p.bytes, cudaMemcpyHostToDevice,
-                                 h->upload_stream));
-    } else {
-      par_memcpy(st + p.off, p.src, p.bytes);
-      RG_CUDA(h, cudaMemcpyAsync(static_cast<char*>(s.buf.p) + p.off, st + p.off, p.bytes, cudaMemcpyHostToDevice,
-                                 h->upload_stream));
+  };
+  const Part topology[] = {{s.lay.face_cells, v->face_cells, 8 * static_cast<size_t>(e)},
+                           {s.lay.cell_faces, v->cell_faces, 4 * static_cast<size_t>(m)},
+                           {s.lay.cell_off, v->cell_face_offset, 4 * (static_cast<size_t>(n) + 1)},
+                           {s.lay.ghost_source, v->ghost_source, 4 * static_cast<size_t>(g)},
+                           {s.lay.ghost_face, v->ghost_face, 4 * static_cast<size_t>(g)}};
+  const Part places[] = {{s.lay.points, v->point_xy, 16 * np},
+                         {s.lay.face_vertices, v->face_vertices, 32 * static_cast<size_t>(e)},
+                         {s.lay.cms, v->cm_xy, 16 * np},
+                         {s.lay.volume, v->volume, 8 * static_cast<size_t>(n)},
+                         {s.lay.cd_volume, v->cd_volume, 8 * static_cast<size_t>(n)}};
+  auto copy = [&](const Part& p, cudaStream_t to) -> rg_status {
+    if (p.bytes == 0 || p.src == nullptr) return RG_OK;  // device geometry: computed below
+    const void* from = p.src;
+    if (!is_pinned(from)) {
+      par_memcpy(st + p.off, from, p.bytes);
+      from = st + p.off;
     }
-  }
+    RG_CUDA(h, cudaMemcpyAsync(static_cast<char*>(s.buf.p) + p.off, from, p.bytes, cudaMemcpyHostToDevice, to));
+    return RG_OK;
+  };
+  // The topology goes first; while the coordinates follow on a stream of their
+  // own, the upload stream checks and orders the cells (512^2: 24 of a
+  // moving-mesh upload's 430 us).
+  for (const Part& p : topology) RG_TRY(copy(p, h->upload_stream));
+  RG_CUDA(h, cudaEventRecord(h->ev_topology, h->upload_stream));
+  RG_CUDA(h, cudaStreamWaitEvent(h->copy_stream, h->ev_topology, 0));
   // every index is checked before any kernel uses it: the validation runs
   // first on the upload stream and the geometry kernels behind it return at
   // once when it has failed, so the host reads both results after one wait
-  RG_TRY(reset_status(h, h->d_valid_status, h->upload_stream));
+  RG_CUDA(h, rg::launch_reset_status(h->d_geom_status, 2, h->upload_stream));  // and the validation's, beside it
   RG_CUDA(h, rg::launch_validate(s.mesh, h->d_valid_status, h->upload_stream));
   rg::MeshDev gm = s.mesh;
   gm.invalid = &h->d_valid_status->err_key;
   // geometry pass on the upload stream (the per-cell kernels take cells in
   // the per-tile neighbour-count order, computed first)
-  RG_TRY(reset_status(h, h->d_geom_status, h->upload_stream));
   RG_CUDA(h, rg::launch_cell_order(gm, at<int>(s.buf.p, s.lay.cell_order), at<int>(s.buf.p, s.lay.cflags),
                                    h->upload_stream));
+  for (const Part& p : places) RG_TRY(copy(p, h->copy_stream));
+  RG_CUDA(h, cudaEventRecord(h->ev_places, h->copy_stream));
+  RG_CUDA(h, cudaStreamWaitEvent(h->upload_stream, h->ev_places, 0));
   if (device_geometry)
     RG_CUDA(h, rg::launch_device_geometry(gm, at<int>(s.buf.p, s.lay.cell_order), at<double2>(s.buf.p, s.lay.cms), at<double>(s.buf.p, s.lay.volume),
                                           at<double>(s.buf.p, s.lay.cd_volume), h->cfg.ghost_kind, h->box,

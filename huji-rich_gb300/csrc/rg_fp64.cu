@@ -35,6 +35,7 @@ constexpr int kBlock = 256;
 // simple_flux_calculator.cpp:91-93 (order 1) or modular_flux_calculator.cpp:12-22
 // with simple_flux_calculator.cpp:27-31 (order 2).
 __global__ void __launch_bounds__(kBlock) k_geom_faces(GeomArgs a) {
+  chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.mesh.e || mesh_rejected(a.mesh)) return;
   const int2 fc = a.mesh.face_cells[e];
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(kBlock) k_geom_faces(GeomArgs a) {
 // state-independent half of calc_naive_slope (LinearGaussImproved.cpp:67-126:
 // matrix, determinant check, inverse, 0.5*r_ij) or of GetBoundarySlope (:401-417).
 __global__ void __launch_bounds__(kBlock) k_geom_cells(GeomArgs a) {
+  chain_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (t >= m.n || mesh_rejected(m)) return;
@@ -158,6 +160,7 @@ __global__ void __launch_bounds__(kBlock) k_geom_cells(GeomArgs a) {
 // Per ghost: which cell it copies and, for rigid walls, the unit normal of
 // RigidWallGenerator.cpp:5-15 (ghost minus real point, divided by its length).
 __global__ void __launch_bounds__(kBlock) k_geom_ghosts(GeomArgs a) {
+  chain_wait();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = a.mesh;
   if (g >= m.g || mesh_rejected(m)) return;
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(kBlock) k_geom_ghosts(GeomArgs a) {
 // taken from the topology and stored as the cell's flag for the per-cell
 // geometry pass; runs after the index validation.
 __global__ void __launch_bounds__(kOrderTile) k_cell_order(MeshDev m, int* order, int* cflags) {
+  chain_wait();
   constexpr int kKeys = 128, kWarps = kOrderTile / 32;
   // count[w][k]: cells of warp w with key k, then their offset within key k
   __shared__ int count[kWarps][kKeys];
@@ -245,6 +249,7 @@ __global__ void __launch_bounds__(kOrderTile) k_cell_order(MeshDev m, int* order
 // (smallest key: faces, then ghosts, then cells) is recorded.  Phase 0 keys:
 // index = array position, value = the offending entry.
 __global__ void __launch_bounds__(kBlock) k_validate(MeshDev m, DevStatus* st) {
+  chain_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int np = m.n + m.g;
   if (t < m.e) {
@@ -1064,6 +1069,17 @@ __global__ void __launch_bounds__(kBlock) k_init_ext(StepArgs a) {
 }
 
 // *flag = 1 if any of v[0..n) is not +-0 (NaN counts as nonzero)
+// The error part of `count` status blocks, emptied: one launch (about 1 us
+// in a chain of kernels), where the two memsets of a block took 5 us.
+__global__ void k_reset_status(DevStatus* st, int count) {
+  chain_wait();
+  if (static_cast<int>(threadIdx.x) < count) {
+    st[threadIdx.x].err_key = ~0ull;
+    st[threadIdx.x].err_status = 0;
+    st[threadIdx.x].lock = 0;
+  }
+}
+
 __global__ void __launch_bounds__(kBlock) k_any_nonzero(const double* v, long long n, int* flag) {
   bool any = false;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
@@ -1125,27 +1141,32 @@ cudaError_t launch_any_nonzero(const double* v, long long n, int* flag, cudaStre
   return cudaGetLastError();
 }
 
+cudaError_t launch_reset_status(DevStatus* st, int count, cudaStream_t s) {
+  chain(s, 1, 32, k_reset_status, st, count);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_validate(const MeshDev& m, DevStatus* st, cudaStream_t s) {
   int work = m.e > m.n ? m.e : m.n;
   work = work > m.g ? work : m.g;
-  k_validate<<<blocks(work > 0 ? work : 1), kBlock, 0, s>>>(m, st);
+  chain(s, blocks(work > 0 ? work : 1), kBlock, k_validate, m, st);
   return cudaGetLastError();
 }
 
 cudaError_t launch_cell_order(const MeshDev& m, int* order, int* cflags, cudaStream_t s) {
-  if (m.n > 0) k_cell_order<<<(m.n + kOrderTile - 1) / kOrderTile, kOrderTile, 0, s>>>(m, order, cflags);
+  if (m.n > 0) chain(s, (m.n + kOrderTile - 1) / kOrderTile, kOrderTile, k_cell_order, m, order, cflags);
   return cudaGetLastError();
 }
 
 cudaError_t launch_geometry(const GeomArgs& a, cudaStream_t s) {
-  if (a.mesh.e > 0) k_geom_faces<<<blocks(a.mesh.e), kBlock, 0, s>>>(a);
-  if (a.mesh.n > 0) k_geom_cells<<<blocks(a.mesh.n), kBlock, 0, s>>>(a);
-  if (a.mesh.g > 0) k_geom_ghosts<<<blocks(a.mesh.g), kBlock, 0, s>>>(a);
+  if (a.mesh.e > 0) chain(s, blocks(a.mesh.e), kBlock, k_geom_faces, a);
+  if (a.mesh.n > 0) chain(s, blocks(a.mesh.n), kBlock, k_geom_cells, a);
+  if (a.mesh.g > 0) chain(s, blocks(a.mesh.g), kBlock, k_geom_ghosts, a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_geom_ghosts(const GeomArgs& a, cudaStream_t s) {
-  if (a.mesh.g > 0) k_geom_ghosts<<<blocks(a.mesh.g), kBlock, 0, s>>>(a);
+  if (a.mesh.g > 0) chain(s, blocks(a.mesh.g), kBlock, k_geom_ghosts, a);
   return cudaGetLastError();
 }
 

@@ -152,11 +152,18 @@ struct rg_handle {
   rg_config cfg{};
   cudaStream_t stream = nullptr;
   cudaStream_t upload_stream = nullptr;
+  // rg_upload_mesh: the coordinates on copy_stream, after the topology's copies
+  // (ev_topology) and before the geometry kernels (ev_places)
+  cudaStream_t copy_stream = nullptr;
+  cudaEvent_t ev_topology = nullptr, ev_places = nullptr;
   cudaEvent_t ev_uploaded = nullptr;  // the upload stream's work for the newest mesh slot
   // rg_get_state_async: its copies run on download_stream after ev_state
   // (recorded on stream); stream waits for ev_downloaded before later work
   cudaStream_t download_stream = nullptr;
   cudaEvent_t ev_state = nullptr, ev_downloaded = nullptr;
+  // rg_advance_begin: the point velocities, formed by ev_motion, go back on
+  // download_stream while the fluxes are formed; stream waits for ev_pv
+  cudaEvent_t ev_motion = nullptr, ev_pv = nullptr;
   bool state_pending = false;
   cudaEvent_t ev_k[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   rgh::MeshSlot slots[2];

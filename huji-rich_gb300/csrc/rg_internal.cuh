@@ -402,6 +402,7 @@ struct GeomArgs {
 };
 
 cudaError_t launch_any_nonzero(const double* v, long long n, int* flag, cudaStream_t s);
+cudaError_t launch_reset_status(DevStatus* st, int count, cudaStream_t s);  // the error parts, emptied
 cudaError_t launch_validate(const MeshDev& m, DevStatus* st, cudaStream_t s);
 cudaError_t launch_problems(const MeshDev& m, const int* offsets, int P, int* cell_problem, DevStatus* st,
                             cudaStream_t s);

@@ -76,6 +76,7 @@ __device__ __forceinline__ void naive_slope(bool boundary, const C4& vx, const C
 // (the roundings on the integer pipe: rg_convert.cuh)
 
 __global__ void __launch_bounds__(kBlock) k_geom32(MixedGeomArgs a) {
+  chain_wait();
   if (a.invalid && *a.invalid != ~0ull) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int stride = gridDim.x * blockDim.x;
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kBlock) k_geom32(MixedGeomArgs a) {
 // as the FP32 reconstruction uses it.  The FP64 pass costs GB300's FP64 pipe
 // (2 operations per clock per SM) for quantities that were only rounded.
 __global__ void __launch_bounds__(kBlock) k_geom_faces32(GeomArgs ga, MixedGeomArgs a) {
+  chain_wait();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = ga.mesh;
   if (e >= m.e || mesh_rejected(m)) return;
@@ -171,6 +173,7 @@ __global__ void __launch_bounds__(kBlock) k_geom_faces32(GeomArgs ga, MixedGeomA
 // sums, or the naive slope's matrix and its inverse), re-reading the face
 // records from cache.
 __global__ void __launch_bounds__(kBlock) k_geom_cells32(GeomArgs ga, MixedGeomArgs a) {
+  chain_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshDev& m = ga.mesh;
   if (mesh_rejected(m)) return;
@@ -1177,14 +1180,14 @@ inline int blocks(int n) { return (n + kBlock - 1) / kBlock; }
 cudaError_t launch_geom32(const MixedGeomArgs& a, cudaStream_t s) {
   const int work = a.e > a.m ? (a.e > a.n ? a.e : a.n) : (a.m > a.n ? a.m : a.n);
   const int nb = blocks(work > 0 ? work : 1);
-  k_geom32<<<nb < 4096 ? nb : 4096, kBlock, 0, s>>>(a);
+  chain(s, nb < 4096 ? nb : 4096, kBlock, k_geom32, a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_geom32_direct(const GeomArgs& ga, const MixedGeomArgs& a, cudaStream_t s) {
-  if (a.e > 0) k_geom_faces32<<<blocks(a.e), kBlock, 0, s>>>(ga, a);
+  if (a.e > 0) chain(s, blocks(a.e), kBlock, k_geom_faces32, ga, a);
   const int work = a.n > a.g ? a.n : a.g;
-  if (work > 0) k_geom_cells32<<<blocks(work), kBlock, 0, s>>>(ga, a);
+  if (work > 0) chain(s, blocks(work), kBlock, k_geom_cells32, ga, a);
   return cudaGetLastError();
 }
 

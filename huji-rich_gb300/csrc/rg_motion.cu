@@ -56,6 +56,7 @@ __device__ __forceinline__ double half_cross(double2 p1, double2 p2) {
 // products run on the integer pipes.  512^2 (1.57 M faces of cells) 80.5 -> 65 us.
 __global__ void __launch_bounds__(kMoBlock) k_dev_geometry(MeshDev m, const int* order, double2* cms,
                                                             double* volume, double* cd_volume) {
+  chain_wait();
   const int th = blockIdx.x * blockDim.x + threadIdx.x;
   if (th >= m.n || mesh_rejected(m)) return;
   const int i = order ? order[th] : th;
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(kMoBlock) k_dev_geometry(MeshDev m, const int*
 }
 
 __global__ void __launch_bounds__(kMoBlock) k_ghost_cms(MeshDev m, double2* cms, int ghost_kind, dbl4 box) {
+  chain_wait();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= m.g || mesh_rejected(m)) return;
   const int p = m.n + g, src = m.ghost_source[g];
@@ -135,6 +137,7 @@ __device__ __forceinline__ double cone_segment(double2 p1, double2 p2, const Cyl
 
 __global__ void __launch_bounds__(kMoBlock) k_cyl_geometry(MeshDev m, double* xarea, double* cd_volume, dbl4 od,
                                                             int unit) {
+  chain_wait();
   if (mesh_rejected(m)) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const CylAxis a = cyl_axis(od, unit != 0);
@@ -306,8 +309,9 @@ inline int mo_blocks(int n) { return (n + kMoBlock - 1) / kMoBlock; }
 
 cudaError_t launch_device_geometry(const MeshDev& m, const int* order, double2* cms, double* volume,
                                    double* cd_volume, int ghost_kind, const double* box, cudaStream_t s) {
-  if (m.n > 0) k_dev_geometry<<<mo_blocks(m.n), kMoBlock, 0, s>>>(m, order, cms, volume, cd_volume);
-  if (m.g > 0) k_ghost_cms<<<mo_blocks(m.g), kMoBlock, 0, s>>>(m, cms, ghost_kind, make_dbl4(box[0], box[1], box[2], box[3]));
+  if (m.n > 0) chain(s, mo_blocks(m.n), kMoBlock, k_dev_geometry, m, order, cms, volume, cd_volume);
+  if (m.g > 0) 
+    chain(s, mo_blocks(m.g), kMoBlock, k_ghost_cms, m, cms, ghost_kind, make_dbl4(box[0], box[1], box[2], box[3]));
   return cudaGetLastError();
 }
 
@@ -315,8 +319,8 @@ cudaError_t launch_cyl_geometry(const MeshDev& m, double* xarea, double* cd_volu
                                 const double* direction, bool unit, cudaStream_t s) {
   const int work = m.e > m.n ? m.e : m.n;
   if (work > 0)
-    k_cyl_geometry<<<mo_blocks(work), kMoBlock, 0, s>>>(
-        m, xarea, cd_volume, make_dbl4(origin[0], origin[1], direction[0], direction[1]), unit ? 1 : 0);
+    chain(s, mo_blocks(work), kMoBlock, k_cyl_geometry, m, xarea, cd_volume,
+          make_dbl4(origin[0], origin[1], direction[0], direction[1]), unit ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -61,10 +61,10 @@ rg_status edges_from_points(rg_handle* h, const rg::StepArgs& a, const rg::Motio
   return RG_OK;
 }
 
-rg_status download_pv(rg_handle* h, double* out) {
+rg_status download_pv(rg_handle* h, double* out, cudaStream_t stream) {
   if (!out) return RG_OK;
   RG_CUDA(h, cudaMemcpyAsync(out, h->pv.p, 16 * static_cast<size_t>(active_slot(h)->n), cudaMemcpyDeviceToHost,
-                             h->stream));
+                             stream));
   return RG_OK;
 }
 
@@ -107,7 +107,7 @@ rg_status rg_point_velocities(rg_handle* h, double* pv_out) {
   const rg::MotionArgs mo = motion_args(h);
   RG_CUDA(h, rg::launch_point_velocities(a, mo, h->stream));
   RG_TRY(edges_from_points(h, a, mo));
-  RG_TRY(download_pv(h, pv_out));
+  RG_TRY(download_pv(h, pv_out, h->stream));
   RG_CUDA(h, cudaStreamSynchronize(h->stream));
   return RG_OK;
 }
@@ -121,7 +121,7 @@ rg_status rg_apply_fix(rg_handle* h, double dt, double* pv_out) {
   const rg::MotionArgs mo = motion_args(h);
   RG_CUDA(h, rg::launch_apply_fix(a, mo, h->stream));
   RG_TRY(edges_from_points(h, a, mo));
-  RG_TRY(download_pv(h, pv_out));
+  RG_TRY(download_pv(h, pv_out, h->stream));
   RG_CUDA(h, cudaStreamSynchronize(h->stream));
   return RG_OK;
 }
@@ -193,6 +193,7 @@ rg_status rg_advance_begin(rg_handle* h, double* dt_out, double* pv_out) {
     RG_CUDA(h, rg::launch_apply_fix(a1, mo, h->stream));
     RG_TRY(edges_from_points(h, a1, mo));
   }
+  if (pv_out) RG_CUDA(h, cudaEventRecord(h->ev_motion, h->stream));
   // fluxes (dt*area scaled) and the extensive update
   if (h->mixed) {
     rg::MixedArgs m = mixed_args(h);
@@ -223,7 +224,14 @@ rg_status rg_advance_begin(rg_handle* h, double* dt_out, double* pv_out) {
     RG_CUDA(h, rg::launch_update(a, h->stream, false, true, false));
     if (tr) RG_CUDA(h, rg::launch_tr_update(a, ta, h->stream, false, true, false));
   }
-  RG_TRY(download_pv(h, pv_out));
+  // the point velocities are final since ev_motion: copied beside the kernels
+  // above (512^2: 24 us), enqueued after them as a pageable copy holds the host
+  if (pv_out) {
+    RG_CUDA(h, cudaStreamWaitEvent(h->download_stream, h->ev_motion, 0));
+    RG_TRY(download_pv(h, pv_out, h->download_stream));
+    RG_CUDA(h, cudaEventRecord(h->ev_pv, h->download_stream));
+    RG_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_pv, 0));
+  }
   h->have_fluxes = false;
   h->dt_next_ready = false;
   const rg_status st = collect(h, h->d_status, h->stream);
