@@ -359,7 +359,7 @@ def run_reference(args, world, rank):
 # ------------------------------------------------------------------ GPU
 
 KERNELS = ["cfl", "slopes", "faces", "update"]
-KERNEL_NAMES = {0: {"cfl": "k_cfl", "slopes": "k_slopes", "faces": "k_faces_lgi", "update": "k_update"},
+KERNEL_NAMES = {0: {"cfl": "k_cfl", "slopes": "k_slopes", "faces": "k_faces", "update": "k_update"},
                 1: {"cfl": "k_cfl32", "slopes": "k_slopes32", "faces": "k_faces32_lgi", "update": "k_update_mixed"}}
 
 

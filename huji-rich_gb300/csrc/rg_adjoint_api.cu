@@ -195,14 +195,18 @@ rg_status check_run(rg_handle* h, int32_t n_steps, double dt, bool allow_mixed =
   return ensure_adjacency(h);
 }
 
+// (faces at rest unless face velocities were set: the buffer is otherwise as
+// it was allocated)
 rg::MixedArgs mixed_fixed_dt(rg_handle* h, double dt) {
   rg::MixedArgs m = mixed_args(h);
+  m.ev_zero = m.ev_zero || !h->have_ev;
   m.dt32 = static_cast<float>(dt);
   m.dt32_from_device = 0;
   return m;
 }
 rg::StepArgs fixed_dt(rg_handle* h, double dt) {
   rg::StepArgs a = step_args(h);
+  a.ev_zero = a.ev_zero || !h->have_ev;
   a.dt_host = dt;
   return a;
 }

@@ -258,10 +258,10 @@ rg_status rg_step(rg_handle* h, double* dt_out);
  * are checked once at the end.  dt_out (n_steps, host) may be NULL. */
 rg_status rg_run(rg_handle* h, int32_t n_steps, double* dt_out);
 /* rg_step with CUDA events between its kernels (the work is identical):
- * kernel_ms[0..3] = CFL (with the ghost fill), LinearGaussImproved slopes
+ * kernel_ms[0..3] = CFL (0 but for its first step), LinearGaussImproved slopes
  * (0 for order 1), face fluxes, gather + cell update.  For the Heun step:
- * CFL, first pass (slopes + faces + update), second pass (ghost fill +
- * slopes + faces), final update. */
+ * CFL, first pass (slopes + faces + update), second pass (slopes + faces),
+ * final update. */
 rg_status rg_step_timed(rg_handle* h, double* dt_out, float* kernel_ms);
 /* Enqueues one fused step on the handle's stream and returns at once; its
  * failures surface at the next rg_synchronize. */
