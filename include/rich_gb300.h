@@ -540,7 +540,8 @@ rg_status rg_get_tracer_slopes(rg_handle* h, double* tracer_slopes);
  * FP64 step with that dt).
  * rg_step_bwd: given cells_bar = dL/dW_n (host, n_cells*4) returns
  * cells0_bar = dL/dW_0 (host, n_cells*4) for the last rg_step_fwd,
- * recomputing each checkpoint interval forward once.  The handle's state is
+ * recomputing each checkpoint interval forward once (but the one whose steps
+ * are still recorded: the last, after rg_step_fwd).  The handle's state is
  * left as rg_step_fwd left it.
  * rg_step_tlm: tangent-linear run: from W_0 (the handle's cells) and a
  * tangent dcells0 (host, n_cells*4) runs n_steps and returns the tangent of
