@@ -7,9 +7,10 @@
 // restates (paths relative to the RICH source root).
 //
 // Passes of one step (hdsim::TimeAdvance, hdsim2d.cpp:149-241, fixed mesh):
-//   k_cfl        per cell: SimpleCFL bound, block min, last block writes dt
-//   k_slopes     per cell: LinearGaussImproved slope + limiter (order 2)
-//   k_faces_*    per face: reconstruction to the face, HLLC in the face frame,
+//   k_cfl        per cell: SimpleCFL bound, block min, last block writes dt (the
+//                first step only: each update forms the next one's)
+//   k_slopes     per cell and component: LinearGaussImproved slope + limiter (order 2)
+//   k_faces      per face: reconstruction to the face, HLLC in the face frame,
 //                rotation back, optional dt*area scaling
 //   k_update     per cell: ascending-face CSR gather of the face fluxes
 //                (SimpleExtensiveUpdater order, no atomics) + SimpleCellUpdater
