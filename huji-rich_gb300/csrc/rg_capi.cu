@@ -325,9 +325,12 @@ namespace {
 // one problem at first order by the face kernel.  A batch is fused on the
 // FP32-mixed path (a CFL pass of its own took 18 us of a step's 185, 96 Riemann
 // problems; in the update 7); the FP64 update screens one minimum, not many.
+// TimeAdvance2Heun forms its dt itself.
 bool fusable(const rg_handle* h) {
-  return !h->external_state && (h->n_problems == 0 || (h->mixed && h->cfg.order == 2 && !h->heun));
+  return !h->external_state && !h->heun && (h->n_problems == 0 || (h->mixed && h->cfg.order == 2));
 }
+// the kernels read no face velocities (as step_args and mixed_args pass it)
+bool at_rest(const rg_handle* h) { return h->ev_zero && !h->external_state; }
 
 // hdsim::TimeAdvance2Heun on a fixed mesh (hdsim2d.cpp:323-449): dt once;
 // pass 1 on the cells writes the mid extensives and mid cells; pass 2 on the
@@ -1380,6 +1383,7 @@ rg_status rg_run_graph(rg_handle* h, int32_t n_steps) {
   h->last = rg_error{};
   if (n_steps == 0) return RG_OK;
   if (h->step_mode == RG_STEP_PERSISTENT) return run_persistent(h, n_steps, nullptr);
+  if (h->graph_exec && (h->graph_fused != fusable(h) || h->graph_ev_zero != at_rest(h))) drop_graph(h);
   RG_TRY(reset_status(h, h->d_status, h->stream));
   if (fusable(h) && !h->dt_next_ready) {
     // one step with its own CFL pass; the captured step is the fused form,
@@ -1402,6 +1406,8 @@ rg_status rg_run_graph(rg_handle* h, int32_t n_steps) {
     }
     if (ce != cudaSuccess) return cuda_fail(h, ce);
     h->graph = g;
+    h->graph_fused = fusable(h);
+    h->graph_ev_zero = at_rest(h);
     RG_CUDA(h, cudaGraphInstantiate(&h->graph_exec, h->graph, 0));
   }
   for (int k = 0; k < n_steps; ++k) RG_CUDA(h, cudaGraphLaunch(h->graph_exec, h->stream));

@@ -185,9 +185,12 @@ struct rg_handle {
   rgh::DevBuf barrier, dt_trace;
   // where the step being enqueued keeps its dt (rg_run's record), or nullptr
   double* step_trace = nullptr;
-  // CUDA graph of one fused step
+  // CUDA graph of one step, and what it captured of the handle's state (a
+  // step with the other form is captured anew): whether it takes its dt from the
+  // update before it, and whether it reads no face velocities
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
+  bool graph_fused = false, graph_ev_zero = false;
   size_t cells_records = 0;
   bool have_cells = false, have_ext = false, have_ev = false, have_fluxes = false;
   rgh::HostBuf staging, host_status, host_dts;
