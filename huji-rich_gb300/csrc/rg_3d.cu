@@ -368,9 +368,11 @@ __global__ void __launch_bounds__(kBlock) k3_update(Step3Args a) {
   chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   Cell3 c{1, 1, V3{0, 0, 0}};
-  const bool live = i < a.mesh.n && update_cell3<kUnscaled, kExt, kCells>(a, i, c);
-  if (kExt && kCells && a.cfl_next)
-    grid_min_times(a.status, cfl3_block_bits(a, live, i, c), a.cfl, &a.status->dt_next);
+  const bool in = i < a.mesh.n, live = in && update_cell3<kUnscaled, kExt, kCells>(a, i, c);
+  if (kExt && kCells && a.cfl_next) {
+    if (in && !live) c = load_cell3(a.cells, i);  // a rejected cell keeps its record, which a CFL pass reads
+    grid_min_times(a.status, cfl3_block_bits(a, in, i, c), a.cfl, &a.status->dt_next);
+  }
 }
 
 // Records of 5 doubles (the host's) <-> 6 (the device's, the last one 0), one

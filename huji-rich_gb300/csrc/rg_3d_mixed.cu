@@ -226,9 +226,11 @@ __global__ void __launch_bounds__(kBlock) k3m_update(Mixed3Args a) {
   chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   C3 c{1.0f, 1.0f, F3{0.0f, 0.0f, 0.0f}};
-  const bool live = i < a.mesh.n && update_cell3m<kUnscaled, kExt, kCells>(a, i, c);
-  if (kExt && kCells && a.cfl_next)
-    grid_min_times(a.status, live ? cfl3m_bits(a, i, c) : kInfBits, a.cfl, &a.status->dt_next, &a.status->dt_next32);
+  const bool in = i < a.mesh.n, live = in && update_cell3m<kUnscaled, kExt, kCells>(a, i, c);
+  if (kExt && kCells && a.cfl_next) {
+    if (in && !live) c = load32(a, i);  // a rejected cell keeps its record, which a CFL pass reads
+    grid_min_times(a.status, in ? cfl3m_bits(a, i, c) : kInfBits, a.cfl, &a.status->dt_next, &a.status->dt_next32);
+  }
 }
 
 __global__ void __launch_bounds__(kBlock) k3m_d2f(const double* a, float* b, int n) {

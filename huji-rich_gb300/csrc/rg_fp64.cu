@@ -1049,6 +1049,11 @@ __global__ void __launch_bounds__(kMaxBlock) k_update(StepArgs a) {
     if (t < a.mesh.n) {
       i = order ? order[t] : t;
       live = update_cell<kBatch, kMode>(a, i, c);
+      if (next && !live) {
+        // a rejected cell keeps its record, which a CFL pass reads
+        c = load_cell(a.cells, i);
+        live = true;
+      }
     }
     if (next) {
       const unsigned long long b = cfl_block_bits<kBatch>(a, live, i, c);

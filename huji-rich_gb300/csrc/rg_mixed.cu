@@ -1006,6 +1006,11 @@ __device__ __forceinline__ unsigned long long cfl32_next(const MixedArgs& a, int
   const float res = (cs + sqrtf(q)) / a.g32.width[i];
   return static_cast<unsigned long long>(__double_as_longlong(widen_exact(1.0f / res)));
 }
+// the bound of a cell that keeps its record (rejected, or frozen)
+template <bool kBatch>
+__device__ __forceinline__ unsigned long long cfl32_kept(const MixedArgs& a, int i) {
+  return a.cfl_next ? cfl32_next<kBatch>(a, i, a.cells32[i]) : kInfBits;
+}
 template <bool kBatch, int kMode>
 __device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArgs& a, int i) {
   constexpr bool do_ext = kMode != kUpCells, do_cells = kMode != kUpUnscaled && kMode != kUpScaled;
@@ -1059,16 +1064,14 @@ __device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArg
     if (a.frozen_mask && (a.stickers[i] & a.frozen_mask)) {
       // simple_cell_updater.cpp:61-83 with (HasSticker, SkipUpdate): the old
       // cell stays (its extensives above still took the fluxes)
-      const float4 c = a.cells32[i];
-      if (a.cells32_out) a.cells32_out[i] = c;
-      if (!a.cfl_next) return kInfBits;
-      return cfl32_next<kBatch>(a, i, c);
+      if (a.cells32_out) a.cells32_out[i] = a.cells32[i];
+      return cfl32_kept<kBatch>(a, i);
     }
     const float mf = narrow(mass);
     const float d = mf * a.g32.inv_cd_volume[i];
     if (d < 0.0f) {
       record_error(a.status, a.step, RG_ERR_NEGATIVE_DENSITY, 5, i, d);
-      return kInfBits;
+      return cfl32_kept<kBatch>(a, i);
     }
     // 1/m: the FP32 reciprocal (relative error < 2^-23) and one Newton step
     // (relative error < 2^-45, far below the FP32 rounding of the results)
@@ -1079,7 +1082,7 @@ __device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArg
     const double energy = en * r - 0.5 * (vx * vx + vy * vy);
     if (lt(energy, 0.0)) {
       record_error(a.status, a.step, RG_ERR_NEGATIVE_ENERGY, 5, i, energy);
-      return kInfBits;
+      return cfl32_kept<kBatch>(a, i);
     }
     const float4 c = make_float4(d, (gamma32<kBatch>(a, i) - 1.0f) * narrow(energy) * d, narrow(vx), narrow(vy));
     (a.cells32_out ? a.cells32_out : a.cells32)[i] = c;
