@@ -1208,7 +1208,7 @@ cudaError_t launch_slopes_trace(const StepArgs& a, SlopeTrace* trace, cudaStream
 }
 
 cudaError_t launch_faces(const StepArgs& a, cudaStream_t s, bool scaled) {
-  if (a.mesh.e == 0) return cudaSuccess;
+  if (a.mesh.e == 0 && !a.take_next_dt) return cudaSuccess;
   const LaunchShape sh = fit_shape(a.shapes.faces, a.mesh.e);
   const int nb = grid_of(sh, a.mesh.e), bs = sh.block;
   const bool b = a.cell_problem != nullptr;

@@ -1281,7 +1281,7 @@ cudaError_t launch_slopes32(const MixedArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t launch_faces32(const MixedArgs& a, cudaStream_t s, bool scaled) {
-  if (a.mesh.e == 0) return cudaSuccess;
+  if (a.mesh.e == 0 && !a.take_next_dt) return cudaSuccess;
   const int nb = grid_of(a.shapes.faces, a.mesh.e), bs = a.shapes.faces.block;
   const bool b = a.cell_problem != nullptr;
   if (a.order == 1) {
