@@ -345,7 +345,8 @@ __device__ __forceinline__ void lane_limit(const StepArgs& a, int b, int nn, dou
             } else {
               const float q = __fdividef(th * fabsf(g), ad);
               const float rel = 2e-6f + 2.0f * __fdividef(err, ad);
-              if (rel < 0.1f) {
+              // (below the normal floats q's error is absolute: formed in FP64)
+              if (rel < 0.1f && q > 1e-30f) {
                 low[k] = q * (1.0f - rel);
                 best = fminf(best, q * (1.0f + rel));
               }
