@@ -141,7 +141,8 @@ static __device__ __noinline__ unsigned long long cfl3_bound_bits(const Step3Arg
 // The smallest bound of the block's cells, formed on the threads whose cell can
 // hold it (the others return +inf): an FP32 estimate of the rate (|v| + c)/width,
 // good to 1e-5, rules the rest out.  Operands outside the normal floats are
-// formed.  Every thread of the block calls this.
+// formed, and rates below 1e-30 (widths above 2^126, by which the approximate
+// quotient is 0, among them).  Every thread of the block calls this.
 __device__ __forceinline__ unsigned long long cfl3_block_bits(const Step3Args& a, bool live, int i, const Cell3& c) {
   __shared__ unsigned best;
   if (threadIdx.x == 0) best = 0u;
@@ -154,7 +155,7 @@ __device__ __forceinline__ unsigned long long cfl3_block_bits(const Step3Args& a
     const float r = __fdividef(sqrtf(fmaf(x, x, fmaf(y, y, z * z))) + cs, w);
     lo = r * 0.9999f;
     hi = r * 1.0001f;
-    if (!(ok && hi < 1e30f && cs > 1e-15f && w > 0.0f)) {
+    if (!(ok && hi > 1e-30f && hi < 1e30f && cs > 1e-15f && w > 0.0f)) {
       lo = 0.0f;
       hi = 3e38f;
     }

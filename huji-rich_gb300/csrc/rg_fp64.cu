@@ -326,7 +326,8 @@ static __device__ __noinline__ unsigned long long cfl_bound_bits(const StepArgs&
 // truncations to 24 bits leave each difference v - w_e within
 // 2^-23 (|v| + |w_e|) and a rounding; cs, the root and the quotient carry a few
 // 2^-24 each.  hi is infinite (and lo 0) where an operand is outside the normal
-// floats or a value is not finite.
+// floats, a value is not finite or the rate is below 1e-30 (a width above 2^126,
+// by which the approximate quotient is 0, among them).
 template <bool kBatch>
 __device__ __forceinline__ void cfl_estimate(const StepArgs& a, int i, const Cell& c, float& lo, float& hi) {
   const MeshDev& m = a.mesh;
@@ -351,7 +352,7 @@ __device__ __forceinline__ void cfl_estimate(const StepArgs& a, int i, const Cel
   const float v = sqrtf(q);
   lo = __fdividef(0.99999f * cs + fmaxf(0.99999f * v - err, 0.0f), r) * 0.99999f;
   hi = __fdividef(1.00001f * cs + 1.00001f * v + err, r) * 1.00001f;
-  if (!(ok && e1 > b && hi < 1e30f && cs > 1e-15f && r > 0.0f)) {
+  if (!(ok && e1 > b && hi > 1e-30f && hi < 1e30f && cs > 1e-15f && r > 0.0f)) {
     lo = 0.0f;
     hi = 3e38f;
   }
