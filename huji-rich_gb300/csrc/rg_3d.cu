@@ -440,7 +440,7 @@ cudaError_t launch3_cfl(const Step3Args& a, cudaStream_t s) {
 
 cudaError_t launch3_faces(const Step3Args& a, bool scaled, cudaStream_t s) {
   if (a.mesh.e == 0) return cudaSuccess;
-  const LaunchShape sh = fit_shape(LaunchShape{kBlock, 0, 0}, a.mesh.e);
+  const LaunchShape sh = fit_shape(LaunchShape{kBlock, 0, 0, a.sms}, a.mesh.e);
   const int nb = grid_of(sh, a.mesh.e);
   if (scaled)
     chain(s, nb, sh.block, k3_faces<true>, a);

@@ -44,6 +44,7 @@ struct Step3Args {
   int cfl_next;           // the fused update also computes the next step's dt (status->dt_next)
   int take_next_dt;       // the face kernel moves status->dt_next to status->dt and scales by it
   double* dt_trace;       // where the step's dt is kept, or nullptr
+  int sms;                // the device's SM count (fit_shape)
 };
 
 // FP32-mixed 3D path (rg_3d_mixed.cu): FP32 primitives, unit normals,

@@ -52,6 +52,7 @@ struct rg3_handle {
   double* h_dts = nullptr;       // pinned, h_dts_len doubles
   size_t h_dts_len = 0;
   bool fvel_set = false;
+  int sms = 0;  // the device's SM count
   // FP32-mixed path (rg_config.precision == RG_FP32_MIXED)
   bool mixed = false;
   Buf nhat32, area32, width32, cells32, vz32, flux32, fen32, fvel32;
@@ -125,6 +126,7 @@ rg::Step3Args args(rg3_handle* h) {
   a.fluxes = static_cast<double*>(h->fluxes.p);
   a.fvel = h->fvel_set ? static_cast<const double*>(h->fvel.p) : nullptr;
   a.status = h->d_status;
+  a.sms = h->sms;
   return a;
 }
 
@@ -246,6 +248,7 @@ rg_status rg3_create(const rg_config* cfg, rg3_handle** out) {
   if ((e = cudaSetDevice(cfg->device)) != cudaSuccess || (e = cudaStreamCreateWithFlags(&h->stream,
                                                                                          cudaStreamNonBlocking)) !=
                                                              cudaSuccess ||
+      (e = cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, cfg->device)) != cudaSuccess ||
       (e = h->status_buf.ensure(sizeof(DevStatus))) != cudaSuccess ||
       (e = cudaMallocHost(&h->h_status, sizeof(DevStatus))) != cudaSuccess ||
       (e = cudaEventCreate(&h->ev[0])) != cudaSuccess || (e = cudaEventCreate(&h->ev[1])) != cudaSuccess ||

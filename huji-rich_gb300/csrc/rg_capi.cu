@@ -686,6 +686,10 @@ rg_status rg_create(const rg_config* cfg, rg_handle** out) {
   };
   cudaError_t e;
   if ((e = cudaSetDevice(cfg->device)) != cudaSuccess) return fail(e);
+  int sms = 0;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device)) != cudaSuccess) return fail(e);
+  for (rg::StepShapes* s : {&h->shapes64, &h->shapes32})
+    for (rg::LaunchShape* k : {&s->cfl, &s->slopes, &s->faces, &s->update}) k->fit_sms = sms;
   if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
   if ((e = cudaStreamCreateWithFlags(&h->upload_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
   if ((e = cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);

@@ -208,19 +208,23 @@ constexpr int kMaxBlock = 512;
 // the FP32-mixed update kernel has register-capped builds 2 and 3 too, and the
 // FP64 slopes kernel register-capped builds 2 and 3 for 3 and 4 resident
 // blocks.
+// fit_sms: the SM count, on the built-in shapes (fit_shape); 0: launched as it is
+// (the shapes that a caller or the autotuner sets).
 struct LaunchShape {
   int block;
   int max_blocks;
   int variant;
+  int fit_sms = 0;
 };
 constexpr LaunchShape kDefaultShape{256, 0, 0};
 constexpr int kCappedBlock = 256;
-// A one-thread-per-item grid of large blocks that would leave SMs without one
-// is launched in smaller blocks (256 x 66-face meshes and the like: the FP64
-// faces of 96 x 101 cells take 16 us in blocks of 64 to 256, 20 us as 57 of 512).
-constexpr int kSms = 152;
+// A built-in one-thread-per-item shape whose large blocks would leave SMs
+// without one is launched in smaller blocks (256 x 66-face meshes and the like: the
+// FP64 faces of 96 x 101 cells take 16 us in blocks of 64 to 256, 20 us as 57 of 512).
 inline LaunchShape fit_shape(LaunchShape s, long long items) {
-  while (s.max_blocks == 0 && s.block > 64 && s.block % 64 == 0 && items < 2LL * kSms * s.block) s.block /= 2;
+  while (s.fit_sms > 0 && s.max_blocks == 0 && s.block > 64 && s.block % 64 == 0 &&
+         items < 2LL * s.fit_sms * s.block)
+    s.block /= 2;
   return s;
 }
 inline int grid_of(const LaunchShape& s, long long items) {

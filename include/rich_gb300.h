@@ -325,7 +325,10 @@ rg_status rg_stream(const rg_handle* h, void** stream);
  * (rg_config.precision; batch or single problem) each run with a launch
  * shape: threads per block (a multiple of 32, 32..512) and max_blocks (0: one
  * thread per cell or face; > 0: a persistent grid of at most that many blocks
- * striding over the items).  Results are identical for every shape. */
+ * striding over the items).  Results are identical for every shape.  The
+ * shapes of a new handle are for large meshes: on small ones (less than two
+ * blocks for every SM) the one-thread-per-item kernels run in smaller blocks.
+ * Shapes that rg_set_launch_shapes or rg_autotune sets are launched as they are. */
 typedef enum { RG_KERNEL_CFL = 0, RG_KERNEL_SLOPES = 1, RG_KERNEL_FACES = 2, RG_KERNEL_UPDATE = 3 } rg_kernel;
 typedef struct {
   int32_t block[4];
