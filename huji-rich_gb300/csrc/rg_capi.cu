@@ -664,20 +664,13 @@ rg_status rg_create(const rg_config* cfg, rg_handle** out) {
   if (!h) return RG_ERR_OUT_OF_MEMORY;
   h->cfg = *cfg;
   h->mixed = cfg->precision == RG_FP32_MIXED;
-  // the FP64 slopes: the build for four resident blocks of 256 (64 registers).
-  // Bound by the FP64 unit's latency and issue, they gain from every warp
-  // (512^2: 172 us; 179 us with three resident blocks, 211 us as the plain
-  // build's two)
-  h->shapes64.slopes = rg::LaunchShape{256, 0, 3};
   // the FP64 faces in blocks of 512 (k_faces)
   h->shapes64.faces = rg::LaunchShape{512, 0, 0};
-  // the FP32-mixed slopes and faces in blocks of 128 (1024^2: slopes 62 us, 67 us
-  // in blocks of 256; faces 50.0 and 51.5 us), the update too, as the build for
-  // six resident blocks of 256 (1024^2: 54 us, 56 us in blocks of 256, 69 us as
-  // the plain build)
+  // the FP32-mixed slopes, faces and update in blocks of 128 (1024^2: slopes 62
+  // us, 67 us in blocks of 256; faces 50.0 and 51.5 us; update 54 and 56 us)
   h->shapes32.slopes = rg::LaunchShape{128, 0, 0};
   h->shapes32.faces = rg::LaunchShape{128, 0, 0};
-  h->shapes32.update = rg::LaunchShape{128, 0, 3};
+  h->shapes32.update = rg::LaunchShape{128, 0, 0};
   h->heun = cfg->time_integrator == RG_TIME_ADVANCE_HEUN;
   auto fail = [&](cudaError_t e) {
     rg_destroy(h);

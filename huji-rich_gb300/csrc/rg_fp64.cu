@@ -507,11 +507,13 @@ __device__ __forceinline__ void slopes_lane(const StepArgs& a, int i, int q, uns
   }
 }
 
-// Four lanes per cell (an item).  kMinBlocks > 0: register-capped builds for
-// blocks of up to kCappedBlock threads with kMinBlocks resident per SM
-// (launch-shape variants 2 and 3)
+// Four lanes per cell (an item).  The plain build holds 64 registers (two
+// resident blocks of kMaxBlock): bound by the FP64 unit's latency and issue, the
+// slopes gain from every warp (512^2: 172 us; 179 us in 80 registers, 211 us
+// with no cap).  kMinBlocks > 0: builds for blocks of up to kCappedBlock threads
+// with kMinBlocks resident per SM (launch-shape variants 2 and 3)
 template <bool kBatch, int kMinBlocks = 0, bool kTrace = false>
-__global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 1)
+__global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 2)
     k_slopes(StepArgs a, SlopeTrace* trace) {
   chain_wait();
   take_next_dt(a);

@@ -1092,10 +1092,12 @@ __device__ __forceinline__ unsigned long long k_update_mixed_item(const MixedArg
   return kInfBits;
 }
 
-// kMinBlocks > 0: register-capped builds for blocks of up to kCappedBlock
-// threads with kMinBlocks resident per SM (launch-shape variants 2 and 3)
+// The plain build holds 40 registers (three resident blocks of kMaxBlock;
+// 1024^2: 54 us, 69 us with no cap).  kMinBlocks > 0: builds for blocks of up to
+// kCappedBlock threads with kMinBlocks resident per SM (launch-shape variants 2
+// and 3)
 template <bool kBatch, int kMode, int kMinBlocks = 0>
-__global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 1)
+__global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlocks ? kMinBlocks : 3)
     k_update_mixed(MixedArgs a) {
   chain_wait();
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
