@@ -1037,7 +1037,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_update(StepArgs a) {
       a.dt_p[p] = dt;
       a.time_p[p] += dt;
       a.dtmin_p[p] = kInfBits;
-      if (p == 0 && a.dt_trace) *a.dt_trace = dt;
+      if (p == 0) {  // what the step's call returns, and the run's record
+        a.status->dt = dt;
+        if (a.dt_trace) *a.dt_trace = dt;
+      }
     }
   }
   unsigned long long bits = kInfBits;

@@ -1107,7 +1107,10 @@ __global__ void __launch_bounds__(kMinBlocks ? kCappedBlock : kMaxBlock, kMinBlo
       a.dt_p[p] = dt;
       a.time_p[p] += dt;
       a.dtmin_p[p] = kInfBits;
-      if (p == 0 && a.dt_trace) *a.dt_trace = dt;
+      if (p == 0) {  // what the step's call returns, and the run's record
+        a.status->dt = dt;
+        if (a.dt_trace) *a.dt_trace = dt;
+      }
     }
   }
   if (kBatch && a.cfl_next) {
@@ -1165,7 +1168,10 @@ __global__ void __launch_bounds__(kPersistBlock, 4)
       a.dt_p[p] = dt;
       a.time_p[p] += dt;
       a.dtmin_p[p] = kInfBits;
-      if (p == 0 && dt_trace) dt_trace[k] = dt;
+      if (p == 0) {
+        a.status->dt = dt;
+        if (dt_trace) dt_trace[k] = dt;
+      }
     }
     for (int i = t0; i < m.n; i += stride) k_update_mixed_item<true, kUpFused>(a, i);
     if (!grid_sync(gb, gen, expected, s_ok, a.status, a.step)) return;
