@@ -63,7 +63,9 @@ def build(force=False, verbose=False):
     os.makedirs(OUT_DIR, exist_ok=True)
     cc = nvcc()
     deps = _deps()
-    common = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
+    # (not compressed: a process's first call unpacks a compressed module, 8 ms for
+    # rg_fp64's 11 MB, which nvcc compresses by default from some size on)
+    common = ARCH + ["--no-compress", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
                      "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
     if verbose:
         common += ["-Xptxas", "-v"]
