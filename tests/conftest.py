@@ -18,6 +18,13 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (GB300, sm_103a)")
 
 
+def pytest_collection_modifyitems(items):
+    # the drop-in tests run the reference's own hdsim, which a tree without the
+    # reference's sources cannot build: they come last, so that a run that stops
+    # at the first failure has run everything else
+    items.sort(key=lambda item: os.path.basename(str(item.path)) == "test_gpu_hdsim.py")
+
+
 GOLDEN_CASES = sorted(os.path.basename(f)[:-4] for f in glob.glob(os.path.join(GOLDEN, "*.npz")))
 # cases that also hold an N-step hdsim run on a mesh hdsim rebuilt unchanged
 RUN_CASES = [c for c in GOLDEN_CASES
