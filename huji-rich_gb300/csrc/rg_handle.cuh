@@ -100,6 +100,9 @@ struct SlotLayout {
     cflags = take(4 * static_cast<size_t>(n));
     nbr = take(4 * static_cast<size_t>(m));
     hr = take(16 * static_cast<size_t>(m));
+    // on the mixed path only the FP64 geometry formed on demand has dmf, and
+    // frec32 is scratch of the pass without it: they share their bytes (m <= 2 e)
+    dmf = frec32 = take(mixed ? 32 * static_cast<size_t>(e) : 8 * static_cast<size_t>(m));
     ghost_real = take(4 * static_cast<size_t>(g));
     ghost_unit = take(16 * static_cast<size_t>(g));
     cell_order = take(4 * static_cast<size_t>(n));
@@ -117,10 +120,6 @@ struct SlotLayout {
     fsign32 = take(k * 4 * static_cast<size_t>(m));
     gunit32 = take(k * 8 * static_cast<size_t>(g));
     icdv32 = take(k * 4 * static_cast<size_t>(n));
-    frec32 = take(k * 32 * static_cast<size_t>(e));
-    // on the mixed path only the FP64 geometry formed on demand has dmf, and
-    // frec32 is scratch of the pass without it: they share their bytes (m <= 2 e)
-    dmf = mixed ? frec32 : take(8 * static_cast<size_t>(m));
     total = o;
   }
 };

@@ -16,8 +16,9 @@ int main() {
         const int n = s[0], g = s[1], e = s[2], m = s[3];
         L.compute(n, g, e, m, mixed, cyl);
         const size_t dmf_end = L.dmf + 8 * static_cast<size_t>(m), frec_end = L.frec32 + 32 * static_cast<size_t>(e);
-        const bool ok = mixed ? L.dmf >= L.frec32 && dmf_end <= frec_end && L.total == rgh::align_up(frec_end)
-                              : L.dmf >= L.frec32 && L.total == rgh::align_up(dmf_end);
+        const bool ok = L.dmf == L.frec32 && (mixed ? dmf_end <= frec_end : true) &&
+                        L.ghost_real == rgh::align_up(mixed ? frec_end : dmf_end) &&
+                        L.total == rgh::align_up(L.icdv32 + (mixed ? 4 * static_cast<size_t>(n) : 0));
         if (!ok) {
           std::printf("n %d e %d m %d mixed %d: dmf %zu..%zu, scratch %zu..%zu, total %zu\n", n, e, m, mixed, L.dmf,
                       dmf_end, L.frec32, frec_end, L.total);
