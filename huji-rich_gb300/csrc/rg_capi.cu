@@ -8,8 +8,8 @@
 // and makes the compute stream wait for it, so an upload overlaps whatever
 // compute work is still in flight on the previous mesh.
 //
-// Every index of a mesh is checked on the host before it is copied: the
-// kernels index with them unchecked.
+// Every index of a mesh is checked on the device (k_validate) before any other
+// kernel indexes with it.
 #include <cuda_runtime.h>
 
 #include <algorithm>

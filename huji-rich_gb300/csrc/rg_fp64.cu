@@ -408,11 +408,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_cfl(StepArgs a) {
 // FP64 operations of a lane are the Green-Gauss sums (8 per neighbour), which
 // the reference's order of additions fixes, plus the limiter's surviving
 // candidates (rg_lgi.cuh).  `quad`: the quad's lanes in the warp (all four run
-// with the same cell).  Bound by the FP64 pipe (85 FP64 instructions per warp
-// of eight cells, 72 % active).  With one thread per cell and every candidate
-// in FP64 (117 per warp of eight cells at full lanes, 5,960 instructions in
-// one chain): 478 us at 512^2, 95 us at 256^2, 89 us at 96 x 101 cells; now
-// 197, 51 and 17 us.
+// with the same cell).  Bound by the FP64 unit (62 % of its issue slots at 512^2).
+// Events around the launch in Sedov's first steps, with one thread per cell and
+// every candidate in FP64 (5,960 instructions in one chain): 489 us at 512^2, 159
+// us at 256^2, 103 us at 96 x 101 cells; now 172, 62 and 25 us.
 template <bool kBatch, bool kTrace>
 __device__ __forceinline__ void slopes_lane(const StepArgs& a, int i, int q, unsigned quad, SlopeTrace* trace) {
   const MeshDev& m = a.mesh;
@@ -1080,7 +1079,6 @@ __global__ void __launch_bounds__(kBlock) k_init_ext(StepArgs a) {
          c.vx * mass, c.vy * mass);
 }
 
-// *flag = 1 if any of v[0..n) is not +-0 (NaN counts as nonzero)
 // The error part of `count` status blocks, emptied: one launch (about 1 us
 // in a chain of kernels), where the two memsets of a block took 5 us.
 __global__ void k_reset_status(DevStatus* st, int count) {
@@ -1092,6 +1090,7 @@ __global__ void k_reset_status(DevStatus* st, int count) {
   }
 }
 
+// *flag = 1 if any of v[0..n) is not +-0 (NaN counts as nonzero)
 __global__ void __launch_bounds__(kBlock) k_any_nonzero(const double* v, long long n, int* flag) {
   bool any = false;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;

@@ -4,8 +4,8 @@
 // Layout in HBM (all arrays owned by one rg_handle):
 //   points  double2[np]   mesh points, real cells then ghosts (np = n + g)
 //   cms     double2[np]   cell centres of mass
-//   cells   dbl4-like  double[4*np]: {density, pressure, vx, vy}; entries
-//                         n..np-1 hold ghost states (filled per step)
+//   cells   double[4*n]   {density, pressure, vx, vy} (a ghost's state is formed
+//                         from its cell's where it is read)
 //   ext     double[4*n]   {mass, energy, px, py}
 //   faces   int2[e]       (first, second) point ids
 //   face geometry (per upload): area, normal n, |n|, parallel p, mid - cm of
@@ -248,7 +248,7 @@ struct StepArgs {
   Divisor gm1;          // gamma - 1 as a divisor (one problem)
   int order, ghost_kind, slf;
   double delta_v, theta, delta_p;
-  double* cells;        // 4*np (ghost entries at the end), read by every pass
+  double* cells;        // 4*n, read by every pass
   double* ext;          // 4*n, read by the update
   double* ext_out;      // where the update writes extensives (nullptr: ext)
   double* cells_out;    // where the update writes cells (nullptr: cells)

@@ -156,7 +156,7 @@ __device__ __forceinline__ void lane_slope(const StepArgs& a, int i, int b, int 
   } else {
     // the first neighbour starts the sums (cell*h, then + nb*h).  The cell's
     // products run on the integer pipes beside the FP64 unit (rg_mul.cuh):
-    // 512^2 slopes 197 -> 172 us, 256^2 51 -> 42 us
+    // 512^2 slopes 197 -> 172 us
     const MulFactor fc = mul_factor(c);
 #pragma unroll
     for (int k = 0; k < kFit; ++k) {

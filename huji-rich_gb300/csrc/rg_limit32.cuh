@@ -30,7 +30,8 @@ __device__ __forceinline__ void shocked32(float dphi, float cv, float cellv, flo
 // The unshocked limiter of one component from the largest and the smallest
 // reconstructed value over the cell's faces: among the faces with a positive
 // centroid difference the largest has the smallest quotient maxd/dphi (the
-// FP32 quotient is monotone in its divisor, checked for every positive float),
+// FP32 quotient is monotone in its divisor, checked over every positive divisor
+// for eight numerators: tests/limit32_check.cu),
 // and it is active if any of them is, as |dphi| and the change of sign only
 // grow with it; with mind the smallest of the negative ones likewise.  psi is
 // their minimum, so no other face can set it.

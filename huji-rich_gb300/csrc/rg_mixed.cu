@@ -418,8 +418,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_cfl32(MixedArgs a) {
 }
 
 // The FP32 slopes of a periodic mesh (no self-mirror neighbour, no boundary
-// slope), written widened and as the FP32 slopes the face kernel reads, with
-// the limiter trace the adjoint's reverse slope kernel reads
+// slope), as the FP32 slopes that the face kernel reads, with the limiter trace the adjoint's reverse slope kernel reads
 // (SlopeTrace32: the unlimited slope, each component's factor, the centroid
 // difference and neighbour of its active candidate).  The arithmetic is
 // k_slopes32_item's; the arg max / min follow the first strict improvement

@@ -151,7 +151,7 @@ rg_status rg_autotune(rg_handle* h, int32_t reps, rg_launch_shapes* chosen) {
   cudaEvent_t e0 = h->ev_k[0], e1 = h->ev_k[1];
   rg::StepShapes& cur = path_shapes(h);
   rg_launch_shapes out{};
-  // inputs of every kernel first: ghosts and dt (CFL), slopes, fluxes
+  // inputs of every kernel first: dt (CFL), slopes, fluxes
   for (int k = 0; k < 3; ++k) RG_TRY(launch_one(h, k, *slot(cur, k), ext_scr.p, cells_scr.p));
   for (int k = 0; k < 4; ++k) {
     float best = 0;

@@ -252,7 +252,7 @@ rg_status rg_cell_update(rg_handle* h);
  * with time_integrator = RG_TIME_ADVANCE_HEUN, hdsim::TimeAdvance2Heun
  * (hdsim2d.cpp:323-449): fluxes on the cells, mid extensives and cells,
  * fluxes on the mid cells, extensives averaged.  dt never leaves the device
- * between the passes; *dt_out receives it. */
+ * between the passes; *dt_out receives it (a batch: problem 0's). */
 rg_status rg_step(rg_handle* h, double* dt_out);
 /* n_steps rg_step calls without a host synchronisation between them; errors
  * are checked once at the end.  dt_out (n_steps, host) may be NULL. */
@@ -291,9 +291,10 @@ rg_status rg_set_problems(rg_handle* h, int32_t n_problems, const int32_t* probl
 rg_status rg_get_problem_times(rg_handle* h, double* time_out, double* dt_last_out);
 
 /* n_steps fused steps replayed from a CUDA graph of one step (captured on
- * first use and after every upload or configuration change), one host
- * synchronisation at the end.  Same results as rg_run; a failure is reported
- * with step 0 in its key. */
+ * first use, after every upload or configuration change, when the face
+ * velocities leave or come to rest and when rg_device_buffers hands out the
+ * state), one host synchronisation at the end.  Same results as rg_run; a
+ * failure is reported with step 0 in its key. */
 rg_status rg_run_graph(rg_handle* h, int32_t n_steps);
 
 /* How rg_run / rg_run_graph run a batch (no reference counterpart).
