@@ -418,12 +418,13 @@ __global__ void __launch_bounds__(kMaxBlock) k_cfl32(MixedArgs a) {
 }
 
 // The FP32 slopes of a periodic mesh (no self-mirror neighbour, no boundary
-// slope), as the FP32 slopes that the face kernel reads, with the limiter trace the adjoint's reverse slope kernel reads
-// (SlopeTrace32: the unlimited slope, each component's factor, the centroid
-// difference and neighbour of its active candidate).  The arithmetic is
-// k_slopes32_item's; the arg max / min follow the first strict improvement
-// as std::max / std::min do, and each psi is the smallest candidate taken in
-// edge order, which is what fminf over the candidates gives.
+// slope), as the FP32 slopes that the face kernel reads, with the limiter trace
+// that the adjoint's reverse slope kernel reads (SlopeTrace32: the unlimited
+// slope, each component's factor, the centroid difference and neighbour of its
+// active candidate).  The arithmetic is k_slopes32_item's; the arg max / min
+// follow the first strict improvement as std::max / std::min do, and each psi is
+// the smallest candidate taken in edge order, which is what fminf over the
+// candidates gives.
 __global__ void __launch_bounds__(kBlock) k_slopes32_trace(MixedArgs a, SlopeTrace32* trace) {
   chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
